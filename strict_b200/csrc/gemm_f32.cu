@@ -6,6 +6,8 @@
 // Rows of X, W and Y may be wider than the product (ldx, ldw, ldy).
 #include "common.cuh"
 
+int k_gemm_f32_tc(strictb200_ctx* ctx, const GemmF32Args& g);  // gemm_f32_tc.cu
+
 namespace {
 constexpr int F32_MT = 8;
 
@@ -83,6 +85,14 @@ int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float
 int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   const int64_t M = g.M, N = g.N, K = g.K;
   if (K % 4 || g.ldx % 4 || g.ldw % 4) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: K and the row strides must be multiples of 4");
+  // One pass over the weights per eight rows (this kernel) or per 32 to 128 (the tensor cores). Measured, us, rows = 9 / 16 / 32 / 128 / 4700:
+  //   N 768  K 768    7.1 / 7.1 / 13.0 /  37.8 / 1197   against   8.5 / 8.5 /  8.7 / 13.9 /  62
+  //   N 3072 K 768   13.2 / 19.8 / 33.1 / 119.8 / 6240            9.3 / 9.3 /  9.5 / 14.9 / 192
+  //   N 1000 K 100    4.3 / 4.4 /  6.2 /  19.8 /  676            6.2 / 7.1 /  7.2 / 13.7 /  28
+  // so two passes over a small matrix stay here. Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336):
+  // 9.2e-8 / 1.0e-7 / 1.6e-7 here, 8.0e-8..9.1e-8 / 9.6e-8..1.0e-7 / 1.3e-7 there.
+  const bool few = M <= F32_MT || (M <= 2 * F32_MT && N * K <= (1 << 20));
+  if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) return k_gemm_f32_tc(ctx, g);
   int ks = 1;  // warps per output channel: slices of at most 1024 columns, as long as the grid stays small
   while (ks < 8 && K > 1024 * (int64_t)ks && (N * ks * 2 + 7) / 8 <= 8 * (int64_t)ctx->sm_count) ks *= 2;
   const int rows = 8 / ks;

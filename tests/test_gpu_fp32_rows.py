@@ -1,0 +1,91 @@
+"""fp32 path of many rows: linear layers through three bf16 terms on the tensor cores, attention over prompts in tiles, attention
+of a new token with the keys spread over groups of lanes."""
+import numpy as np
+import pytest
+
+import strict_b200 as sb
+from strict_b200 import native as N
+from strict_b200.kernel import DeviceVariable as DV
+from test_gpu_models import TINY_GPT2
+
+pytestmark = pytest.mark.gpu
+L = N.lib
+
+
+def _gemm(ctx, x, w, b):
+    dx, dw, dy = DV.of(ctx, x), DV.of(ctx, w), DV(ctx, len(x) * len(w))
+    db = DV.of(ctx, b) if b is not None else None
+    N.check(L().strictb200_gemm_f32(ctx.h, len(x), len(w), x.shape[1], dx.p, dw.p, db.p if db else None, dy.p))
+    y = dy.to_host().reshape(len(x), len(w))
+    for v in (dx, dw, dy, db):
+        if v:
+            v.free()
+    return y
+
+
+# rows around the token tiles (32, 64, 128), channels around a block's 128, columns around the 64 of a stage, the 1024 of a block and
+# two and eight blocks of a cluster
+@pytest.mark.parametrize("M,N_,K", [(9, 1, 4), (31, 127, 60), (32, 128, 64), (33, 129, 68), (64, 130, 1024), (65, 257, 1028), (128, 768, 3072),
+                                    (129, 300, 772), (300, 96, 8200), (1000, 40, 14336)])
+def test_gemm_f32_many_rows(ctx, rng, M, N_, K):
+    x = (rng.standard_normal((M, K)) * np.exp2(rng.integers(-6, 7, (M, K)))).astype(np.float32)
+    w = (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(N_).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm(ctx, x, w, None)
+    # of the sum of the products' magnitudes: two cut-off instructions and two additions per 64 columns of the large product (at most
+    # 2 * 2^-23 + 2^-24), one addition per 64 columns of a block's at most ceil(K / 8) or 1024 columns, seven between blocks, one unit for the rest
+    per_block = max(1024, (K + 7) // 8)
+    unit = 2.0 ** -24
+    assert (np.abs(got - want) <= (6 + per_block / 64 + 7 + 1) * unit * size).all()
+    rms = np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2))
+    assert rms < 2e-7  # plain fp32 sums of this length: 1e-7 to 1.6e-7
+    assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
+
+
+def test_gemm_f32_many_rows_not_finite(ctx, rng):
+    """Infinities and NaN reach exactly the results they reach in a plain sum; an operand row at the end of the fp32 range is computed."""
+    x, w = rng.standard_normal((40, 200)).astype(np.float32), rng.standard_normal((70, 200)).astype(np.float32)
+    x[3, 5], x[7, 9], w[13, 2] = np.inf, np.nan, -np.inf
+    x[11], x[11, 0] = 0.0, 3.4e38
+    w[:, 0] = np.clip(w[:, 0], -0.9, 0.9)
+    with np.errstate(invalid="ignore"):
+        want = x.astype(np.float64) @ w.astype(np.float64).T
+    got = _gemm(ctx, x, w, None).astype(np.float64)
+    fine = np.isfinite(want)
+    assert np.array_equal(np.isnan(want), np.isnan(got)) and np.array_equal(want[~fine & ~np.isnan(want)], got[~fine & ~np.isnan(want)])
+    assert np.allclose(got[fine], want[fine], rtol=1e-5, atol=1e-4)
+
+
+# head widths of the two kernels (64) and of the decode kernel alone (32, 128), one that neither takes; prompts around the 64-row tile
+@pytest.mark.parametrize("head_dim,lens", [(64, [1, 63, 64, 65, 130]), (64, [200, 3]), (32, [70, 9]), (128, [66, 40]), (48, [20, 33])])
+def test_gpt2_prompts_and_decode(ctx, oracle, head_dim, lens):
+    cfg = dict(TINY_GPT2, d_model=2 * head_dim, head_dim=head_dim, d_ff=4 * head_dim, max_pos=256, vocab=300)
+    B, S, seed = len(lens), max(lens), 11
+    m, om = sb.Model(ctx, cfg).init_random(seed), oracle.Model(cfg, seed)
+    kv, st = m.new_cache(B, S + 40), om.new_state(B, S + 40)
+    toks, lens = oracle.gen_tokens(seed, 1, B * S, cfg["vocab"]).reshape(B, S), np.array(lens, np.int32)
+    want = st.prefill(toks, lens)
+    # the same prompts in two portions: the second one's rows see keys that are in the cache
+    head = np.maximum(1, lens // 3).astype(np.int32)
+    rest = lens - head
+    kv.prefill(toks, head)
+    if (rest > 0).all():
+        tail = np.zeros_like(toks)
+        for b in range(B):
+            tail[b, :rest[b]] = toks[b, head[b]:lens[b]]
+        _, logits = kv.prefill(tail, rest, want_logits=True)
+    else:
+        kv.reset()
+        _, logits = kv.prefill(toks, lens, want_logits=True)
+    # fp32 on both sides: logits of size 1, a few hundred roundings apart
+    assert np.abs(logits - want).max() < 2e-5
+    for _ in range(34):
+        ids = oracle.argmax(want)
+        _, logits = kv.decode_step(ids, want_logits=True)
+        want = st.decode(ids)
+        assert np.abs(logits - want).max() < 2e-5
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
