@@ -641,110 +641,6 @@ __global__ void __launch_bounds__(1024) attn_combine_decode_kernel(const float* 
   SB_TRACE_END(SB_K_COMBINE, 0);
 }
 
-// ------------------------------------------------------------------ fp32 attention (GPT-2 path)
-__global__ void kv_append_f32_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
-                                     const int32_t* __restrict__ seq, const int32_t* __restrict__ pos, const int32_t* __restrict__ lens, int H,
-                                     int Dh, int maxlen) {
-  pdl_trigger();
-  pdl_wait();
-  int64_t t = blockIdx.x;
-  int b = seq ? seq[t] : (int)t;
-  int p = pos ? pos[t] : lens[b];
-  if (p < 0 || p >= maxlen) return;
-  int hd = H * Dh;
-  for (int e = threadIdx.x; e < hd; e += blockDim.x) {
-    int h = e / Dh, d = e - h * Dh;
-    int64_t dst = (((int64_t)b * H + h) * maxlen + p) * Dh + d;
-    kc[dst] = qkv[t * 3 * hd + hd + e];
-    vc[dst] = qkv[t * 3 * hd + 2 * hd + e];
-  }
-}
-// grid (H, T), 256 threads; scores of one (token, head) live in shared memory.
-__global__ void __launch_bounds__(256) attn_f32_kernel(const float* __restrict__ qkv, const float* __restrict__ kc, const float* __restrict__ vc,
-                                                       const int32_t* __restrict__ seq, const int32_t* __restrict__ pos,
-                                                       const int32_t* __restrict__ lens, int H, int Dh, int maxlen, float scale,
-                                                       float* __restrict__ out, float* kc_new, float* vc_new) {
-  // kc_new/vc_new (decode: every row is its own sequence) make this block also append its head's
-  // new key and value; it then takes position p from the projection output, not from the cache.
-  pdl_trigger();
-  pdl_wait();
-  extern __shared__ __align__(16) float sc[];  // [maxlen rounded up to 4] scores, [Dh] query, [blockDim.x] float4 partial rows
-  __shared__ float red[32];
-  int h = blockIdx.x;
-  int64_t t = blockIdx.y;
-  int b = seq ? seq[t] : (int)t;
-  int p = pos ? pos[t] : lens[b];
-  if (p < 0 || p >= maxlen) return;
-  int n = p + 1;
-  float* qs = sc + ((maxlen + 3) & ~3);
-  int hd = H * Dh;
-  for (int d = threadIdx.x; d < Dh; d += blockDim.x) qs[d] = qkv[t * 3 * hd + h * Dh + d];
-  __syncthreads();
-  const float* kb = kc + ((int64_t)b * H + h) * maxlen * Dh;
-  const float* vb = vc + ((int64_t)b * H + h) * maxlen * Dh;
-  const float* k_own = qkv + t * 3 * hd + hd + h * Dh;
-  const float* v_own = k_own + hd;
-  const int own = kc_new ? p : -1;
-  if (kc_new)
-    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
-      const int64_t dst = (((int64_t)b * H + h) * maxlen + p) * Dh + d;
-      kc_new[dst] = k_own[d];
-      vc_new[dst] = v_own[d];
-    }
-  float mx = -INFINITY;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const float4* kr = (const float4*)(j == own ? k_own : kb + (int64_t)j * Dh);
-    float acc = 0.f;
-    for (int d4 = 0; d4 < Dh / 4; d4++) {
-      float4 kv = kr[d4];
-      acc += kv.x * qs[4 * d4] + kv.y * qs[4 * d4 + 1] + kv.z * qs[4 * d4 + 2] + kv.w * qs[4 * d4 + 3];
-    }
-    acc *= scale;
-    sc[j] = acc;
-    mx = fmaxf(mx, acc);
-  }
-  mx = block_max(mx, red);
-  float l = 0.f;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    float e = expf(sc[j] - mx);
-    sc[j] = e;
-    l += e;
-  }
-  l = block_sum(l, red);
-  __syncthreads();
-  float inv = 1.0f / l;
-  // P.V: the block's threads form groups of Dh/4 lanes; group g adds the keys g, g+G, ... with one
-  // float4 of the value row per lane (a single query row would otherwise walk all keys on Dh
-  // threads, one dependent step per key), then the groups' partial rows are added in group order.
-  const int dl = Dh / 4, G = (int)blockDim.x / dl;
-  float* part = qs + Dh;  // [blockDim.x] float4
-  if (G >= 1) {
-    const int g = (int)threadIdx.x / dl, c = (int)threadIdx.x % dl;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (g < G) {
-#pragma unroll 8
-      for (int j = g; j < n; j += G) {
-        const float4 v = *(const float4*)((j == own ? v_own : vb + (int64_t)j * Dh) + 4 * c);
-        const float pj = sc[j];
-        acc.x += pj * v.x; acc.y += pj * v.y; acc.z += pj * v.z; acc.w += pj * v.w;
-      }
-    }
-    *(float4*)(part + 4 * threadIdx.x) = acc;
-    __syncthreads();
-    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
-      float o = 0.f;
-      for (int gg = 0; gg < G; gg++) o += part[(gg * dl + d / 4) * 4 + (d & 3)];
-      out[t * hd + h * Dh + d] = o * inv;
-    }
-  } else {  // head wider than four times the block: one thread per output column
-    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
-      float acc = 0.f;
-      for (int j = 0; j < n; j++) acc += sc[j] * (j == own ? v_own[d] : vb[(int64_t)j * Dh + d]);
-      out[t * hd + h * Dh + d] = acc * inv;
-    }
-  }
-}
-
 }  // namespace
 
 int k_attn_prefill_tc(strictb200_ctx* ctx, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, const int32_t* past,
@@ -885,38 +781,6 @@ int k_attn_decode(strictb200_ctx* ctx, const bf16* q, const bf16* kc, const bf16
     return STRICTB200_OK;
   }
   SB_CUDA(sb_launch(ctx, attn_combine_kernel, dim3(B), dim3(CB_THREADS), 0, o_part, ml_part, lens, len_add, Hq, maxlen, chunk, nsplit, out, q_out, qscale_out));
-  ctx->launches++;
-  return STRICTB200_OK;
-}
-
-int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, const int32_t* seq, const int32_t* pos, const int32_t* lens,
-               int64_t T, int H, int Dh, int maxlen, float scale, float* out) {
-  if (Dh % 4) return sb_fail(STRICTB200_ERR_INVALID_ARG, "attention: head_dim must be a multiple of 4");
-  const int threads = 256;
-  size_t smem = ((size_t)((maxlen + 3) & ~3) + Dh + 4 * threads) * sizeof(float);
-  if (smem > 200 * 1024) return sb_fail(STRICTB200_ERR_UNSUPPORTED, "attention: fp32 path supports at most ~50k positions");
-  {
-    static std::mutex mu;
-    static size_t attr_smem[64] = {};  // largest size this device's kernel has been opened for
-    std::lock_guard<std::mutex> lock(mu);
-    size_t& have = attr_smem[ctx->device & 63];
-    if (have < 48 * 1024) have = 48 * 1024;
-    if (smem > have) {
-      SB_CUDA(cudaFuncSetAttribute(attn_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      have = smem;
-    }
-  }
-  if (T > 65535) return sb_fail(STRICTB200_ERR_INVALID_ARG, "attention: too many rows for the fp32 path");
-  // rows that are sequences of their own (decode) append inside the attention kernel; prompt rows
-  // need the keys of other rows of their sequence, so those are appended by a kernel of its own first
-  const bool fused_append = seq == nullptr;
-  if (!fused_append) {
-    SB_CUDA(sb_launch(ctx, kv_append_f32_kernel, dim3((unsigned)T), dim3(256), 0, qkv, kc, vc, seq, pos, lens, H, Dh, maxlen));
-    ctx->launches++;
-  }
-  dim3 grid(H, (unsigned)T);
-  SB_CUDA(sb_launch(ctx, attn_f32_kernel, grid, dim3(threads), smem, (const float*)qkv, (const float*)kc, (const float*)vc, seq, pos, lens, H, Dh, maxlen,
-                    scale, out, fused_append ? kc : (float*)nullptr, fused_append ? vc : (float*)nullptr));
   ctx->launches++;
   return STRICTB200_OK;
 }

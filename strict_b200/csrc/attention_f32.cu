@@ -1,0 +1,368 @@
+// fp32 attention of the GPT-2 path: prompts in tiles, decode rows with the keys spread over half-warps, and a kernel for any head width.
+#include "common.cuh"
+
+namespace {
+__global__ void kv_append_f32_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
+                                     const int32_t* __restrict__ seq, const int32_t* __restrict__ pos, const int32_t* __restrict__ lens, int H,
+                                     int Dh, int maxlen) {
+  pdl_trigger();
+  pdl_wait();
+  int64_t t = blockIdx.x;
+  int b = seq ? seq[t] : (int)t;
+  int p = pos ? pos[t] : lens[b];
+  if (p < 0 || p >= maxlen) return;
+  int hd = H * Dh;
+  for (int e = threadIdx.x; e < hd; e += blockDim.x) {
+    int h = e / Dh, d = e - h * Dh;
+    int64_t dst = (((int64_t)b * H + h) * maxlen + p) * Dh + d;
+    kc[dst] = qkv[t * 3 * hd + hd + e];
+    vc[dst] = qkv[t * 3 * hd + 2 * hd + e];
+  }
+}
+// Any head width. grid (H, T), 256 threads; scores of one (token, head) live in shared memory.
+__global__ void __launch_bounds__(256) attn_f32_kernel(const float* __restrict__ qkv, const float* __restrict__ kc, const float* __restrict__ vc,
+                                                       const int32_t* __restrict__ seq, const int32_t* __restrict__ pos,
+                                                       const int32_t* __restrict__ lens, int H, int Dh, int maxlen, float scale,
+                                                       float* __restrict__ out, float* kc_new, float* vc_new) {
+  // kc_new/vc_new (decode: every row is its own sequence) make this block also append its head's
+  // new key and value; it then takes position p from the projection output, not from the cache.
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) float sc[];  // [maxlen rounded up to 4] scores, [Dh] query, [blockDim.x] float4 partial rows
+  __shared__ float red[32];
+  int h = blockIdx.x;
+  int64_t t = blockIdx.y;
+  int b = seq ? seq[t] : (int)t;
+  int p = pos ? pos[t] : lens[b];
+  if (p < 0 || p >= maxlen) return;
+  int n = p + 1;
+  float* qs = sc + ((maxlen + 3) & ~3);
+  int hd = H * Dh;
+  for (int d = threadIdx.x; d < Dh; d += blockDim.x) qs[d] = qkv[t * 3 * hd + h * Dh + d];
+  __syncthreads();
+  const float* kb = kc + ((int64_t)b * H + h) * maxlen * Dh;
+  const float* vb = vc + ((int64_t)b * H + h) * maxlen * Dh;
+  const float* k_own = qkv + t * 3 * hd + hd + h * Dh;
+  const float* v_own = k_own + hd;
+  const int own = kc_new ? p : -1;
+  if (kc_new)
+    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
+      const int64_t dst = (((int64_t)b * H + h) * maxlen + p) * Dh + d;
+      kc_new[dst] = k_own[d];
+      vc_new[dst] = v_own[d];
+    }
+  float mx = -INFINITY;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const float4* kr = (const float4*)(j == own ? k_own : kb + (int64_t)j * Dh);
+    float acc = 0.f;
+    for (int d4 = 0; d4 < Dh / 4; d4++) {
+      float4 kv = kr[d4];
+      acc += kv.x * qs[4 * d4] + kv.y * qs[4 * d4 + 1] + kv.z * qs[4 * d4 + 2] + kv.w * qs[4 * d4 + 3];
+    }
+    acc *= scale;
+    sc[j] = acc;
+    mx = fmaxf(mx, acc);
+  }
+  mx = block_max(mx, red);
+  float l = 0.f;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    float e = expf(sc[j] - mx);
+    sc[j] = e;
+    l += e;
+  }
+  l = block_sum(l, red);
+  __syncthreads();
+  float inv = 1.0f / l;
+  // P.V: the block's threads form groups of Dh/4 lanes; group g adds the keys g, g+G, ... with one
+  // float4 of the value row per lane (a single query row would otherwise walk all keys on Dh
+  // threads, one dependent step per key), then the groups' partial rows are added in group order.
+  const int dl = Dh / 4, G = (int)blockDim.x / dl;
+  float* part = qs + Dh;  // [blockDim.x] float4
+  if (G >= 1) {
+    const int g = (int)threadIdx.x / dl, c = (int)threadIdx.x % dl;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g < G) {
+#pragma unroll 8
+      for (int j = g; j < n; j += G) {
+        const float4 v = *(const float4*)((j == own ? v_own : vb + (int64_t)j * Dh) + 4 * c);
+        const float pj = sc[j];
+        acc.x += pj * v.x; acc.y += pj * v.y; acc.z += pj * v.z; acc.w += pj * v.w;
+      }
+    }
+    *(float4*)(part + 4 * threadIdx.x) = acc;
+    __syncthreads();
+    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
+      float o = 0.f;
+      for (int gg = 0; gg < G; gg++) o += part[(gg * dl + d / 4) * 4 + (d & 3)];
+      out[t * hd + h * Dh + d] = o * inv;
+    }
+  } else {  // head wider than four times the block: one thread per output column
+    for (int d = threadIdx.x; d < Dh; d += blockDim.x) {
+      float acc = 0.f;
+      for (int j = 0; j < n; j++) acc += sc[j] * (j == own ? v_own[d] : vb[(int64_t)j * Dh + d]);
+      out[t * hd + h * Dh + d] = acc * inv;
+    }
+  }
+}
+
+
+// ------------------------------------------------------------------ prompts, 64-dim heads
+// One block: 64 queries of a sequence and one head, over 64 keys at a time with a running maximum. Bound by the fp32 FMA pipe (two
+// 64 x 64 x 64 products per tile and block, 4 x 4 results per thread and eight 128-bit shared-memory reads per 64 FMAs). A tile's sums
+// start from zero and are added to the running ones once, so that a long row is not one long chain of additions.
+// Prompts of 300 to 901 tokens, batch 8: 1405 us per layer with one block per row and head, 195 us here.
+constexpr int PT = 64, PD = 64, PS = PD + 4;  // queries and keys per tile, head dims, row stride in shared memory
+constexpr int PROMPT_SMEM = 4 * PT * PS * 4;
+__global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* __restrict__ qkv, const float* __restrict__ kc, const float* __restrict__ vc,
+                                                              const int32_t* __restrict__ qstart, const int32_t* __restrict__ past,
+                                                              const int32_t* __restrict__ after, int b0, int H, int maxlen, float scale,
+                                                              float* __restrict__ out) {
+  extern __shared__ __align__(16) float ps[];
+  float *qs = ps, *ks = ps + PT * PS, *vs = ks + PT * PS, *pr = vs + PT * PS;
+  pdl_trigger();
+  pdl_wait();
+  const int j = blockIdx.z, h = blockIdx.y, q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * PT;  // the longest rows first
+  const int p0 = past[j], n_new = after[j] - p0;
+  if (q0 >= n_new) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, hd = H * PD;
+  const int64_t row0 = qstart[j] + q0;
+  const float* kb = kc + ((int64_t)(b0 + j) * H + h) * maxlen * PD;
+  const float* vb = vc + ((int64_t)(b0 + j) * H + h) * maxlen * PD;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // thread: columns 4 tx.. of the rows ty, ty + 16, ...
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int r = ty + 16 * i;
+    *(float4*)(qs + r * PS + 4 * tx) = q0 + r < n_new ? *(const float4*)(qkv + (row0 + r) * 3 * hd + h * PD + 4 * tx) : zero;
+  }
+  const int n_keys = p0 + min(q0 + PT, n_new);
+  float4 rk[4], rv[4];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int k = k0 + ty + 16 * i;
+      rk[i] = k < n_keys ? *(const float4*)(kb + (int64_t)k * PD + 4 * tx) : zero;
+      rv[i] = k < n_keys ? *(const float4*)(vb + (int64_t)k * PD + 4 * tx) : zero;
+    }
+  };
+  load(0);
+  float o[4][4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    m[i] = -INFINITY; l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; c++) o[i][c] = 0.f;
+  }
+  for (int k0 = 0; k0 < n_keys; k0 += PT) {
+    __syncthreads();  // the last tile's keys and values have been read
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      *(float4*)(ks + (ty + 16 * i) * PS + 4 * tx) = rk[i];
+      *(float4*)(vs + (ty + 16 * i) * PS + 4 * tx) = rv[i];
+    }
+    __syncthreads();
+    if (k0 + PT < n_keys) load(k0 + PT);
+    // scores of the rows 4 ty + i and the keys k0 + tx + 16 c
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) s[i][c] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < PD; d += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = *(const float4*)(qs + (4 * ty + i) * PS + d);
+#pragma unroll
+      for (int c = 0; c < 4; c++) b[c] = *(const float4*)(ks + (tx + 16 * c) * PS + d);
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) s[i][c] = fmaf(a[i].w, b[c].w, fmaf(a[i].z, b[c].z, fmaf(a[i].y, b[c].y, fmaf(a[i].x, b[c].x, s[i][c]))));
+    }
+    __syncwarp();  // the warp's own rows of the weights have been read
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int last = p0 + q0 + 4 * ty + i - k0;  // keys up to here are visible
+      float mx = m[i];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        s[i][c] *= scale;
+        if (tx + 16 * c <= last) mx = fmaxf(mx, s[i][c]);
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+      const float alpha = expf(m[i] - mx);
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float e = tx + 16 * c <= last ? expf(s[i][c] - mx) : 0.f;
+        pr[(4 * ty + i) * PS + tx + 16 * c] = e;
+        sum += e;
+      }
+      l[i] = fmaf(l[i], alpha, sum);
+      m[i] = mx;
+#pragma unroll
+      for (int c = 0; c < 4; c++) { o[i][c] *= alpha; s[i][c] = 0.f; }
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int k = 0; k < PT; k += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = *(const float4*)(pr + (4 * ty + i) * PS + k);
+#pragma unroll
+      for (int c = 0; c < 4; c++) b[c] = *(const float4*)(vs + (k + c) * PS + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        s[i][0] = fmaf(a[i].w, b[3].x, fmaf(a[i].z, b[2].x, fmaf(a[i].y, b[1].x, fmaf(a[i].x, b[0].x, s[i][0]))));
+        s[i][1] = fmaf(a[i].w, b[3].y, fmaf(a[i].z, b[2].y, fmaf(a[i].y, b[1].y, fmaf(a[i].x, b[0].y, s[i][1]))));
+        s[i][2] = fmaf(a[i].w, b[3].z, fmaf(a[i].z, b[2].z, fmaf(a[i].y, b[1].z, fmaf(a[i].x, b[0].z, s[i][2]))));
+        s[i][3] = fmaf(a[i].w, b[3].w, fmaf(a[i].z, b[2].w, fmaf(a[i].y, b[1].w, fmaf(a[i].x, b[0].w, s[i][3]))));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) o[i][c] += s[i][c];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], w);
+    const int r = 4 * ty + i;
+    if (q0 + r < n_new) {
+      const float inv = 1.0f / l[i];
+      *(float4*)(out + (row0 + r) * hd + h * PD + 4 * tx) = make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ decode rows, heads of 4 LANES dims
+// One block per row and head, and it appends the row's key and value to the cache. LANES lanes share a key (one 128-bit load of the
+// key and one of the value per lane), each such group walks every GROUPS-th key with a running maximum and its own sum, eight keys'
+// loads in flight; the groups meet in shared memory. Bound by the latency of those loads: 144 keys on average took 13.6 us of a GPT-2 step
+// with a key per thread and a second pass for the values, 3.7 us here.
+template <int LANES>
+__global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* __restrict__ qkv, float* kc, float* vc, const int32_t* __restrict__ lens, int H,
+                                                              int maxlen, float scale, float* __restrict__ out) {
+  constexpr int D = 4 * LANES, GROUPS = 512 / LANES, BATCH = 8;
+  __shared__ float red_m[GROUPS], red_l[GROUPS];
+  __shared__ __align__(16) float red_o[GROUPS][D];
+  pdl_trigger();
+  const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x % LANES, grp = threadIdx.x / LANES, hd = H * D;
+  float* kb = kc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
+  float* vb = vc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
+  pdl_wait();
+  const int p = lens[b];
+  if (p < 0 || p >= maxlen) return;
+  const float* row = qkv + (int64_t)b * 3 * hd + h * D + 4 * c;
+  const float4 q = *(const float4*)row, k_own = *(const float4*)(row + hd), v_own = *(const float4*)(row + 2 * hd);
+  if (grp == 0) {
+    *(float4*)(kb + (int64_t)p * D) = k_own;
+    *(float4*)(vb + (int64_t)p * D) = v_own;
+  }
+  float m = -INFINITY, l = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int base = 0; base <= p; base += BATCH * GROUPS) {  // the same number of rounds for every group: their lanes share warps, and shuffles
+    const int j0 = base + grp;
+    float4 k[BATCH], v[BATCH];
+#pragma unroll
+    for (int i = 0; i < BATCH; i++) {
+      const int j = j0 + i * GROUPS;
+      if (j < p) {
+        k[i] = *(const float4*)(kb + (int64_t)j * D);
+        v[i] = *(const float4*)(vb + (int64_t)j * D);
+      } else {
+        k[i] = k_own;
+        v[i] = v_own;
+      }
+    }
+    float s[BATCH], mx = m;
+#pragma unroll
+    for (int i = 0; i < BATCH; i++) {
+      s[i] = fmaf(k[i].w, q.w, fmaf(k[i].z, q.z, fmaf(k[i].y, q.y, k[i].x * q.x)));
+#pragma unroll
+      for (int w = LANES / 2; w > 0; w >>= 1) s[i] += __shfl_xor_sync(0xffffffffu, s[i], w, LANES);
+      s[i] *= scale;
+      if (j0 + i * GROUPS <= p) mx = fmaxf(mx, s[i]);
+    }
+    const float alpha = expf(m - mx);
+    m = mx;
+    l *= alpha;
+    o.x *= alpha; o.y *= alpha; o.z *= alpha; o.w *= alpha;
+#pragma unroll
+    for (int i = 0; i < BATCH; i++) {
+      if (j0 + i * GROUPS <= p) {
+        const float e = expf(s[i] - mx);
+        l += e;
+        o.x = fmaf(e, v[i].x, o.x); o.y = fmaf(e, v[i].y, o.y); o.z = fmaf(e, v[i].z, o.z); o.w = fmaf(e, v[i].w, o.w);
+      }
+    }
+  }
+  if (c == 0) { red_m[grp] = m; red_l[grp] = l; }
+  *(float4*)&red_o[grp][4 * c] = o;
+  __syncthreads();
+  if (threadIdx.x < D) {
+    const int n = min(GROUPS, p + 1);  // groups that have seen a key
+    float mx = red_m[0];
+    for (int g = 1; g < n; g++) mx = fmaxf(mx, red_m[g]);
+    float sum = 0.f, acc = 0.f;
+    for (int g = 0; g < n; g++) {
+      const float e = expf(red_m[g] - mx);
+      sum = fmaf(e, red_l[g], sum);
+      acc = fmaf(e, red_o[g][threadIdx.x], acc);
+    }
+    out[(int64_t)b * hd + h * D + threadIdx.x] = acc * (1.0f / sum);
+  }
+}
+}  // namespace
+
+int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, const int32_t* seq, const int32_t* pos, const int32_t* lens,
+               int64_t T, int H, int Dh, int maxlen, float scale, float* out, const F32Prompts* prompts) {
+  if (Dh % 4) return sb_fail(STRICTB200_ERR_INVALID_ARG, "attention: head_dim must be a multiple of 4");
+  const bool rows16 = (((uintptr_t)qkv | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) & 15) == 0;
+  if (!seq && rows16 && (Dh == 32 || Dh == 64 || Dh == 128) && T <= 65535) {  // rows that are sequences of their own
+    auto kernel = Dh == 32 ? attn_f32_decode_kernel<8> : Dh == 64 ? attn_f32_decode_kernel<16> : attn_f32_decode_kernel<32>;
+    SB_CUDA(sb_launch(ctx, kernel, dim3((unsigned)H, (unsigned)T), dim3(512), 0, qkv, kc, vc, lens, H, maxlen, scale, out));
+    ctx->launches++;
+    return STRICTB200_OK;
+  }
+  if (seq && prompts && rows16 && Dh == PD && T <= 65535 && prompts->nb <= 65535 && H <= 65535) {
+    SB_CUDA(sb_launch(ctx, kv_append_f32_kernel, dim3((unsigned)T), dim3(256), 0, qkv, kc, vc, seq, pos, lens, H, Dh, maxlen));
+    ctx->launches++;
+    static SbDeviceOnce once;
+    SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(attn_f32_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PROMPT_SMEM); }));
+    SB_CUDA(sb_launch(ctx, attn_f32_prompt_kernel, dim3((unsigned)((prompts->max_new + PT - 1) / PT), (unsigned)H, (unsigned)prompts->nb), dim3(256), (size_t)PROMPT_SMEM,
+                      (const float*)qkv, (const float*)kc, (const float*)vc, prompts->qstart, prompts->past, prompts->after, prompts->b0, H, maxlen, scale, out));
+    ctx->launches++;
+    return STRICTB200_OK;
+  }
+  const int threads = 256;
+  size_t smem = ((size_t)((maxlen + 3) & ~3) + Dh + 4 * threads) * sizeof(float);
+  if (smem > 200 * 1024) return sb_fail(STRICTB200_ERR_UNSUPPORTED, "attention: fp32 path supports at most ~50k positions");
+  {
+    static std::mutex mu;
+    static size_t attr_smem[64] = {};  // largest size this device's kernel has been opened for
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& have = attr_smem[ctx->device & 63];
+    if (have < 48 * 1024) have = 48 * 1024;
+    if (smem > have) {
+      SB_CUDA(cudaFuncSetAttribute(attn_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      have = smem;
+    }
+  }
+  if (T > 65535) return sb_fail(STRICTB200_ERR_INVALID_ARG, "attention: too many rows for the fp32 path");
+  // rows that are sequences of their own (decode) append inside the attention kernel; prompt rows
+  // need the keys of other rows of their sequence, so those are appended by a kernel of its own first
+  const bool fused_append = seq == nullptr;
+  if (!fused_append) {
+    SB_CUDA(sb_launch(ctx, kv_append_f32_kernel, dim3((unsigned)T), dim3(256), 0, qkv, kc, vc, seq, pos, lens, H, Dh, maxlen));
+    ctx->launches++;
+  }
+  dim3 grid(H, (unsigned)T);
+  SB_CUDA(sb_launch(ctx, attn_f32_kernel, grid, dim3(threads), smem, (const float*)qkv, (const float*)kc, (const float*)vc, seq, pos, lens, H, Dh, maxlen,
+                    scale, out, fused_append ? kc : (float*)nullptr, fused_append ? vc : (float*)nullptr));
+  ctx->launches++;
+  return STRICTB200_OK;
+}

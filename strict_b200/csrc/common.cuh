@@ -567,8 +567,13 @@ int k_attn_decode(strictb200_ctx*, const bf16* q, const bf16* kc, const bf16* vc
                   const RopeArgs* rope = nullptr, int chunk = 0);
 int k_attn_decode_chunks(strictb200_ctx*, int HD, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, int B, int Hq, int Hkv, int maxlen,
                          float scale, int nsplit, int chunk, float* o_part, float* ml_part);
+// attention_f32.cu. `prompts` (with seq and pos): the rows as sequences b0.. of the cache, one after the other
+struct F32Prompts {
+  const int32_t *qstart = nullptr, *past = nullptr, *after = nullptr;  // [nb] first row, length of the cache before and after these rows
+  int b0 = 0, nb = 0, max_new = 0;
+};
 int k_attn_f32(strictb200_ctx*, const float* qkv, float* kc, float* vc, const int32_t* seq, const int32_t* pos, const int32_t* lens,
-               int64_t T, int H, int D, int maxlen, float scale, float* out);
+               int64_t T, int H, int D, int maxlen, float scale, float* out, const F32Prompts* prompts = nullptr);
 // sampling.cu
 int k_embedding_bf16(strictb200_ctx*, const bf16* table, const int32_t* ids, int64_t T, int64_t d, int64_t vocab, bf16* out);
 int k_embedding_bf16_f32(strictb200_ctx*, const bf16* table, const int32_t* ids, int64_t T, int64_t d, int64_t vocab, float* out);

@@ -261,7 +261,7 @@ int qwen_decode_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
 // xf [T,d] must already hold wte[id]+wpe[pos]. seq/pos may be null for decode (row t = sequence
 // t at position lens[t]).
 int gpt2_layers(strictb200_model* m, strictb200_kv* kv, int64_t T, float* xf, float* af, float* bf_, const int32_t* seq,
-                const int32_t* pos) {
+                const int32_t* pos, const F32Prompts* prompts) {
   strictb200_ctx* ctx = m->ctx;
   const auto& c = m->c;
   const int64_t d = c.d_model;
@@ -270,7 +270,7 @@ int gpt2_layers(strictb200_model* m, strictb200_kv* kv, int64_t T, float* xf, fl
     LayerW& w = m->L[l];
     SB_TRY(k_layernorm(ctx, xf, w.norm1_g, w.norm1_b, c.eps, T, d, af));
     SB_TRY(k_gemm_f32(ctx, T, 3 * d, d, af, w.fqkv.w, w.fqkv.b, bf_, 0));
-    SB_TRY(k_attn_f32(ctx, bf_, kv_kf(kv, l), kv_vf(kv, l), seq, pos, kv->d_lens, T, c.n_q_heads, c.head_dim, kv->maxlen, scale, af));
+    SB_TRY(k_attn_f32(ctx, bf_, kv_kf(kv, l), kv_vf(kv, l), seq, pos, kv->d_lens, T, c.n_q_heads, c.head_dim, kv->maxlen, scale, af, prompts));
     SB_TRY(k_gemm_f32(ctx, T, d, d, af, w.fo.w, w.fo.b, xf, 1));
     SB_TRY(k_layernorm(ctx, xf, w.norm2_g, w.norm2_b, c.eps, T, d, af));
     SB_TRY(k_gemm_f32(ctx, T, c.d_ff, d, af, w.ffc.w, w.ffc.b, bf_, 2));  // GELU in the epilogue
@@ -284,7 +284,7 @@ int gpt2_decode_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
   const auto& c = m->c;
   const int64_t B = kv->B, d = c.d_model;
   SB_TRY(k_embedding_f32(ctx, m->wte, m->wpe, kv->d_ids, nullptr, kv->d_lens, B, d, c.vocab, c.max_pos, b.xf));
-  SB_TRY(gpt2_layers(m, kv, B, b.xf, b.af, b.bf, nullptr, nullptr));
+  SB_TRY(gpt2_layers(m, kv, B, b.xf, b.af, b.bf, nullptr, nullptr, nullptr));
   SB_TRY(k_layernorm(ctx, b.xf, m->normf_g, m->normf_b, c.eps, B, d, b.af));
   SB_TRY(k_gemm_f32(ctx, B, c.vocab, d, b.af, m->wte, nullptr, b.logits, 0));
   SB_TRY(k_argmax(ctx, b.logits, B, c.vocab, c.vocab, kv->d_next, nullptr, b.am_ws));
@@ -493,7 +493,10 @@ int gpt2_prefill_chunk(strictb200_model* m, strictb200_kv* kv, const PrefillChun
   const int64_t d = c.d_model;
   float *xf = cb.xf, *af = cb.af, *bf_ = cb.bf_, *last = cb.last, *lastn = cb.lastn, *logits = cb.logits;
   SB_TRY(k_embedding_f32(ctx, m->wte, m->wpe, pc.ix.tok, pc.ix.pos, nullptr, T, d, c.vocab, c.max_pos, xf));
-  SB_TRY(gpt2_layers(m, kv, T, xf, af, bf_, pc.ix.seq, pc.ix.pos));
+  F32Prompts prompts;
+  prompts.qstart = pc.ix.qs; prompts.past = pc.ix.past; prompts.after = pc.ix.la;
+  prompts.b0 = pc.b0; prompts.nb = pc.nb; prompts.max_new = pc.max_new;
+  SB_TRY(gpt2_layers(m, kv, T, xf, af, bf_, pc.ix.seq, pc.ix.pos, &prompts));
   SB_TRY(k_gather_rows(ctx, xf, pc.ix.last, n_rows, d * 4, last));
   SB_TRY(k_layernorm(ctx, last, m->normf_g, m->normf_b, c.eps, n_rows, d, lastn));
   SB_TRY(k_gemm_f32(ctx, n_rows, c.vocab, d, lastn, m->wte, nullptr, logits, 0));
