@@ -303,6 +303,9 @@ struct GemmArgs {
   int i8 = 0;                   // 1: int8 weights and two int8 activation terms (gemm_int8.cu); part then holds int32 sums [splits][2][M,N]
 };
 int k_gemm_fp8(strictb200_ctx*, const GemmArgs& a);
+// many tokens: W = [gate | up], out = bf16 silu(gate) * up [M, N / 2] (gemm_tmem_pair.cu)
+bool sb_gemm_fp8_swiglu_fits(strictb200_ctx*, int64_t M, int64_t N, int64_t K);
+int k_gemm_fp8_swiglu(strictb200_ctx*, const GemmArgs& a);
 int sb_gemm_pick_splits(strictb200_ctx*, int64_t M, int64_t N, int64_t K);
 int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
 // gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
