@@ -1,4 +1,6 @@
 // fp32 attention of the GPT-2 path: prompts in tiles, decode rows with the keys spread over half-warps, and a kernel for any head width.
+// Inputs that another kernel of the chain writes are not declared __restrict__ in the kernels below: loads of invariant data may be
+// moved in front of the dependency wait.
 #include "common.cuh"
 
 namespace {
@@ -113,10 +115,10 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(const float* __restrict__
 // Prompts of 300 to 901 tokens, batch 8: 1405 us per layer with one block per row and head, 195 us here.
 constexpr int PT = 64, PD = 64, PS = PD + 4;  // queries and keys per tile, head dims, row stride in shared memory
 constexpr int PROMPT_SMEM = 4 * PT * PS * 4;
-__global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* __restrict__ qkv, const float* __restrict__ kc, const float* __restrict__ vc,
+__global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* qkv, const float* kc, const float* vc,
                                                               const int32_t* __restrict__ qstart, const int32_t* __restrict__ past,
                                                               const int32_t* __restrict__ after, int b0, int H, int maxlen, float scale,
-                                                              float* __restrict__ out) {
+                                                              float* out) {
   extern __shared__ __align__(16) float ps[];
   float *qs = ps, *ks = ps + PT * PS, *vs = ks + PT * PS, *pr = vs + PT * PS;
   pdl_trigger();
@@ -244,8 +246,8 @@ __global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* __res
 // loads in flight; the groups meet in shared memory. Bound by the latency of those loads: 144 keys on average took 13.6 us of a GPT-2 step
 // with a key per thread and a second pass for the values, 3.7 us here.
 template <int LANES>
-__global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* __restrict__ qkv, float* kc, float* vc, const int32_t* __restrict__ lens, int H,
-                                                              int maxlen, float scale, float* __restrict__ out) {
+__global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, float* kc, float* vc, const int32_t* lens, int H,
+                                                              int maxlen, float scale, float* out) {
   constexpr int D = 4 * LANES, GROUPS = 512 / LANES, BATCH = 8;
   __shared__ float red_m[GROUPS], red_l[GROUPS];
   __shared__ __align__(16) float red_o[GROUPS][D];

@@ -356,8 +356,11 @@ struct GemmF32Args {
   float act_pos = 0.f, act_neg = 0.f;
   const float* col_scale = nullptr;
   float alpha = 1.f;
+  const float *ln_gain = nullptr, *ln_bias = nullptr;  // layer norm of the rows of x in front of the product (sb_gemm_f32_takes_norm)
+  float ln_eps = 0.f;
 };
 int k_gemm_f32(strictb200_ctx*, const GemmF32Args& g);
+bool sb_gemm_f32_takes_norm(int64_t M, int64_t K);
 // attention.cu
 int k_attn_prefill(strictb200_ctx*, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, const int32_t* past,
                    const int32_t* qstart, int B, int S, int64_t q_rows, int Hq, int Hkv, int D, int maxlen, float scale, bf16* out);

@@ -1,6 +1,7 @@
 // fp32 linear layer of the GPT-2 path: Y[M,N] = X[M,K] . W[N,K]^T + bias. Decode (M = 1) is
-// a pure HBM stream over W; one warp (or 2-8 for a long row) per output channel, lanes split K with 128-bit loads,
-// warp-shuffle reduction. Up to 8 token rows share one pass over a weight row. `accumulate`: 0
+// a pure HBM stream over W; one warp (or 2-8 for a long row) per output channel or two, lanes split K with 128-bit loads,
+// warp-shuffle reduction. With ln_gain the rows of X are layer-normed on the way in, by every block for itself (3 KB from L2
+// against a launch of its own). Up to 8 token rows share one pass over a weight row. `accumulate`: 0
 // stores the result, 1 adds it to Y (residual), 2 stores GELU(result) (the MLP's first layer), 3 xIELU(result), 4 adds
 // alpha * col_scale[n] * result to Y.
 // Rows of X, W and Y may be wider than the product (ldx, ldw, ldy).
@@ -10,70 +11,169 @@ int k_gemm_f32_tc(strictb200_ctx* ctx, const GemmF32Args& g);  // gemm_f32_tc.cu
 
 namespace {
 constexpr int F32_MT = 8;
+constexpr int F32_PRE = 8;   // float4 of a weight row a lane fetches before the dependency wait (a slice of at most 1024 columns)
+constexpr int LN_K = 1024;   // widest row the layer norm in front of the product takes
+constexpr size_t X_SMEM = 96 * 1024;
 
-constexpr int F32_PRE = 8;  // float4 of its weight row a lane fetches before the dependency wait (covers K <= 1024)
+// Sum over the lanes of each of the n values (n a power of two, at most 16): the halves of the values change sides as the lanes are
+// folded, n - 1 + log2(32 / n) shuffles instead of 5 n. Lane l returns the sum of the value whose index is the top log2(n) bits of l.
+template <int n, int o = 16>
+__device__ __forceinline__ float fold_sums(float* v, int lane) {
+  if constexpr (n > 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n / 2; i++) {
+      const float send = up ? v[i] : v[n / 2 + i], keep = up ? v[n / 2 + i] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+    return fold_sums<n / 2, o / 2>(v, lane);
+  } else if constexpr (o > 0) {
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return fold_sums<1, o / 2>(v, lane);
+  } else {
+    return v[0];
+  }
+}
 
-__global__ void __launch_bounds__(256) gemm_f32_kernel(int M, int N, int K, const float* __restrict__ x, int64_t ldx, const float* __restrict__ w,
-                                                       int64_t ldw, const float* __restrict__ bias, float* __restrict__ y, int64_t ldy, int accumulate, int ks,
-                                                       float act_pos, float act_neg, const float* __restrict__ col_scale, float alpha) {
-  // The block's 8 warps are 8/ks output channels x ks slices of K: a long row (K > 1024) is
-  // walked by several warps at once so that every lane still has all its loads in flight in one
-  // round trip; the slices' sums meet in shared memory and are added in slice order.
-  __shared__ float part[8][F32_MT];
+// MT rows at most, NC channels per warp. The block's 8 warps are 8/ks groups of NC channels x ks slices of K: a long row is walked by
+// several warps at once so that every lane has all its weight loads in flight in one round trip; the slices' sums meet in shared
+// memory and are added in slice order. STAGED: the rows of X (or their layer norm, LN) are in shared memory. X is read from L2 and is
+// not declared invariant: loads of invariant data may be moved in front of the dependency wait.
+template <int MT, int NC, bool STAGED, bool LN>
+__global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, const float* x, int64_t ldx, const float* __restrict__ w,
+                                                       int64_t ldw, const float* __restrict__ bias, float* y, int64_t ldy, int accumulate, int ks,
+                                                       float act_pos, float act_neg, const float* __restrict__ col_scale, float alpha,
+                                                       const float* __restrict__ ln_gain, const float* __restrict__ ln_bias, float ln_eps) {
+  extern __shared__ __align__(16) float xs[];
+  __shared__ float part[8][MT * NC];
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rows = 8 / ks, slice = warp % ks;
-  const int n = blockIdx.x * rows + warp / ks;
-  const int m0 = blockIdx.y * F32_MT;
-  const bool live = n < N;
+  const int groups = 8 / ks, slice = warp % ks;
+  const int n0 = (blockIdx.x * groups + warp / ks) * NC;
+  const int m0 = blockIdx.y * MT, mt = min(MT, M - m0);
   const int nk4 = K / 4, per = (nk4 + ks - 1) / ks;
   const int k4_lo = slice * per, k4_hi = min(nk4, k4_lo + per);
-  const float4* wr = (const float4*)(w + (int64_t)(live ? n : 0) * ldw);
-  // the weights are constants: the head of the slice streams in while the previous kernel still runs
-  // (streaming loads: a step reads its 0.5 GB of weights once each, and they should not push the
-  // kernels' code and the activations out of L2)
-  float4 wpre[F32_PRE];
+  // the weights are constants: the slice streams in while the previous kernel still runs (streaming loads: a step reads its
+  // 0.5 GB of weights once each, and they should not push the kernels' code and the activations out of L2)
+  float4 wpre[NC][F32_PRE];
 #pragma unroll
-  for (int i = 0; i < F32_PRE; i++)
-    if (live && k4_lo + lane + 32 * i < k4_hi) wpre[i] = __ldcs(wr + k4_lo + lane + 32 * i);
-  const float bn = bias && live ? bias[n] : 0.f;
+  for (int c = 0; c < NC; c++)
+#pragma unroll
+    for (int i = 0; i < F32_PRE; i++)
+      if (n0 + c < N && k4_lo + lane + 32 * i < k4_hi) wpre[c][i] = __ldcs((const float4*)(w + (int64_t)(n0 + c) * ldw) + k4_lo + lane + 32 * i);
+  const float4 *gain = (const float4*)xs + MT * nk4, *shift = gain + nk4;
+  if (LN) {
+    for (int i = threadIdx.x; i < nk4; i += 256) {
+      ((float4*)xs)[MT * nk4 + i] = ((const float4*)ln_gain)[i];
+      ((float4*)xs)[(MT + 1) * nk4 + i] = ((const float4*)ln_bias)[i];
+    }
+    __syncthreads();
+  }
+  const int oc = n0 + lane;  // lanes that will finish a channel
+  const float bn = bias && lane < NC && oc < N ? bias[oc] : 0.f;
   pdl_wait();
-  float acc[F32_MT];
+  if (LN) {
+    if (warp < mt) {  // a warp per row
+      const float4* xr = (const float4*)(x + (int64_t)(m0 + warp) * ldx);
+      float4 v[F32_PRE];
+      float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < F32_MT; i++) acc[i] = 0.f;
-  const int mt = min(F32_MT, M - m0);
-  auto fma_row = [&](int k4, const float4& wv) {
+      for (int i = 0; i < F32_PRE; i++)
+        if (lane + 32 * i < nk4) { v[i] = __ldcg(xr + lane + 32 * i); sum += (v[i].x + v[i].y) + (v[i].z + v[i].w); }
+      const float mean = __fdiv_rn(warp_sum(sum), (float)K);
+      float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < F32_MT; i++) {
+      for (int i = 0; i < F32_PRE; i++)
+        if (lane + 32 * i < nk4) {
+          v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+          sq += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+        }
+      const float var = __fdiv_rn(warp_sum(sq), (float)K);
+      const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, ln_eps)));
+#pragma unroll
+      for (int i = 0; i < F32_PRE; i++)
+        if (lane + 32 * i < nk4) {
+          const float4 gn = gain[lane + 32 * i], sh = shift[lane + 32 * i];
+          ((float4*)xs)[warp * nk4 + lane + 32 * i] = make_float4(__fadd_rn(__fmul_rn(__fmul_rn(v[i].x, r), gn.x), sh.x), __fadd_rn(__fmul_rn(__fmul_rn(v[i].y, r), gn.y), sh.y),
+                                                                  __fadd_rn(__fmul_rn(__fmul_rn(v[i].z, r), gn.z), sh.z), __fadd_rn(__fmul_rn(__fmul_rn(v[i].w, r), gn.w), sh.w));
+        }
+    }
+    __syncthreads();
+  } else if (STAGED) {
+    for (int i = threadIdx.x; i < mt * nk4; i += 256) ((float4*)xs)[i] = __ldcg((const float4*)(x + (int64_t)(m0 + i / nk4) * ldx) + i % nk4);
+    __syncthreads();
+  }
+  float acc[NC * MT];
+#pragma unroll
+  for (int i = 0; i < NC * MT; i++) acc[i] = 0.f;
+  auto fma_rows = [&](int k4, const float4* wv) {
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
       if (i < mt) {
-        float4 xv = *((const float4*)(x + (int64_t)(m0 + i) * ldx) + k4);
-        acc[i] += wv.x * xv.x + wv.y * xv.y + wv.z * xv.z + wv.w * xv.w;
+        const float4 xv = STAGED ? ((const float4*)xs)[i * nk4 + k4] : __ldcg((const float4*)(x + (int64_t)(m0 + i) * ldx) + k4);
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[c * MT + i] += wv[c].x * xv.x + wv[c].y * xv.y + wv[c].z * xv.z + wv[c].w * xv.w;
       }
     }
   };
-  if (live) {
 #pragma unroll
-    for (int i = 0; i < F32_PRE; i++)
-      if (k4_lo + lane + 32 * i < k4_hi) fma_row(k4_lo + lane + 32 * i, wpre[i]);
-#pragma unroll 4
-    for (int k4 = k4_lo + lane + 32 * F32_PRE; k4 < k4_hi; k4 += 32) fma_row(k4, __ldcs(wr + k4));
-  }
+  for (int i = 0; i < F32_PRE; i++)
+    if (k4_lo + lane + 32 * i < k4_hi) {
+      float4 wv[NC];
 #pragma unroll
-  for (int i = 0; i < F32_MT; i++) {
-    const float v = warp_sum(acc[i]);
-    if (lane == 0) part[warp][i] = v;
+      for (int c = 0; c < NC; c++) wv[c] = n0 + c < N ? wpre[c][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      fma_rows(k4_lo + lane + 32 * i, wv);
+    }
+#pragma unroll 2
+  for (int k4 = k4_lo + lane + 32 * F32_PRE; k4 < k4_hi; k4 += 32) {
+    float4 wv[NC];
+#pragma unroll
+    for (int c = 0; c < NC; c++) wv[c] = n0 + c < N ? __ldcs((const float4*)(w + (int64_t)(n0 + c) * ldw) + k4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    fma_rows(k4, wv);
   }
+  constexpr int VALS = NC * MT, STEP = 32 / VALS;
+  const float sum = fold_sums<VALS>(acc, lane);
+  if (lane % STEP == 0) part[warp][lane / STEP] = sum;
   __syncthreads();
-  if (live && slice == 0 && lane < mt) {
-    float v = 0.f;
-    for (int s2 = 0; s2 < ks; s2++) v += part[warp + s2][lane];
-    const int64_t o = (int64_t)(m0 + lane) * ldy + n;
-    v += bn;
-    if (accumulate == 4) { y[o] += alpha * (col_scale ? col_scale[n] : 1.f) * v; return; }
-    y[o] = accumulate == 1 ? y[o] + v : accumulate == 2 ? sb_gelu_tanh(v) : accumulate == 3 ? sb_xielu(v, act_pos, act_neg) : v;
+  if (slice == 0 && lane < NC && oc < N) {
+    for (int i = 0; i < mt; i++) {
+      float v = 0.f;
+      for (int s2 = 0; s2 < ks; s2++) v += part[warp + s2][lane * MT + i];
+      const int64_t o = (int64_t)(m0 + i) * ldy + oc;
+      v += bn;
+      if (accumulate == 4) y[o] += alpha * (col_scale ? col_scale[oc] : 1.f) * v;
+      else y[o] = accumulate == 1 ? y[o] + v : accumulate == 2 ? sb_gelu_tanh(v) : accumulate == 3 ? sb_xielu(v, act_pos, act_neg) : v;
+    }
   }
 }
+
+template <int MT, int NC, bool STAGED, bool LN>
+int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
+  const int rows = 8 / ks * NC;
+  dim3 grid((unsigned)((g.N + rows - 1) / rows), (unsigned)((g.M + MT - 1) / MT));
+  if (grid.y > 65535) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: M too large");
+  const size_t smem = LN ? (size_t)(MT + 2) * g.K * 4 : STAGED ? (size_t)MT * g.K * 4 : 0;
+  static SbDeviceOnce once;  // one per instantiation
+  SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_f32_kernel<MT, NC, STAGED, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X_SMEM); }));
+  SB_CUDA(sb_launch(ctx, gemm_f32_kernel<MT, NC, STAGED, LN>, grid, dim3(256), smem, (int)g.M, (int)g.N, (int)g.K, g.x, g.ldx, g.w, g.ldw, g.bias, g.y, g.ldy, g.mode, ks,
+                    g.act_pos, g.act_neg, g.col_scale, g.alpha, g.ln_gain, g.ln_bias, g.ln_eps));
+  ctx->launches++;
+  return STRICTB200_OK;
+}
+template <int MT, int NC>
+int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
+  if (g.ln_gain) return launch_rows<MT, NC, true, true>(ctx, g, ks);
+  // one row is a few loads per lane, straight from L2; several rows would be read once per channel
+  if (MT > 1 && (size_t)MT * g.K * 4 <= X_SMEM) return launch_rows<MT, NC, true, false>(ctx, g, ks);
+  return launch_rows<MT, NC, false, false>(ctx, g, ks);
+}
+template <int MT>
+int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks, bool two) {
+  return two ? launch_rows<MT, 2>(ctx, g, ks) : launch_rows<MT, 1>(ctx, g, ks);
+}
 }  // namespace
+
+bool sb_gemm_f32_takes_norm(int64_t M, int64_t K) { return M <= F32_MT && K <= LN_K; }
 
 int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float* x, const float* w, const float* bias, float* y,
                int accumulate) {
@@ -89,17 +189,22 @@ int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   //   N 768  K 768    7.1 / 7.1 / 13.0 /  37.8 / 1197   against   8.5 / 8.5 /  8.7 / 13.9 /  62
   //   N 3072 K 768   13.2 / 19.8 / 33.1 / 119.8 / 6240            9.3 / 9.3 /  9.5 / 14.9 / 192
   //   N 1000 K 100    4.3 / 4.4 /  6.2 /  19.8 /  676            6.2 / 7.1 /  7.2 / 13.7 /  28
-  // so two passes over a small matrix stay here. Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336):
-  // 9.2e-8 / 1.0e-7 / 1.6e-7 here, 8.0e-8..9.1e-8 / 9.6e-8..1.0e-7 / 1.3e-7 there.
-  const bool few = M <= F32_MT || (M <= 2 * F32_MT && N * K <= (1 << 20));
+  // so two passes over a small matrix stay here, and five to eight rows over a large one go there (4096 x 4096: 46.8 us against 26.4).
+  // Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336): 9.2e-8 / 1.0e-7 / 1.6e-7 here, 8.0e-8..9.1e-8 /
+  // 9.6e-8..1.0e-7 / 1.3e-7 there.
+  const bool few = M <= 4 || (M <= F32_MT && (g.ln_gain || N * K <= (8 << 20))) || (M <= 2 * F32_MT && N * K <= (1 << 20));
   if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) return k_gemm_f32_tc(ctx, g);
-  int ks = 1;  // warps per output channel: slices of at most 1024 columns, as long as the grid stays small
-  while (ks < 8 && K > 1024 * (int64_t)ks && (N * ks * 2 + 7) / 8 <= 8 * (int64_t)ctx->sm_count) ks *= 2;
-  const int rows = 8 / ks;
-  dim3 grid((unsigned)((N + rows - 1) / rows), (unsigned)((M + F32_MT - 1) / F32_MT));
-  if (grid.y > 65535) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: M too large");
-  SB_CUDA(sb_launch(ctx, gemm_f32_kernel, grid, dim3(256), 0, (int)M, (int)N, (int)K, g.x, g.ldx, g.w, g.ldw, g.bias, g.y, g.ldy, g.mode, ks, g.act_pos,
-                    g.act_neg, g.col_scale, g.alpha));
-  ctx->launches++;
-  return STRICTB200_OK;
+  if (g.ln_gain && !sb_gemm_f32_takes_norm(M, K)) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: rows for the layer norm in front are at most 8 of 1024");
+  // Warps per output channel: slices of at most 1024 columns, and two for a long enough row, while all blocks are resident at once (two
+  // per SM with the norm in front or several rows, else four); two channels per warp where they would not be. With the norm in front
+  // 3072 channels of 768 columns took 6.6 us as 384 blocks of two waves, 3.0 us as 192.
+  const int64_t cap = (M == 1 && !g.ln_gain ? 4 : 2) * (int64_t)ctx->sm_count;
+  int ks = 1;
+  while (ks < 8 && K > 1024 * (int64_t)ks && (N * ks * 2 + 7) / 8 <= 2 * cap) ks *= 2;
+  if (ks == 1 && K >= 512 && (N * 2 + 7) / 8 <= cap) ks = 2;
+  const bool two = (N * ks + 7) / 8 > cap;
+  if (M == 1) return launch_rows<1>(ctx, g, ks, two);
+  if (M == 2) return launch_rows<2>(ctx, g, ks, two);
+  if (M <= 4) return launch_rows<4>(ctx, g, ks, two);
+  return launch_rows<8>(ctx, g, ks, two);
 }

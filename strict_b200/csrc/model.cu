@@ -266,14 +266,24 @@ int gpt2_layers(strictb200_model* m, strictb200_kv* kv, int64_t T, float* xf, fl
   const auto& c = m->c;
   const int64_t d = c.d_model;
   const float scale = 1.0f / sqrtf((float)c.head_dim);
+  // norm, then product: in one launch where the product's kernel takes the norm along
+  auto norm_gemm = [&](const float* g, const float* b, const FW& w, float* y, int mode) -> int {
+    GemmF32Args a;
+    a.M = T; a.N = w.N; a.K = d; a.x = xf; a.ldx = d; a.w = w.w; a.ldw = d; a.bias = w.b; a.y = y; a.ldy = w.N; a.mode = mode;
+    if (sb_gemm_f32_takes_norm(T, d)) {
+      a.ln_gain = g; a.ln_bias = b; a.ln_eps = c.eps;
+    } else {
+      SB_TRY(k_layernorm(ctx, xf, g, b, c.eps, T, d, af));
+      a.x = af;
+    }
+    return k_gemm_f32(ctx, a);
+  };
   for (int l = 0; l < c.n_layers; l++) {
     LayerW& w = m->L[l];
-    SB_TRY(k_layernorm(ctx, xf, w.norm1_g, w.norm1_b, c.eps, T, d, af));
-    SB_TRY(k_gemm_f32(ctx, T, 3 * d, d, af, w.fqkv.w, w.fqkv.b, bf_, 0));
+    SB_TRY(norm_gemm(w.norm1_g, w.norm1_b, w.fqkv, bf_, 0));
     SB_TRY(k_attn_f32(ctx, bf_, kv_kf(kv, l), kv_vf(kv, l), seq, pos, kv->d_lens, T, c.n_q_heads, c.head_dim, kv->maxlen, scale, af, prompts));
     SB_TRY(k_gemm_f32(ctx, T, d, d, af, w.fo.w, w.fo.b, xf, 1));
-    SB_TRY(k_layernorm(ctx, xf, w.norm2_g, w.norm2_b, c.eps, T, d, af));
-    SB_TRY(k_gemm_f32(ctx, T, c.d_ff, d, af, w.ffc.w, w.ffc.b, bf_, 2));  // GELU in the epilogue
+    SB_TRY(norm_gemm(w.norm2_g, w.norm2_b, w.ffc, bf_, 2));  // GELU in the epilogue
     SB_TRY(k_gemm_f32(ctx, T, d, c.d_ff, bf_, w.fproj.w, w.fproj.b, xf, 1));
   }
   return STRICTB200_OK;

@@ -44,6 +44,21 @@ def test_gemm_f32_many_rows(ctx, rng, M, N_, K):
     assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
 
 
+# the row kernel's instances: one to eight rows, one or two channels per warp, rows split over warps, rows of X that do not fit shared memory
+@pytest.mark.parametrize("M,N_,K", [(1, 9600, 300), (2, 2500, 768), (3, 4999, 1028), (4, 2400, 2048), (4, 40, 6200), (7, 500, 512), (8, 6001, 64),
+                                    (8, 300, 12000), (16, 700, 1200)])
+def test_gemm_f32_few_rows(ctx, rng, M, N_, K):
+    x, w = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(N_).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm(ctx, x, w, None)
+    # a lane adds its part of at most K columns four at a time, then 5 folds and 8 slices: each addition at most 2^-24 of the magnitudes
+    assert (np.abs(got - want) <= (K / 32 + 4 + 5 + 8) * 2.0 ** -24 * size).all()
+    assert np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2)) < 2e-7
+    assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
+
+
 def test_gemm_f32_many_rows_not_finite(ctx, rng):
     """Infinities and NaN reach exactly the results they reach in a plain sum; an operand row at the end of the fp32 range is computed."""
     x, w = rng.standard_normal((40, 200)).astype(np.float32), rng.standard_normal((70, 200)).astype(np.float32)
@@ -59,9 +74,11 @@ def test_gemm_f32_many_rows_not_finite(ctx, rng):
 
 
 # head widths of the two kernels (64) and of the decode kernel alone (32, 128), one that neither takes; prompts around the 64-row tile
-@pytest.mark.parametrize("head_dim,lens", [(64, [1, 63, 64, 65, 130]), (64, [200, 3]), (32, [70, 9]), (128, [66, 40]), (48, [20, 33])])
-def test_gpt2_prompts_and_decode(ctx, oracle, head_dim, lens):
-    cfg = dict(TINY_GPT2, d_model=2 * head_dim, head_dim=head_dim, d_ff=4 * head_dim, max_pos=256, vocab=300)
+# a wide feed-forward: the norm in front of a product with two channels per warp
+@pytest.mark.parametrize("head_dim,lens,d_ff", [(64, [1, 63, 64, 65, 130], 0), (64, [200, 3], 2560), (32, [70, 9], 0), (128, [66, 40, 5, 1, 9, 2, 3], 2560),
+                                                (64, [12] * 9, 0), (48, [20, 33], 0)])
+def test_gpt2_prompts_and_decode(ctx, oracle, head_dim, lens, d_ff):
+    cfg = dict(TINY_GPT2, d_model=2 * head_dim, head_dim=head_dim, d_ff=d_ff or 4 * head_dim, max_pos=256, vocab=300)
     B, S, seed = len(lens), max(lens), 11
     m, om = sb.Model(ctx, cfg).init_random(seed), oracle.Model(cfg, seed)
     kv, st = m.new_cache(B, S + 40), om.new_state(B, S + 40)
