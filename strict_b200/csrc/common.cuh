@@ -245,6 +245,7 @@ __device__ __forceinline__ float sb_xielu_bf16(float z, float pos, float neg) {
   const float t = z > -0.0625f ? series : e - 1.0f - z;
   return fmaf(z > 0.f ? pos : neg, z > 0.f ? zz : t, 0.5f * z);
 }
+__device__ __forceinline__ float sb_silu_mul(float g, float u) { return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u); }
 // tanh-approximated GELU in fp32 with the operation order of the element-wise kernel
 __device__ __forceinline__ float sb_gelu_tanh(float v) {
   const float u = __fmul_rn(0.797884583f, __fadd_rn(v, __fmul_rn(0.044715f, __fmul_rn(__fmul_rn(v, v), v))));

@@ -16,10 +16,10 @@
 //   warp 1      TMEM allocation (both blocks, cta_group::2: 512 columns = two accumulators);
 //               the leader's lane 0 issues the MMAs for the pair and one tcgen05.commit per
 //               block (frees the stage in both blocks, publishes the accumulator to both)
-//   warps 2..5  epilogue of this block's 128 channels; hand the accumulator back by arriving on
-//               the leader's barrier (remote mbarrier.arrive from the second block)
-// Persistent schedule: one pair per two SMs, pair c owns tiles [c*tiles/pairs, (c+1)*tiles/pairs),
-// two accumulators so the epilogue of a tile overlaps the MMAs of the next one.
+//   warps 2..9  epilogue of this block's 128 channels, half of the columns each; hand the accumulator back by
+//               arriving on the leader's barrier (remote mbarrier.arrive from the second block)
+// Persistent schedule: one pair per two SMs, pair c owns the tiles c, c + pairs, ... of a walk in which neighbouring
+// numbers share operands (tile_at), two accumulators so the epilogue of a tile overlaps the MMAs of the next one.
 // Every mbarrier wait is bounded: on expiry the block records an error word in host-visible
 // memory and stops issuing work; TMEM is freed and the pair leaves together.
 #include <cuda.h>
@@ -37,6 +37,8 @@ constexpr int UMMA_K = 32;    // bytes (= E4M3 elements) of K per tcgen05.mma
 constexpr int STAGES = 7;
 constexpr int STAGE_BYTES = BN * BK + BTH * BK;  // 32 KB per block
 constexpr int ACC_COLS = 256, TMEM_COLS = 512;
+constexpr int EPI_WARPS = 8, THREADS = 32 * (2 + EPI_WARPS);
+constexpr int RASTER = 8;  // token tiles that are walked side by side
 constexpr uint32_t WAIT_LIMIT = 1u << 22;  // try_wait attempts before giving up (each blocks up to ~1 us)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -114,13 +116,13 @@ __device__ __forceinline__ void tc_wait_ld16(uint32_t* r) {
                :
                : "memory");
 }
-// Barrier over the 4 epilogue warps that also ORs a predicate (all 128 leave the tile loop together).
+// Barrier over the epilogue warps that also ORs a predicate (all of them leave the tile loop together).
 __device__ __forceinline__ bool epi_any(bool pred) {
   uint32_t out;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.or.pred p, 1, 128, q;\n\t"
+      "bar.red.or.pred p, 1, 256, q;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(out)
       : "r"((uint32_t)pred)
@@ -153,17 +155,35 @@ struct PairArgs {
   void* out;
   int out_f32;
   int* status;   // host-visible error word
-  int tiles_n;   // 256-channel tiles; tile = tt * tiles_n + tn
-  int tiles;
+  int tiles_n;   // 256-channel tiles
+  int tiles;     // tiles_n times the token tiles
   Bf16Epilogue e;        // BF16 only, and so are the rest
   int group_n, group_k;  // block-diagonal product: channels per group, bytes of an operand row per group (0: dense)
 };
 
+// Tile number -> channel tile tn and token tile tt. RASTER token tiles are walked together, one channel tile after the other, so
+// that the pairs at work at a time (74 consecutive numbers) read about 8 token tiles and 10 channel tiles of the operands instead
+// of up to 74 of one of them: the bytes that leave L2 for the SMs stay the same, those that enter it fall. 6577 tokens through a layer of
+// Qwen3-8B: the four products took 2883 us with a run of consecutive channel tiles per pair (24576 channels of 4096 alone stream 100 MB
+// of weights per token tile), 2374 us so, with two epilogue warps per 32 channels in place of one.
+__device__ __forceinline__ void tile_at(const PairArgs& a, int tile, int& tn, int& tt) {
+  const int tiles_t = a.tiles / a.tiles_n, g = tile / (RASTER * a.tiles_n), r = tile - g * RASTER * a.tiles_n;
+  const int h = min(RASTER, tiles_t - g * RASTER);
+  tn = r / h;
+  tt = g * RASTER + r - tn * h;
+}
+
 // BF16: plain bf16 operands, one operand row (accumulator column) per token, so a tile is 256 channels x 256 tokens; K
 // counts bytes, and a row that ends inside a 128-byte block is filled with zeros by the copy.
-template <bool BF16>
-__global__ void __launch_bounds__(192) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+// GLU: E4M3 weights whose rows are [gate | up]; the product leaves as bf16 silu(gate) * up. Every 16 gate rows are staged beside the
+// 16 up rows of the same channels (boxes of 16 rows), so that the two accumulators of a channel sit 16 lanes apart in one warp; the
+// lanes trade half of their tokens. Against fp32 results and a kernel that multiplies them this saves 12 bytes a channel and token: 223 us
+// of that kernel for 6577 tokens x 12288 channels became 59 us of the split of bf16 rows.
+enum { PAIR_F8 = 0, PAIR_BF16 = 1, PAIR_GLU = 2 };
+template <int KIND>
+__global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                         PairArgs a) {
+  constexpr bool BF16 = KIND == PAIR_BF16, GLU = KIND == PAIR_GLU;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
@@ -176,13 +196,13 @@ __global__ void __launch_bounds__(192) gemm_pair_kernel(const __grid_constant__ 
   const bool leader = rank == 0;
   const int nkb = (a.K + BK - 1) / BK;
   const int pairs = gridDim.x / 2, c = blockIdx.x / 2;
-  const int tile_begin = (int)((int64_t)c * a.tiles / pairs), tile_end = (int)((int64_t)(c + 1) * a.tiles / pairs);
-  const int n_my = (tile_end - tile_begin) * nkb;  // K blocks this pair walks through
+  const int my_tiles = (a.tiles - c + pairs - 1) / pairs;
+  const int n_my = my_tiles * nkb;  // K blocks this pair walks through
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(smem_u32(&bar_full[s]), 1); mbar_init(smem_u32(&bar_empty[s]), 1); }
-    // accumulator hand-back: the 128 epilogue threads of each block arrive on the leader's barrier
-    for (int s = 0; s < 2; s++) { mbar_init(smem_u32(&bar_acc_full[s]), 1); mbar_init(smem_u32(&bar_acc_empty[s]), 256); }
+    // accumulator hand-back: one lane of every epilogue warp of both blocks arrives on the leader's barrier
+    for (int s = 0; s < 2; s++) { mbar_init(smem_u32(&bar_acc_full[s]), 1); mbar_init(smem_u32(&bar_acc_empty[s]), 2 * EPI_WARPS); }
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -200,18 +220,25 @@ __global__ void __launch_bounds__(192) gemm_pair_kernel(const __grid_constant__ 
   if (warp == 0) {
     if (lane == 0) {
       pdl_wait();
+      int tn = 0, tt = 0, kb = -1;
       for (int it = 0; it < n_my; it++) {
         const int s = it % STAGES;
         if (it >= STAGES && !mbar_wait(smem_u32(&bar_empty[s]), ((it / STAGES) & 1) ^ 1)) { set_status(a.status, 1); abort_flag = 1; break; }
         if (*(volatile int*)&abort_flag) break;
-        const int tile = tile_begin + it / nkb, kb = it % nkb;
-        const int wy = (tile % a.tiles_n) * 2 * BN + (int)rank * BN, xy0 = (tile / a.tiles_n) * 2 * BTH + (int)rank * BTH;
-        const int xy = BF16 && a.e.n_switch > 0 && (tile % a.tiles_n) * 2 * BN >= a.e.n_switch ? a.e.x_row_off + xy0 : xy0;
+        if (++kb == nkb || it == 0) { kb = 0; tile_at(a, c + it / nkb * pairs, tn, tt); }
+        const int wy = tn * 2 * BN + (int)rank * BN, xy0 = tt * 2 * BTH + (int)rank * BTH;
+        const int xy = BF16 && a.e.n_switch > 0 && tn * 2 * BN >= a.e.n_switch ? a.e.x_row_off + xy0 : xy0;
         const uint32_t full_leader = map_to_rank(smem_u32(&bar_full[s]), 0);
         if (leader) mbar_expect_tx(smem_u32(&bar_full[s]), 2 * STAGE_BYTES);  // the bytes of both blocks
         const uint32_t dst = smem_u32(smem + (size_t)s * STAGE_BYTES);
-        tma_load_2d_pair(dst, &map_w, kb * BK, wy, full_leader);
-        const int xk = BF16 && a.group_n > 0 ? (tile % a.tiles_n) * 2 * BN / a.group_n * a.group_k : 0;
+        if constexpr (GLU) {
+          const int hc = tn * BN + (int)rank * (BN / 2);  // first of this block's 64 channels
+#pragma unroll
+          for (int i = 0; i < 8; i++) tma_load_2d_pair(dst + i * 16 * BK, &map_w, kb * BK, (i & 1 ? a.N / 2 : 0) + hc + (i >> 1) * 16, full_leader);
+        } else {
+          tma_load_2d_pair(dst, &map_w, kb * BK, wy, full_leader);
+        }
+        const int xk = BF16 && a.group_n > 0 ? tn * 2 * BN / a.group_n * a.group_k : 0;
         tma_load_2d_pair(dst + BN * BK, &map_x, xk + kb * BK, xy, full_leader);
       }
     }
@@ -246,51 +273,68 @@ __global__ void __launch_bounds__(192) gemm_pair_kernel(const __grid_constant__ 
     }
   } else {
     // epilogue: warp w may touch TMEM lanes [32*(w%4), +32) = channels of this block's half
-    const int lg = warp & 3;
+    const int lg = warp & 3, half = (warp - 2) >> 2;
     const int ch = lg * 32 + lane;
+    constexpr int HALF = ACC_COLS / 2;
     pdl_wait();  // the scales and the output buffer belong to the dependency chain
-    for (int seg = 0; seg < tile_end - tile_begin; seg++) {
-      const int tile = tile_begin + seg;
+    for (int seg = 0; seg < my_tiles; seg++) {
+      int tn, tt;
+      tile_at(a, c + seg * pairs, tn, tt);
       bool bad = !mbar_wait(smem_u32(&bar_acc_full[seg & 1]), (seg >> 1) & 1);
       if (bad && lane == 0) set_status(a.status, 3);
       if (epi_any(bad)) break;
       tc_fence_after();
-      const uint32_t acc = tmem + (uint32_t)((seg & 1) * ACC_COLS) + ((uint32_t)(lg * 32) << 16);
-      const int n = (tile % a.tiles_n) * 2 * BN + (int)rank * BN + ch;
-      const int tok_base = (tile / a.tiles_n) * BTH;  // 256 operand rows = 128 tokens per tile
-      const float swn = !BF16 && n < a.N ? a.sw[n] : 0.f;
-      if constexpr (BF16) {  // 256 tokens per tile, 32 at a time
+      const uint32_t acc = tmem + (uint32_t)((seg & 1) * ACC_COLS + half * HALF) + ((uint32_t)(lg * 32) << 16);
+      // output channel of this lane; GLU: the one whose gate (lanes 0..15) or up (16..31) it holds
+      const int n = GLU ? tn * BN + (int)rank * (BN / 2) + lg * 16 + (lane & 15) : tn * 2 * BN + (int)rank * BN + ch;
+      const int n_end = GLU ? a.N / 2 : a.N;
+      const float swn = !BF16 && n < n_end ? a.sw[GLU && lane >= 16 ? n_end + n : n] : 0.f;
 #pragma unroll 1
-        for (int grp = 0; grp < ACC_COLS / 16; grp += 2) {
-          uint32_t r[32];
-          tc_ld16(acc + (uint32_t)(grp * 16), r);
-          tc_ld16(acc + (uint32_t)(grp * 16 + 16), r + 16);
-          tc_wait_ld16(r);
-          tc_wait_ld16(r + 16);
-          sb_bf16_store16(a.e, a.M, a.N, 2 * tok_base + grp * 16, n, r);
-          sb_bf16_store16(a.e, a.M, a.N, 2 * tok_base + grp * 16 + 16, n, r + 16);
-        }
-      } else {
-#pragma unroll 1
-        for (int grp = 0; grp < ACC_COLS / 16; grp++) {
-          uint32_t r[16];
-          tc_ld16(acc + (uint32_t)(grp * 16), r);
-          tc_wait_ld();
+      for (int grp = 0; grp < HALF / 16; grp += 2) {  // 32 operand rows at a time
+        uint32_t r[32];
+        tc_ld16(acc + (uint32_t)(grp * 16), r);
+        tc_ld16(acc + (uint32_t)(grp * 16 + 16), r + 16);
+        tc_wait_ld16(r);
+        tc_wait_ld16(r + 16);
+        if constexpr (BF16) {
+          const int tok = tt * 2 * BTH + half * HALF + grp * 16;
+          sb_bf16_store16(a.e, a.M, a.N, tok, n, r);
+          sb_bf16_store16(a.e, a.M, a.N, tok + 16, n, r + 16);
+        } else {
+          const int tok0 = tt * BTH + half * (HALF / 2) + grp * 8;  // operand rows 16g.. hold tokens 8g..
+          if constexpr (GLU) {
+            const bool up = lane >= 16;
+            float y[16];
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int tok = tok_base + grp * 8 + j;  // operand rows 16g.. hold tokens 8g..
+            for (int j = 0; j < 16; j++) {
+              const int k = (j & 8) * 2 + (j & 7);
+              const float v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
+              y[j] = __fmul_rn(__fmul_rn(v, tok0 + j < a.M ? a.sx[tok0 + j] : 0.f), swn);
+            }
+            bf16* o = (bf16*)a.out + (int64_t)(tok0 + (up ? 8 : 0)) * n_end + n;
+#pragma unroll
+            for (int j = 0; j < 8; j++, o += n_end) {
+              const float got = __shfl_xor_sync(0xffffffffu, up ? y[j] : y[8 + j], 16);
+              if (n < n_end && tok0 + (up ? 8 : 0) + j < a.M) *o = __float2bfloat16_rn(sb_silu_mul(up ? got : y[j], up ? y[8 + j] : got));
+            }
+            continue;
+          }
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            const int tok = tok0 + j, k = (j & 8) * 2 + (j & 7);
             if (tok < a.M && n < a.N) {
-              float v = __fadd_rn(__uint_as_float(r[j]), __fmul_rn(0.0625f, __uint_as_float(r[8 + j])));
-              float y = __fmul_rn(__fmul_rn(v, a.sx[tok]), swn);
+              const float v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
+              const float y = __fmul_rn(__fmul_rn(v, a.sx[tok]), swn);
               if (a.out_f32) ((float*)a.out)[(int64_t)tok * a.N + n] = y;
               else ((bf16*)a.out)[(int64_t)tok * a.N + n] = __float2bfloat16_rn(y);
             }
           }
         }
       }
-      // the accumulator is drained in this block: tell the leader's MMA warp
+      // the accumulator is drained by this warp: tell the leader's MMA warp
       tc_fence_before();
-      mbar_arrive_cluster(map_to_rank(smem_u32(&bar_acc_empty[seg & 1]), 0));
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&bar_acc_empty[seg & 1]), 0));
     }
   }
   // Nobody leaves while the other block may still signal one of its barriers or use its tensor memory.
@@ -316,11 +360,11 @@ int get_encode() {
   return STRICTB200_OK;
 }
 
-// 2D map of a row-major byte matrix [rows, K] (row stride ld bytes), box = 128 rows x 128 bytes, 128-byte swizzle.
-int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld) {
+// 2D map of a row-major byte matrix [rows, K] (row stride ld bytes), box = box_rows x 128 bytes, 128-byte swizzle.
+int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows = 128) {
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)ld};
-  cuuint32_t box[2] = {(cuuint32_t)BK, 128u};
+  cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -330,8 +374,8 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_
 
 }  // namespace
 
-// Y = ((X . Wq^T) * sx) * sw for many tokens (prefill). ERR_UNSUPPORTED for shapes this kernel does not take.
-int k_gemm_fp8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) {
+template <int KIND>
+static int launch_f8(strictb200_ctx* ctx, const GemmArgs& g) {
   if (g.K % BK || g.splits != 1 || g.raw || !g.out) return sb_fail(STRICTB200_ERR_UNSUPPORTED, "paired tensor-memory GEMM: K % 128, no splits, no raw output");
   if (((uintptr_t)g.xq | (uintptr_t)g.wq | (uintptr_t)g.ldx | (uintptr_t)g.ldw) & 15)
     return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_fp8: operands and row strides must be 16-byte aligned");
@@ -341,17 +385,26 @@ int k_gemm_fp8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) {
   if (tiles > INT32_MAX / 2) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_fp8: too many output tiles");
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;  // + slack for the 1024-byte round-up
   static SbDeviceOnce once;
-  SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
+  SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_pair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
   CUtensorMap mw, mx;
-  SB_TRY(make_map(&mw, g.wq, g.N, g.K, g.ldw));
+  SB_TRY(make_map(&mw, g.wq, g.N, g.K, g.ldw, KIND == PAIR_GLU ? 16 : 128));
   SB_TRY(make_map(&mx, g.xq, Mq, g.K, g.ldx));
   PairArgs pa{(int)g.M, (int)Mq, (int)g.N, (int)g.K, g.sx, g.sw, g.out, g.out_f32, ctx->d_status, (int)tiles_n, (int)tiles, {}, 0, 0};
   int64_t pairs = ctx->sm_count / 2;
   if (pairs > tiles) pairs = tiles;
-  SB_CUDA(sb_launch_cluster(ctx, gemm_pair_kernel<false>, dim3((unsigned)(2 * pairs)), dim3(192), smem, dim3(2, 1, 1), mw, mx, pa));
+  SB_CUDA(sb_launch_cluster(ctx, gemm_pair_kernel<KIND>, dim3((unsigned)(2 * pairs)), dim3(THREADS), smem, dim3(2, 1, 1), mw, mx, pa));
   ctx->launches++;
   return STRICTB200_OK;
 }
+
+// Y = ((X . Wq^T) * sx) * sw for many tokens (prefill). ERR_UNSUPPORTED for shapes this kernel does not take.
+int k_gemm_fp8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) { return launch_f8<PAIR_F8>(ctx, g); }
+
+// bf16 silu(gate) * up [M, N/2] of the same product with W = [gate | up], where the many-token kernel takes the shape.
+bool sb_gemm_fp8_swiglu_fits(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K) {
+  return ctx->opt.gemm_pair && ctx->sm_count >= 2 && sb_qrows(M) > 256 && N >= 256 && N % 2 == 0 && K % BK == 0;
+}
+int k_gemm_fp8_swiglu(strictb200_ctx* ctx, const GemmArgs& g) { return launch_f8<PAIR_GLU>(ctx, g); }
 
 // The same for bf16 operands, finished values through b.e.
 int k_gemm_bf16_tmem_pair(strictb200_ctx* ctx, const GemmBf16Args& b) {
@@ -360,7 +413,7 @@ int k_gemm_bf16_tmem_pair(strictb200_ctx* ctx, const GemmBf16Args& b) {
   if (tiles > INT32_MAX / 2) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_bf16: too many output tiles");
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
   static SbDeviceOnce once;
-  SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
+  SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_pair_kernel<PAIR_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
   CUtensorMap mw, mx;
   if (b.group_n && (b.group_n % (2 * BN) || b.group_k % 8)) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_bf16: groups must fill channel tiles");
   SB_TRY(make_map(&mw, b.w, b.N, kbytes, 2 * b.ldw));
@@ -368,7 +421,7 @@ int k_gemm_bf16_tmem_pair(strictb200_ctx* ctx, const GemmBf16Args& b) {
   PairArgs pa{(int)b.M, (int)b.M, (int)b.N, (int)kbytes, nullptr, nullptr, nullptr, 1, ctx->d_status, (int)tiles_n, (int)tiles, b.e, b.group_n, (int)(2 * b.group_k)};
   int64_t pairs = ctx->sm_count / 2;
   if (pairs > tiles) pairs = tiles;
-  SB_CUDA(sb_launch_cluster(ctx, gemm_pair_kernel<true>, dim3((unsigned)(2 * pairs)), dim3(192), smem, dim3(2, 1, 1), mw, mx, pa));
+  SB_CUDA(sb_launch_cluster(ctx, gemm_pair_kernel<PAIR_BF16>, dim3((unsigned)(2 * pairs)), dim3(THREADS), smem, dim3(2, 1, 1), mw, mx, pa));
   ctx->launches++;
   return STRICTB200_OK;
 }

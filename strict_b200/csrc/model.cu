@@ -452,8 +452,17 @@ int qwen_prefill_chunk(strictb200_model* m, strictb200_kv* kv, const PrefillChun
       a.x_f32 = y; a.residual_f32 = x; a.gain = w.norm2_g; a.eps = c.eps; a.q = aq; a.qscale = sa;
       SB_TRY(k_rownorm(ctx, a, T, d));
     }
-    SB_TRY(run_gemm(m, T, w.wgu, aq, sa, gu, 1, nullptr, 1, 0));
-    SB_TRY(k_swiglu(ctx, nullptr, gu, T, m->I_l, nullptr, aq, sa));
+    if (sb_gemm_fp8_swiglu_fits(ctx, T, w.wgu.N, w.wgu.K)) {
+      // the product's epilogue applies SwiGLU (bf16, in the space of the fp32 results); the row maximum the split needs is a pass of its own
+      GemmArgs g;
+      g.M = T; g.N = w.wgu.N; g.K = w.wgu.K;
+      g.xq = aq; g.ldx = w.wgu.K; g.sx = sa; g.wq = w.wgu.q; g.ldw = w.wgu.K; g.sw = w.wgu.s; g.out = gu;
+      SB_TRY(k_gemm_fp8_swiglu(ctx, g));
+      SB_TRY(k_quantize_rows(ctx, (const bf16*)gu, T, m->I_l, m->I_l, aq, sa));
+    } else {
+      SB_TRY(run_gemm(m, T, w.wgu, aq, sa, gu, 1, nullptr, 1, 0));
+      SB_TRY(k_swiglu(ctx, nullptr, gu, T, m->I_l, nullptr, aq, sa));
+    }
     {
       RowNormArgs a;
       SB_TRY(run_gemm(m, T, w.wdown, aq, sa, y, 1, nullptr, 1, 0));

@@ -478,10 +478,6 @@ __global__ void add_f32_kernel(float* __restrict__ x, const float* __restrict__ 
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = __fadd_rn(x[i], y[i]);
 }
 
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))), u);
-}
-
 // gate_up [M, 2I] (bf16, or the projection's fp32 result) -> h = bf16(silu(gate)*up); optional
 // two-term E4M3 split of h per row. 512 threads; a thread owns up to 4 groups of 8 columns and
 // keeps h in registers between the absmax pass and the split (rows wider than 16384 recompute).
@@ -500,7 +496,7 @@ __global__ void __launch_bounds__(SW_THREADS) swiglu_kernel(const bf16* __restri
     if (gu32) { load8_f32(gu32 + row * 2 * I + k, g); load8_f32(gu32 + row * 2 * I + I + k, u); }
     else { load8_bf16(gu + row * 2 * I + k, g); load8_bf16(gu + row * 2 * I + I + k, u); }
 #pragma unroll
-    for (int i = 0; i < 8; i++) h[i] = round_bf16(silu_mul(g[i], u[i]));
+    for (int i = 0; i < 8; i++) h[i] = round_bf16(sb_silu_mul(g[i], u[i]));
   };
   if (in_regs) {
 #pragma unroll
@@ -561,7 +557,7 @@ __global__ void __launch_bounds__(512) swiglu_decode_kernel(const float* __restr
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    h[i] = round_bf16(silu_mul(g[i], u[i]));
+    h[i] = round_bf16(sb_silu_mul(g[i], u[i]));
     amax = fmaxf(amax, fabsf(h[i]));
   }
   if (y) store8_bf16(y + row * I + k, h);
@@ -611,7 +607,7 @@ __global__ void __launch_bounds__(512) swiglu_decode_part_kernel(const float* __
   float h[4], amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    h[i] = round_bf16(silu_mul(__fmul_rn(__fmul_rn(g[i], sxr), wgv[i]), __fmul_rn(__fmul_rn(u[i], sxr), wuv[i])));
+    h[i] = round_bf16(sb_silu_mul(__fmul_rn(__fmul_rn(g[i], sxr), wgv[i]), __fmul_rn(__fmul_rn(u[i], sxr), wuv[i])));
     amax = fmaxf(amax, fabsf(h[i]));
   }
   amax = block_max(amax, red);
