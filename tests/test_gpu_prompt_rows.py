@@ -1,0 +1,41 @@
+"""Kernels that only the rows of longer prompts reach: SwiGLU in the product's epilogue, the walk over output tiles, norms, rotations and
+splits of whole rows."""
+import numpy as np
+import pytest
+
+from strict_b200 import native as N
+from strict_b200.kernel import DeviceVariable as DV
+from conftest import TOL_FP8, logits_close
+from test_gpu_models import TINY_QWEN, _run_pair
+
+pytestmark = pytest.mark.gpu
+L = N.lib
+
+
+# feed-forwards that end inside a tile of 128 channels; more than eight token tiles of 128 and an odd rest of them; norms of one, two and
+# eight column groups per thread (the last with a width that is no multiple of 128 and takes other products); more than 32 and fewer heads
+@pytest.mark.parametrize("over,lens", [(dict(d_ff=192), [100, 77, 40]), (dict(d_ff=320, n_q_heads=36, n_kv_heads=3, head_dim=128), [90, 211]),
+                                       (dict(d_model=1152, d_ff=128), [700, 520]), (dict(d_model=4160, d_ff=128), [12, 9]), (dict(d_model=2048, d_ff=256), [1100])],
+                         ids=["ff192", "heads42", "d1152", "d4160", "d2048"])
+def test_prompts_vs_oracle(ctx, oracle, over, lens):
+    cfg = dict(TINY_QWEN, n_layers=2, vocab=512, max_pos=1200, **over)
+    m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 7, len(lens), max(lens), lens, 1, random_gains=True)
+    ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+    assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
+
+
+@pytest.mark.parametrize("K", [2048, 2056, 4096, 4104, 12288, 12296, 16384])
+def test_quantize_rows_widths(ctx, oracle, rng, K):
+    M = 9
+    x = oracle.round_bf16((rng.standard_normal((M, K)) * rng.uniform(0.01, 30, (M, 1))).astype(np.float32))
+    x[2, K - 1] = 300.0  # the largest value in the last column
+    dx, dq, ds = DV.of(ctx, oracle.f32_to_bf16(x)), DV(ctx, 32 * K, np.uint8), DV(ctx, M)
+    dq.zero()
+    N.check(L().strictb200_quantize_rows(ctx.h, dx.p, M, K, dq.p, ds.p))
+    q, s = oracle.split_rows_device_layout(x)
+    assert np.array_equal(ds.to_host(), s) and np.array_equal(dq.to_host().reshape(32, K), q)
+    for v in (dx, dq, ds):
+        v.free()
