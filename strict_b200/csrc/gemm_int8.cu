@@ -13,6 +13,7 @@
 #include "common.cuh"
 
 int k_gemm_fp8_tmem_split(strictb200_ctx* ctx, const GemmArgs& g);  // gemm_tmem_split.cu
+int k_gemm_int8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g);  // gemm_tmem_pair.cu
 
 namespace {
 
@@ -37,33 +38,84 @@ __device__ __forceinline__ float int8_row_scale(float absmax) {
   return ldexpf(1.f, m <= 0.9921875f ? e - 14 : e - 13);
 }
 
+// v = 128 h + l with h in [-127, 127], l in [-64, 63].
+__device__ __forceinline__ int split_int8(float x, float inv, int& l) {
+  const int v = __float2int_rn(__fmul_rn(x, inv)), h = (v + 64) >> 7;
+  l = v - (h << 7);
+  return h;
+}
+
+// Rows of the last group of 8 that hold no token are zeroed by the last token's block, so that the MMA reads defined bytes.
+__device__ __forceinline__ void zero_pad_rows(int8_t* hi, int8_t* lo, int64_t row, int64_t M, int64_t K) {
+  if (row != M - 1) return;
+  const int64_t n = (7 - (row & 7)) * K;  // they follow this row, in both terms
+  for (int64_t i = threadIdx.x; i < n; i += QT) hi[K + i] = lo[K + i] = 0;
+}
+
 // One block per token row.
-__global__ void __launch_bounds__(QT) quantize_rows_int8_kernel(const bf16* __restrict__ x, int64_t K, int8_t* __restrict__ q, float* __restrict__ scale) {
+__global__ void __launch_bounds__(QT) quantize_rows_int8_kernel(const bf16* x, int64_t M, int64_t K, int8_t* q, float* scale) {
   __shared__ float red[QT / 32];
+  pdl_trigger();
+  pdl_wait();
   const int64_t row = blockIdx.x;
+  int8_t* hi = q + ((row >> 3) * 16 + (row & 7)) * K;
+  int8_t* lo = hi + 8 * K;
+  zero_pad_rows(hi, lo, row, M, K);
   const bf16* xr = x + row * K;
   float amax = 0.f;
   for (int64_t k = threadIdx.x; k < K; k += QT) amax = fmaxf(amax, fabsf(__bfloat162float(xr[k])));
   amax = block_absmax(amax, red);
   const float s = int8_row_scale(amax), inv = 1.f / s;  // a power of two: the division and the product below are exact
   if (threadIdx.x == 0) scale[row] = s;
-  int8_t* hi = q + ((row >> 3) * 16 + (row & 7)) * K;
-  int8_t* lo = hi + 8 * K;
   for (int64_t k = threadIdx.x; k < K; k += QT) {
-    const int v = __float2int_rn(__fmul_rn(__bfloat162float(xr[k]), inv));
-    const int h = (v + 64) >> 7;
-    hi[k] = (int8_t)h;
-    lo[k] = (int8_t)(v - (h << 7));
+    int l;
+    hi[k] = (int8_t)split_int8(__bfloat162float(xr[k]), inv, l);
+    lo[k] = (int8_t)l;
   }
 }
-// Rows of the last group that hold no token are zeroed, so the MMA reads defined bytes.
-__global__ void zero_pad_rows_kernel(int8_t* __restrict__ q, int64_t M, int64_t K) {
-  const int64_t pad = (8 - (M & 7)) & 7, g = M >> 3;
-  const int64_t total = pad * 2 * K, step = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
-    const int64_t r = i / K, k = i - r * K;  // r in [0, 2*pad): hi pads then lo pads
-    const int64_t slot = (M & 7) + (r % pad) + (r / pad) * 8;
-    q[(g * 16 + slot) * K + k] = 0;
+// The same for rows that are 16-byte aligned and a multiple of 8 wide, up to IT * QT * 8 columns: a row is loaded once, eight columns per load
+// and store, and stays in registers between the maximum and the split. Bound by HBM (four bytes per column).
+template <int IT>
+__global__ void __launch_bounds__(QT) quantize_rows_int8_wide_kernel(const bf16* x, int M, int K, int8_t* q, float* scale) {
+  __shared__ float red[QT / 32];
+  pdl_trigger();
+  pdl_wait();
+  const int row = blockIdx.x;
+  int8_t* hi = q + ((int64_t)(row >> 3) * 16 + (row & 7)) * K;
+  int8_t* lo = hi + (int64_t)8 * K;
+  zero_pad_rows(hi, lo, row, M, K);
+  uint4 w[IT];
+#pragma unroll
+  for (int i = 0; i < IT; i++) {
+    const int k = (i * QT + threadIdx.x) * 8;
+    w[i] = k < K ? *(const uint4*)(x + (int64_t)row * K + k) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  auto column = [](const uint4& u, int j) {
+    const uint32_t t = j < 2 ? u.x : j < 4 ? u.y : j < 6 ? u.z : u.w;
+    return __uint_as_float(j & 1 ? t & 0xFFFF0000u : t << 16);
+  };
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < IT; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(column(w[i], j)));
+  amax = block_absmax(amax, red);
+  const float s = int8_row_scale(amax), inv = 1.f / s;
+  if (threadIdx.x == 0) scale[row] = s;
+#pragma unroll
+  for (int i = 0; i < IT; i++) {
+    const int k = (i * QT + threadIdx.x) * 8;
+    if (k >= K) break;
+    uint32_t h[2] = {0u, 0u}, l[2] = {0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      int lj;
+      const int hj = split_int8(column(w[i], j), inv, lj);
+      h[j >> 2] |= (uint32_t)(hj & 255) << (8 * (j & 3));
+      l[j >> 2] |= (uint32_t)(lj & 255) << (8 * (j & 3));
+    }
+    *(uint2*)(hi + k) = make_uint2(h[0], h[1]);
+    *(uint2*)(lo + k) = make_uint2(l[0], l[1]);
   }
 }
 
@@ -104,12 +156,14 @@ __global__ void finish_int8_kernel(const int32_t* __restrict__ part, int splits,
 }  // namespace
 
 int k_quantize_rows_int8(strictb200_ctx* ctx, const bf16* x, int64_t M, int64_t K, int8_t* q, float* scale) {
-  quantize_rows_int8_kernel<<<(unsigned)M, QT, 0, ctx->stream>>>(x, K, q, scale);
-  SB_LAUNCHED(ctx);
-  if (M & 7) {
-    zero_pad_rows_kernel<<<64, 256, 0, ctx->stream>>>(q, M, K);
-    SB_LAUNCHED(ctx);
+  const dim3 grid((unsigned)M);
+  if (K % 8 == 0 && K <= 8 * 8 * QT && (((uintptr_t)x & 15) | ((uintptr_t)q & 7)) == 0) {
+    auto kernel = K <= 8 * QT ? quantize_rows_int8_wide_kernel<1> : K <= 2 * 8 * QT ? quantize_rows_int8_wide_kernel<2> : K <= 4 * 8 * QT ? quantize_rows_int8_wide_kernel<4> : quantize_rows_int8_wide_kernel<8>;
+    SB_CUDA(sb_launch(ctx, kernel, grid, dim3(QT), 0, x, (int)M, (int)K, q, scale));
+  } else {
+    SB_CUDA(sb_launch(ctx, quantize_rows_int8_kernel, grid, dim3(QT), 0, x, M, K, q, scale));
   }
+  ctx->launches++;
   return STRICTB200_OK;
 }
 
@@ -120,6 +174,10 @@ int k_gemm_int8w(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const int
   g.xq = (const uint8_t*)xq; g.ldx = K; g.sx = sx;
   g.wq = (const uint8_t*)wq; g.ldw = K; g.sw = sw;
   g.out = y; g.out_f32 = 0; g.part = (float*)part; g.splits = splits; g.raw = 0; g.kernel = 3; g.i8 = 1;
+  // More than one tile of tokens: SM pairs and 256 x 256 tiles, the line of the E4M3 path (k_gemm_fp8_tmem). Linear layer of 2048 tokens,
+  // 4096 x 4096: 110 us with 128 x 256 tiles of one SM each, one launch of blocks per tile, and a quantiser of two-byte loads; 75 us so.
+  const int64_t rows = sb_qrows(M);
+  if (splits == 1 && ctx->opt.gemm_pair && rows > 256 && rows <= 65535 * 256 && N >= 256 && ctx->sm_count >= 2) return k_gemm_int8_tmem_pair(ctx, g);
   SB_TRY(k_gemm_fp8_tmem_split(ctx, g));
   if (splits > 1) {
     const int64_t total = M * N;

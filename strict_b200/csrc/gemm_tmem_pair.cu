@@ -148,6 +148,17 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t tmem_d, uint64_t desc_
       : "memory");
 }
 
+// Signed 8-bit integer operands, 32-bit integer accumulator (K = 32 per instruction).
+__device__ __forceinline__ void tc_mma_i8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+
 struct PairArgs {
   int M, Mq, N, K;
   const float* sx;
@@ -179,11 +190,12 @@ __device__ __forceinline__ void tile_at(const PairArgs& a, int tile, int& tn, in
 // 16 up rows of the same channels (boxes of 16 rows), so that the two accumulators of a channel sit 16 lanes apart in one warp; the
 // lanes trade half of their tokens. Against fp32 results and a kernel that multiplies them this saves 12 bytes a channel and token: 223 us
 // of that kernel for 6577 tokens x 12288 channels became 59 us of the split of bf16 rows.
-enum { PAIR_F8 = 0, PAIR_BF16 = 1, PAIR_GLU = 2 };
+// I8: int8 weights and two int8 activation terms, x = s * (128 * hi + lo); integer sums, joined exactly before the one conversion.
+enum { PAIR_F8 = 0, PAIR_BF16 = 1, PAIR_GLU = 2, PAIR_I8 = 3 };
 template <int KIND>
 __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                         PairArgs a) {
-  constexpr bool BF16 = KIND == PAIR_BF16, GLU = KIND == PAIR_GLU;
+  constexpr bool BF16 = KIND == PAIR_BF16, GLU = KIND == PAIR_GLU, I8 = KIND == PAIR_I8;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
@@ -244,8 +256,9 @@ __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constan
     }
   } else if (warp == 1) {
     if (leader && lane == 0) {
-      // instruction descriptor: D = F32, A = B = E4M3 (or bf16), both K-major, N = 256 (>> 3 at bit 17), M = 256 (>> 4 at bit 24)
-      constexpr uint32_t idesc = (1u << 4) | (BF16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+      // instruction descriptor: D = F32 (integers: S32), A = B = E4M3 (or bf16, or signed 8 bit), both K-major, N = 256 (>> 3 at bit 17),
+      // M = 256 (>> 4 at bit 24)
+      constexpr uint32_t idesc = (I8 ? 2u << 4 : 1u << 4) | (BF16 || I8 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       // The operand tiles cannot arrive before the producer's dependency wait has returned; waiting for the same
       // dependency here keeps the bounded waits below for progress inside this kernel (a predecessor that itself
       // waits for another rank may take longer than any of them).
@@ -265,7 +278,8 @@ __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constan
         const uint32_t acc = tmem + (uint32_t)((seg & 1) * ACC_COLS);
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; k++)
-          if (BF16) tc_mma_bf16_pair(acc, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, (kb | k) ? 1u : 0u);
+          if (I8) tc_mma_i8_pair(acc, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, (kb | k) ? 1u : 0u);
+          else if (BF16) tc_mma_bf16_pair(acc, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, (kb | k) ? 1u : 0u);
           else tc_mma_f8_pair(acc, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc, (kb | k) ? 1u : 0u);
         tc_commit_pair(smem_u32(&bar_empty[s]));                             // the stage is free in both blocks
         if (kb == nkb - 1) tc_commit_pair(smem_u32(&bar_acc_full[seg & 1]));  // accumulator complete, both blocks
@@ -323,7 +337,14 @@ __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constan
           for (int j = 0; j < 16; j++) {
             const int tok = tok0 + j, k = (j & 8) * 2 + (j & 7);
             if (tok < a.M && n < a.N) {
-              const float v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
+              float v;
+              if constexpr (I8) {
+                const int hi = (int)r[k], lo = (int)r[k + 8];
+                // 128 * hi + lo stays below 2^31 up to here (lo <= 64 * 127 * K <= 2^30); larger sums in 64 bits
+                v = abs(hi) < (1 << 23) ? __int2float_rn(hi * 128 + lo) : __ll2float_rn((int64_t)hi * 128 + (int64_t)lo);
+              } else {
+                v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
+              }
               const float y = __fmul_rn(__fmul_rn(v, a.sx[tok]), swn);
               if (a.out_f32) ((float*)a.out)[(int64_t)tok * a.N + n] = y;
               else ((bf16*)a.out)[(int64_t)tok * a.N + n] = __float2bfloat16_rn(y);
@@ -399,6 +420,9 @@ static int launch_f8(strictb200_ctx* ctx, const GemmArgs& g) {
 
 // Y = ((X . Wq^T) * sx) * sw for many tokens (prefill). ERR_UNSUPPORTED for shapes this kernel does not take.
 int k_gemm_fp8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) { return launch_f8<PAIR_F8>(ctx, g); }
+
+// The same product of int8 operands (gemm_int8.cu), which all fits as above. 2048 tokens, 4096 x 4096: see k_gemm_int8w.
+int k_gemm_int8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) { return launch_f8<PAIR_I8>(ctx, g); }
 
 // bf16 silu(gate) * up [M, N/2] of the same product with W = [gate | up], where the many-token kernel takes the shape.
 bool sb_gemm_fp8_swiglu_fits(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K) {

@@ -27,7 +27,7 @@ def test_prompts_vs_oracle(ctx, oracle, over, lens):
     st.close(), om.close()
 
 
-@pytest.mark.parametrize("K", [2048, 2056, 4096, 4104, 12288, 12296, 16384])
+@pytest.mark.parametrize("K", [2048, 2064, 4096, 4112, 12288, 12304, 16384])
 def test_quantize_rows_widths(ctx, oracle, rng, K):
     M = 9
     x = oracle.round_bf16((rng.standard_normal((M, K)) * rng.uniform(0.01, 30, (M, 1))).astype(np.float32))
@@ -38,4 +38,36 @@ def test_quantize_rows_widths(ctx, oracle, rng, K):
     q, s = oracle.split_rows_device_layout(x)
     assert np.array_equal(ds.to_host(), s) and np.array_equal(dq.to_host().reshape(32, K), q)
     for v in (dx, dq, ds):
+        v.free()
+
+
+# one, two, four and eight column groups per thread, wider rows, widths that are no multiple of 8
+@pytest.mark.parametrize("M,K", [(1, 2048), (9, 2056), (16, 4104), (7, 8200), (3, 16384), (5, 16392), (10, 1028), (2, 13)])
+def test_quantize_rows_int8_widths(ctx, oracle, rng, M, K):
+    x = oracle.round_bf16((rng.standard_normal((M, K)) * rng.uniform(0.01, 30, (M, 1))).astype(np.float32))
+    x[M // 2, K - 1] = 300.0  # the largest value in the last column
+    rows = 16 * ((M + 7) // 8)
+    dx, dq, ds = DV.of(ctx, oracle.f32_to_bf16(x)), DV(ctx, rows * K, np.int8), DV(ctx, M)
+    N.check(L().strictb200_memset(ctx.h, dq.p, 0x55, rows * K))
+    N.check(L().strictb200_quantize_rows_int8(ctx.h, dx.p, M, K, dq.p, ds.p))
+    hi, lo, s = oracle.quantize_rows_int8(x)
+    want = np.zeros((rows // 2, 2, K), np.int8)
+    want[:M, 0], want[:M, 1] = hi, lo
+    assert np.array_equal(dq.to_host().reshape(rows // 16, 2, 8, K), want.reshape(rows // 16, 8, 2, K).transpose(0, 2, 1, 3))
+    assert np.array_equal(ds.to_host(), s)
+    for v in (dx, dq, ds):
+        v.free()
+
+
+# tiles of 256 channels and 128 tokens that end inside, more than eight token tiles; sums beyond 32 bits (the last)
+@pytest.mark.parametrize("M,N_,K", [(129, 256, 128), (250, 272, 384), (1100, 528, 256), (140, 400, 16384)])
+def test_gemm_int8_many_rows_exact(ctx, oracle, rng, M, N_, K):
+    x = oracle.round_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    wq, sw = rng.integers(-127, 128, (N_, K)).astype(np.int8), rng.uniform(0.01, 1, N_).astype(np.float32)
+    if K > 8192:
+        x[1], x[2], wq[3] = 5.0, -5.0, 127
+    dx, dw, ds, dy = DV.of(ctx, oracle.f32_to_bf16(x)), DV.of(ctx, wq), DV.of(ctx, sw), DV(ctx, M * N_, np.uint16)
+    N.check(L().strictb200_gemm_int8w(ctx.h, M, N_, K, dx.p, dw.p, ds.p, dy.p))
+    assert np.array_equal(dy.to_host().reshape(M, N_), oracle.gemm_int8w(x, wq, sw))
+    for v in (dx, dw, ds, dy):
         v.free()
