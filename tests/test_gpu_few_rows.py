@@ -1,0 +1,30 @@
+"""Linear layers of a decode step's few rows."""
+import numpy as np
+import pytest
+
+from strict_b200 import native as N
+from strict_b200.kernel import DeviceVariable as DV
+
+pytestmark = pytest.mark.gpu
+L = N.lib
+
+
+# one and two groups of 8 rows; channels around a block's 32 and 64; columns around a load's 32, a unit of 64, the 1024 a block holds ahead, and
+# more of them; grids beyond two blocks per SM (two tiles per block); the largest matrix of the kernel and one beyond
+@pytest.mark.parametrize("M,N_,K", [(1, 1, 8), (8, 31, 24), (9, 33, 40), (16, 64, 1024), (3, 100, 1032), (5, 40, 5000), (8, 9600, 136), (13, 9599, 1024),
+                                    (8, 16384, 1024), (2, 16385, 1024), (17, 64, 64)])
+def test_gemm_bf16_few_rows(ctx, oracle, rng, M, N_, K):
+    x = oracle.round_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w = oracle.round_bf16((rng.standard_normal((N_, K)) * 0.05).astype(np.float32))
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    dx, dw, dy = DV.of(ctx, oracle.f32_to_bf16(x)), DV.of(ctx, oracle.f32_to_bf16(w)), DV(ctx, M * N_)
+    N.check(L().strictb200_gemm_bf16(ctx.h, M, N_, K, dx.p, dw.p, dy.p, 1))
+    got = dy.to_host().reshape(M, N_)
+    # exact products; at most one cut-off (2^-23) per product instruction and per addition of the warps' sums, of the sum of the magnitudes
+    assert (np.abs(got - want) <= (K / 16 + 8) * 2.0 ** -23 * size).all()
+    N.check(L().strictb200_gemm_bf16(ctx.h, M, N_, K, dx.p, dw.p, dy.p, 0))
+    half = dy.to_host().view(np.uint16)[:M * N_].reshape(M, N_)
+    assert np.array_equal(half, oracle.f32_to_bf16(got).reshape(M, N_))
+    for v in (dx, dw, dy):
+        v.free()
