@@ -706,8 +706,9 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
   // At most 8 chunks per sequence: that is what the fast merge kernel takes. 16 chunks for the few
   // (sequence, head) pairs of TP=8 shortened the attention kernel but the general merge kernel they
   // need cost more than that (21.9 against 17.0 us per layer for the pair, measured on eight GPUs).
+  // Short caches get chunks of one or two tiles while the grid stays in one wave (8 sequences of 544 keys, 8 KV heads: chunks of 256 keys
+  // walked four tiles one after the other on some SMs and one on others, 8.7 us; chunks of 128, 5.7 us).
   for (int c = (tiles + 7) / 8; c <= tiles; c++) {
-    if (c < 4 && c < tiles) continue;  // at least 256 keys per block
     // (counting a stub as a whole block is deliberate: weighting blocks by their length made the rule pick three long
     // chunks where five short ones measured 47 us against 66)
     const int64_t blocks = pairs * ((tiles_plan + c - 1) / c), waves = (blocks + slots - 1) / slots;
