@@ -481,7 +481,8 @@ static int gemm_entry(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, cons
   g.splits = 1;
   // few tokens, automatic kernel choice: the job is a stream of weights, so K is split until the
   // grid covers the GPU and a second kernel sums the partial results
-  const int splits = (kernel == 0 || kernel == 3) && N % 4 == 0 ? sb_gemm_pick_splits(ctx, M, N, K) : 1;
+  if (kernel == 0 && sb_gemm_rows_takes(M, N, K, true, true)) g.kernel = 4;
+  const int splits = N % 4 || (kernel != 0 && kernel != 3) || M > 128 || K % 128 ? 1 : g.kernel == 4 ? sb_gemm_rows_splits(ctx, N, K, true) : sb_pick_splits_kb(ctx, M, N, K / 128);
   if (splits > 1) {
     void* ws;
     SB_TRY(sb_ws2(ctx, (size_t)splits * M * N * sizeof(float), &ws));

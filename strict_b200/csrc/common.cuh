@@ -300,7 +300,7 @@ struct GemmArgs {
   float* part = nullptr;        // [splits][M,N] raw accumulators (when splits > 1 or raw)
   int splits = 1;
   int raw = 0;                  // 1: always write raw accumulators to part, even for splits == 1
-  int kernel = 0;               // 0 auto, 1 skinny, 2 mma.sync tiles, 3 tcgen05
+  int kernel = 0;               // 0 auto, 1 skinny, 2 mma.sync tiles, 3 tcgen05, 4 few rows (gemm_rows.cu)
   int i8 = 0;                   // 1: int8 weights and two int8 activation terms (gemm_int8.cu); part then holds int32 sums [splits][2][M,N]
 };
 int k_gemm_fp8(strictb200_ctx*, const GemmArgs& a);
@@ -308,6 +308,9 @@ int k_gemm_fp8(strictb200_ctx*, const GemmArgs& a);
 bool sb_gemm_fp8_swiglu_fits(strictb200_ctx*, int64_t M, int64_t N, int64_t K);
 int k_gemm_fp8_swiglu(strictb200_ctx*, const GemmArgs& a);
 int sb_gemm_pick_splits(strictb200_ctx*, int64_t M, int64_t N, int64_t K);
+// gemm_rows.cu: at most 16 rows
+bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished);
+int sb_gemm_rows_splits(strictb200_ctx*, int64_t N, int64_t K, bool f8);
 int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
 // gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
 // Where a finished value goes. Columns from n_switch on (0 = none) belong to a second product of the same launch: its

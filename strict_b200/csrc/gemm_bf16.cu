@@ -5,13 +5,11 @@
 
 int k_gemm_bf16_tmem_split(strictb200_ctx* ctx, const GemmBf16Args& g);  // gemm_tmem_split.cu
 int k_gemm_bf16_tmem_pair(strictb200_ctx* ctx, const GemmBf16Args& g);   // gemm_tmem_pair.cu
-bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K);                // gemm_rows.cu
-int sb_gemm_rows_splits(strictb200_ctx* ctx, int64_t N, int64_t K);
-int k_gemm_rows_bf16(strictb200_ctx* ctx, const GemmBf16Args& g);
+int k_gemm_rows_bf16(strictb200_ctx* ctx, const GemmBf16Args& g);         // gemm_rows.cu
 
 int sb_gemm_bf16_splits(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K) {
   if (M > 128) return 1;
-  if (sb_gemm_rows_takes(M, N, K)) return sb_gemm_rows_splits(ctx, N, K);
+  if (sb_gemm_rows_takes(M, N, K, false, false)) return sb_gemm_rows_splits(ctx, N, K, false);
   return sb_pick_splits_kb(ctx, M, N, (K + 63) / 64);
 }
 
@@ -23,7 +21,7 @@ int k_gemm_bf16(strictb200_ctx* ctx, const GemmBf16Args& g) {
   if (g.e.n_switch % 256) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_bf16: the second product must begin at a multiple of 256 columns");
   const Bf16Epilogue& e = g.e;
   const bool plain = g.part || (g.splits == 1 && !e.accumulate && !e.act_out && !e.col_scale && e.alpha == 1.f);
-  if (plain && sb_gemm_rows_takes(g.M, g.N, g.K)) return k_gemm_rows_bf16(ctx, g);
+  if (plain && sb_gemm_rows_takes(g.M, g.N, g.K, false, !g.part)) return k_gemm_rows_bf16(ctx, g);
   if (g.M <= 128 || (g.part && g.M <= 256)) return k_gemm_bf16_tmem_split(ctx, g);
   if (!g.part) return k_gemm_bf16_tmem_pair(ctx, g);
   if (g.splits != 1) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_bf16: K splits are for at most 256 tokens");

@@ -4,7 +4,8 @@
 // 2M operand rows and the epilogue adds acc_hi + acc_lo/16, so every product is exact and no
 // weight is ever dequantised in the kernel.
 //
-// Three kernels, chosen by shape:
+// Kernels, chosen by shape:
+//  * at most 16 tokens and not too many weights: gemm_rows.cu
 //  * skinny (M <= 32, decode): an HBM stream over the weights. Each warp owns 16 output
 //    channels and walks K with 128-bit loads straight from global memory into mma.sync
 //    m16n8k32 A-fragments (weights are the A operand, tokens the B operand, so no row of
@@ -23,6 +24,7 @@
 #include "common.cuh"
 
 int k_gemm_fp8_tmem(strictb200_ctx* ctx, const GemmArgs& a);  // gemm_tmem.cu
+int k_gemm_rows_fp8(strictb200_ctx* ctx, const GemmArgs& a);  // gemm_rows.cu
 
 namespace {
 
@@ -263,6 +265,7 @@ int launch_skinny(strictb200_ctx* ctx, const GemmDev& d) {
 // Number of K splits for a skinny GEMM so that the grid covers the SMs about twice.
 int sb_gemm_pick_splits(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K) {
   if (M > 128 || K % 128) return 1;
+  if (sb_gemm_rows_takes(M, N, K, true, false)) return sb_gemm_rows_splits(ctx, N, K, true);
   return sb_pick_splits_kb(ctx, M, N, K / 128);
 }
 int sb_pick_splits_kb(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t nkb) {
@@ -292,7 +295,8 @@ int k_gemm_fp8(strictb200_ctx* ctx, const GemmArgs& g) {
     return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_fp8: operands and row strides must be 16-byte aligned");
   if (g.M > INT32_MAX || g.N > INT32_MAX || g.K > INT32_MAX) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_fp8: dimension too large");
   int kernel = g.kernel;
-  if (kernel == 0) kernel = 3;
+  if (kernel == 0) kernel = sb_gemm_rows_takes(g.M, g.N, g.K, true, !g.raw && g.splits == 1) ? 4 : 3;
+  if (kernel == 4) return k_gemm_rows_fp8(ctx, g);
   if (kernel == 3) {
     int st = k_gemm_fp8_tmem(ctx, g);
     if (st != STRICTB200_ERR_UNSUPPORTED || g.kernel == 3) return st;

@@ -216,7 +216,7 @@ int strictb200_gemm_int8(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, c
   if (!M) return STRICTB200_OK;
   SB_REQUIRE(d_split && d_sx && d_wq && d_sw && d_y_bf16, "null pointer");
   SB_REQUIRE((((uintptr_t)d_wq | (uintptr_t)d_split) & 15) == 0, "the operands must be 16-byte aligned");
-  const int splits = sb_gemm_pick_splits(ctx, M, N, K);
+  const int splits = M > 128 ? 1 : sb_pick_splits_kb(ctx, M, N, K / 128);
   void* ws = nullptr;
   if (splits > 1) SB_TRY(sb_ws(ctx, (size_t)splits * 2 * M * N * 4, &ws));
   return k_gemm_int8w(ctx, M, N, K, d_split, d_sx, d_wq, d_sw, (bf16*)d_y_bf16, splits, (int32_t*)ws);
@@ -231,7 +231,7 @@ int strictb200_gemm_int8w(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, 
   if (!M) return STRICTB200_OK;
   SB_REQUIRE(d_x_bf16 && d_wq && d_sw && d_y_bf16, "null pointer");
   SB_REQUIRE(((uintptr_t)d_wq & 15) == 0, "the weights must be 16-byte aligned");
-  const int splits = sb_gemm_pick_splits(ctx, M, N, K);
+  const int splits = M > 128 ? 1 : sb_pick_splits_kb(ctx, M, N, K / 128);
   const size_t qbytes = ((size_t)sb_qrows(M) * K + 255) & ~(size_t)255, sbytes = ((size_t)M * 4 + 255) & ~(size_t)255;
   const size_t pbytes = splits > 1 ? (size_t)splits * 2 * M * N * 4 : 0;
   void* ws;

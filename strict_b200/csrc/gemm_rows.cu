@@ -1,4 +1,4 @@
-// bf16 linear layers of a decode step's few rows: Y[M,N] = X[M,K] . W[N,K]^T with at most 16 rows of X.
+// Linear layers of a decode step's few rows, bf16 or E4M3 weights: Y[M,N] = X[M,K] . W[N,K]^T with at most 16 rows of X.
 //
 // Bound by the stream over W, and in the chain of a decode step by what lies between the dependency wait and the last store. A tile of
 // 128 channels per block (gemm_tmem_split.cu) leaves 8 to 64 blocks for the 1024 channels of an output product, each of which pulls its
@@ -8,19 +8,24 @@
 // of two products (the columns of a fragment may come in any order as long as W and X agree), so no operand passes shared memory.
 // The legacy tensor path is enough: one product of 32 channels x 16 columns per 1 KB of weights.
 // Where such blocks would not all be resident (two per SM hold 19 MB in registers) a block takes a second tile of 32 channels, whose weights
-// wait in shared memory, each thread's own where it put them: 38 MB are on their way before the wait.
+// wait in shared memory, each thread's own where it put them: 38 MB are on their way before the wait (bf16 only).
+// E4M3: a load is 16 columns. Weights become fp16 pairs, and so does the sum of the two E4M3 terms of X, hi + lo / 16 (both without
+// rounding: the sum has at most 9 significant bits down to units of 2^-13), so one product serves both terms.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
 constexpr int TILE = 32;     // channels per block
 constexpr int WARPS = 8;
-constexpr int STEP = 32;     // columns per load
-constexpr int AHEAD = 4;     // steps whose weights a warp holds at a time
+// Loads per weight row that a thread holds at a time; a load of a warp is 64 bytes of a row (a step). E4M3 weights are held as fp16.
+constexpr int ahead(bool f8) { return f8 ? 2 : 4; }
 
 struct RowsArgs {
-  const bf16 *x, *w;
-  int64_t ldx, ldw;
+  const void *x, *w;
+  int64_t ldx, ldw;             // elements
   int M, N, K, splits;
+  const float *sx, *sw;         // E4M3: scales of the rows of X and of the channels (finished outputs)
   int kb_switch, splits0;       // in units of 64 columns, as in GemmBf16Args::k_switch
   int n_switch, x_row_off;      // rows of x of the channels from n_switch on (n_switch 0: all read the first rows)
   int group_n;
@@ -31,16 +36,34 @@ struct RowsArgs {
   int64_t ldo;
 };
 
+template <bool F16>
 __device__ __forceinline__ void mma_rows(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  if constexpr (F16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Four E4M3 values -> two fp16 pairs (exact).
+__device__ __forceinline__ void unpack4(uint32_t v, uint32_t* h) {
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;\n\t}" : "=r"(h[0]), "=r"(h[1]) : "r"(v));
+}
+__device__ __forceinline__ uint32_t join_terms(uint32_t hi, uint32_t lo) {  // hi + lo / 16
+  uint32_t v;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(0x2C002C00u), "r"(hi));
+  return v;
 }
 
 // NT: groups of 8 rows of X. TWO: a second tile of channels, through shared memory (for at most AHEAD steps per warp).
-template <int NT, bool TWO>
+template <bool F8, int NT, bool TWO>
 __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
   constexpr int TILES = TWO ? 2 : 1, CH = TILES * TILE;
+  constexpr int AHEAD = ahead(F8), WORDS = F8 ? 8 : 4;  // words of a load, as operands
+  constexpr int COLS = F8 ? 16 : 8, STEP = 4 * COLS;    // columns of a thread's load and of a warp's
+  using T = std::conditional_t<F8, uint8_t, bf16>;
   extern __shared__ __align__(16) uint4 second[];  // [AHEAD * 4][threads]
   __shared__ float red[WARPS][8 * NT][CH + 4];     // the fragments of a warp in 32 banks
   SB_TRACE_BEGIN();
@@ -59,34 +82,43 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
     u0 = (int)((int64_t)z * units / a.splits);
     u1 = (int)((int64_t)(z + 1) * units / a.splits);
   }
-  // the warp's columns, in steps of 32
-  const int steps_all = 2 * (u1 - u0), s0 = 2 * u0 + warp * steps_all / WARPS, s1 = 2 * u0 + (warp + 1) * steps_all / WARPS;
-  const bf16* wr = a.w + (int64_t)(n0 + g) * a.ldw + 8 * t;
+  // the warp's steps
+  constexpr int PER = 64 / STEP;  // steps per unit
+  const int steps_all = PER * (u1 - u0), s0 = PER * u0 + warp * steps_all / WARPS, s1 = PER * u0 + (warp + 1) * steps_all / WARPS;
+  const T* wr = (const T*)a.w + (int64_t)(n0 + g) * a.ldw + COLS * t;
   const int64_t xk = a.group_n > 0 ? n0 / a.group_n * a.group_k : 0;
-  const bf16* xr = a.x + (int64_t)((a.n_switch > 0 && n0 >= a.n_switch ? a.x_row_off : 0) + g) * a.ldx + xk + 8 * t;
+  const T* xr = (const T*)a.x + (int64_t)((a.n_switch > 0 && n0 >= a.n_switch ? a.x_row_off : 0) + g) * a.ldx + xk + COLS * t;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  uint4 w[AHEAD][4], x[AHEAD][NT];
+  uint32_t w[AHEAD][4][WORDS], x[AHEAD][NT][WORDS];
+  auto unpack = [](const uint4& u, uint32_t* o) {
+    if constexpr (F8) { unpack4(u.x, o); unpack4(u.y, o + 2); unpack4(u.z, o + 4); unpack4(u.w, o + 6); }
+    else { o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w; }
+  };
   auto load_w = [&](int s) {
+    uint4 raw[AHEAD][4];
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int k = (s + i) * STEP;
-        w[i][r] = s + i < s1 && k + 8 * t < a.K && n0 + g + 8 * r < a.N ? __ldcs((const uint4*)(wr + (int64_t)(8 * r) * a.ldw + k)) : zero;
+        raw[i][r] = s + i < s1 && k + COLS * t < a.K && n0 + g + 8 * r < a.N ? __ldcs((const uint4*)(wr + (int64_t)(8 * r) * a.ldw + k)) : zero;
       }
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) unpack(raw[i][r], w[i][r]);
   };
-  load_w(s0);  // weights are constants
+  load_w(s0);  // weights are constants, and E4M3 ones are converted before the wait too (the conversions took longer than all that follows)
   if constexpr (TWO) {
-    const uint64_t once = l2_evict_first_policy();
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int k = (s0 + i) * STEP;
-        const bool in = s0 + i < s1 && k + 8 * t < a.K && n0 + TILE + g + 8 * r < a.N;
-        const bf16* from = in ? wr + (int64_t)(TILE + 8 * r) * a.ldw + k : a.w;
+        const bool in = s0 + i < s1 && k + COLS * t < a.K && n0 + TILE + g + 8 * r < a.N;
+        const T* from = in ? wr + (int64_t)(TILE + 8 * r) * a.ldw + k : (const T*)a.w;
         const uint32_t to = (uint32_t)__cvta_generic_to_shared(second + (i * 4 + r) * 32 * WARPS + threadIdx.x);
-        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(to), "l"(from), "r"(in ? 16 : 0), "l"(once) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
       }
   }
   pdl_wait();
@@ -102,20 +134,35 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
 #pragma unroll
       for (int j = 0; j < NT; j++)
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          float* c = acc[2 * tile + h][j];
-          mma_rows(c, w[i][2 * h].x, w[i][2 * h + 1].x, w[i][2 * h].y, w[i][2 * h + 1].y, x[i][j].x, x[i][j].y);
-          mma_rows(c, w[i][2 * h].z, w[i][2 * h + 1].z, w[i][2 * h].w, w[i][2 * h + 1].w, x[i][j].z, x[i][j].w);
-        }
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int q = 0; q < WORDS; q += 2)
+            mma_rows<F8>(acc[2 * tile + h][j], w[i][2 * h][q], w[i][2 * h + 1][q], w[i][2 * h][q + 1], w[i][2 * h + 1][q + 1], x[i][j][q], x[i][j][q + 1]);
   };
+  constexpr int TERMS = F8 ? 2 : 1;
   for (int s = s0; s < s1; s += AHEAD) {
     if (s > s0) load_w(s);
+    uint4 raw[AHEAD][NT][TERMS];
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int e = 0; e < TERMS; e++) {
+          const int k = (s + i) * STEP;
+          raw[i][j][e] = s + i < s1 && k + COLS * t < a.K && g + 8 * j < a.M ? __ldcg((const uint4*)(xr + (int64_t)(8 * (TERMS * j + e)) * a.ldx + k)) : zero;
+        }
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int j = 0; j < NT; j++) {
-        const int k = (s + i) * STEP;
-        x[i][j] = s + i < s1 && k + 8 * t < a.K && g + 8 * j < a.M ? __ldcg((const uint4*)(xr + (int64_t)(8 * j) * a.ldx + k)) : zero;
+        unpack(raw[i][j][0], x[i][j]);
+        if constexpr (F8) {
+          uint32_t lo[WORDS];
+          unpack(raw[i][j][1], lo);
+#pragma unroll
+          for (int q = 0; q < WORDS; q++) x[i][j][q] = join_terms(x[i][j][q], lo[q]);
+        }
       }
     multiply(0);
     if constexpr (TWO) {
@@ -123,7 +170,7 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
 #pragma unroll
       for (int i = 0; i < AHEAD; i++)
 #pragma unroll
-        for (int r = 0; r < 4; r++) w[i][r] = second[(i * 4 + r) * 32 * WARPS + threadIdx.x];
+        for (int r = 0; r < 4; r++) unpack(second[(i * 4 + r) * 32 * WARPS + threadIdx.x], w[i][r]);
       multiply(1);
     }
   }
@@ -141,6 +188,7 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
     float v = red[0][m][c];
 #pragma unroll
     for (int j = 1; j < WARPS; j++) v += red[j][m][c];
+    if (F8 && !a.part) v = __fmul_rn(__fmul_rn(v, a.sx[m]), a.sw[n]);
     if (a.part) a.part[((int64_t)z * a.M + m) * a.N + n] = v;
     else if (a.out_f32) a.out_f32[m * a.ldo + n] = v;
     else a.out_bf16[m * a.ldo + n] = __float2bfloat16_rn(v);
@@ -148,15 +196,25 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
   SB_TRACE_END(SB_K_GEMM, (uint32_t)a.N ^ ((uint32_t)a.K << 12));
 }
 
-template <int NT, bool TWO>
+template <bool F8, int NT, bool TWO>
 int launch(strictb200_ctx* ctx, const RowsArgs& a) {
-  constexpr size_t smem = TWO ? AHEAD * 4 * 32 * WARPS * sizeof(uint4) : 0;
+  constexpr size_t smem = TWO ? ahead(F8) * 4 * 32 * WARPS * sizeof(uint4) : 0;
   static SbDeviceOnce once;  // one per instantiation
-  if (TWO) SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_rows_kernel<NT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
+  if (TWO) SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_rows_kernel<F8, NT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
   const int ch = TWO ? 2 * TILE : TILE;
-  SB_CUDA(sb_launch(ctx, gemm_rows_kernel<NT, TWO>, dim3((unsigned)((a.N + ch - 1) / ch), (unsigned)a.splits), dim3(32 * WARPS), smem, a));
+  SB_CUDA(sb_launch(ctx, gemm_rows_kernel<F8, NT, TWO>, dim3((unsigned)((a.N + ch - 1) / ch), (unsigned)a.splits), dim3(32 * WARPS), smem, a));
   ctx->launches++;
   return STRICTB200_OK;
+}
+template <bool F8>
+int launch(strictb200_ctx* ctx, const RowsArgs& a) {
+  if constexpr (!F8) {
+    // longest run of columns a block gets, in units of 64
+    const int units = (a.K + 63) / 64, n0 = a.splits0, n1 = a.splits - n0;
+    const int run = n0 ? std::max((a.kb_switch + n0 - 1) / n0, (units - a.kb_switch + n1 - 1) / n1) : (units + n1 - 1) / n1;
+    if ((int64_t)((a.N + TILE - 1) / TILE) * a.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= ahead(F8) * WARPS) return a.M <= 8 ? launch<F8, 1, true>(ctx, a) : launch<F8, 2, true>(ctx, a);
+  }
+  return a.M <= 8 ? launch<F8, 1, false>(ctx, a) : launch<F8, 2, false>(ctx, a);
 }
 }  // namespace
 
@@ -168,20 +226,31 @@ SB_TRACE_TU(gemm_rows)
 //   N 1024  K 5120  25.5 / 25.6 / 25.6 -> 8.6 / 8.7 / 11.3       N 14336 K 4096   23.2 / 23.0 / 23.1, beyond what the blocks hold ahead
 // and error against 64 bits (K 1024 / 5120): 9.8e-7 / 5.6e-6 there (tcgen05 cuts off after every instruction), 1.3e-7 / 6.0e-7 here.
 // A decode step of 8 sequences (28 layers of latent attention, 1024 wide): 926 -> 763 us.
-bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K) { return M <= 16 && K % 8 == 0 && N * K <= (16 << 20); }
-int sb_gemm_rows_splits(strictb200_ctx* ctx, int64_t N, int64_t K) {
-  const int64_t tiles = (N + TILE - 1) / TILE, units = (K + 63) / 64;
-  int64_t s = (K + STEP * AHEAD * WARPS - 1) / (STEP * AHEAD * WARPS);             // every weight in registers before the wait
-  s = std::max(s, std::min((int64_t)ctx->sm_count / tiles, units / 4));           // a block per SM, while a warp has a step
+// Beyond 32 MB of weights the rows of X, which every block reads, and the later rounds of blocks cost more than the K splits of the large
+// tiles; a finished product has no K splits there, and with few tiles it stays here (4096 x 14336: 66.8 -> 26.7 us with 8 rows, 38.3 with 16;
+// 14336 x 4096: 23.2 -> 21.1 with 8, but 28.2 with 16; 28672 x 4096 36.2 -> 37.7).
+// E4M3 weights, whose large tiles are half as long a stream and whose conversion is work here: 1 / 16 rows, us, the row split in front included,
+//   N 4096 K 1024  8.1 / 8.0 -> 5.9 / 5.9     N 1024 K 3072  8.1 / 8.4 -> 7.9 / 7.9     N 1024 K 14336  12.4 / 12.8 -> 10.8 / 12.6
+//   N 6144 K 1024  8.1 / 8.0 -> 5.8 / 5.8     N 4096 K 4096  9.6 / 10.6, 9.9 / 12.6 here; N 6144 K 4096  10.4 / 11.0, 13.1 / 16.9 here
+// A decode step of Qwen3-0.6B: 774 -> 711 us (batch 1).
+bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished) {
+  if (M > 16 || K % (f8 ? 16 : 8)) return false;
+  const int64_t weights = N * K;
+  if (f8) return weights <= (8 << 20) || (N <= 1024 && weights <= (16 << 20));
+  return weights <= (16 << 20) || (finished && (N <= 8192 || (M <= 8 && weights <= (64 << 20))));
+}
+int sb_gemm_rows_splits(strictb200_ctx* ctx, int64_t N, int64_t K, bool f8) {
+  const int64_t tiles = (N + TILE - 1) / TILE, units = (K + 63) / 64, held = ahead(f8) * WARPS / (f8 ? 1 : 2);
+  int64_t s = (units + held - 1) / held;                                          // every weight in registers before the wait
+  s = std::max(s, std::min((int64_t)ctx->sm_count / tiles, units / (f8 ? 8 : 4)));  // a block per SM, while every warp has a step
   return (int)std::max<int64_t>(1, std::min<int64_t>(s, 8));                       // eight results are what the consumers take
 }
 int k_gemm_rows_bf16(strictb200_ctx* ctx, const GemmBf16Args& b) {
-  const RowsArgs a{b.x, b.w, b.ldx, b.ldw, (int)b.M, (int)b.N, (int)b.K, b.splits, (int)(b.k_switch / 64), b.k_switch ? b.splits0 : 0,
-                   b.e.n_switch, b.e.x_row_off, b.group_n, b.group_k, b.part, b.e.out_f32, b.e.out_bf16, b.e.ldo};
-  // longest run of columns a block gets, in units of 64
-  const int64_t units = (b.K + 63) / 64, u0 = b.k_switch ? b.k_switch / 64 : 0;
-  const int64_t run = b.k_switch ? std::max((u0 + b.splits0 - 1) / b.splits0, (units - u0 + b.splits - b.splits0 - 1) / (b.splits - b.splits0)) : (units + b.splits - 1) / b.splits;
-  const bool two = (b.N + TILE - 1) / TILE * b.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= AHEAD * WARPS;
-  if (b.M <= 8) return two ? launch<1, true>(ctx, a) : launch<1, false>(ctx, a);
-  return two ? launch<2, true>(ctx, a) : launch<2, false>(ctx, a);
+  return launch<false>(ctx, RowsArgs{b.x, b.w, b.ldx, b.ldw, (int)b.M, (int)b.N, (int)b.K, b.splits, nullptr, nullptr, (int)(b.k_switch / 64), b.k_switch ? b.splits0 : 0,
+                                     b.e.n_switch, b.e.x_row_off, b.group_n, b.group_k, b.part, b.e.out_f32, b.e.out_bf16, b.e.ldo});
+}
+int k_gemm_rows_fp8(strictb200_ctx* ctx, const GemmArgs& g) {
+  const bool part = g.raw || g.splits > 1;
+  return launch<true>(ctx, RowsArgs{g.xq, g.wq, g.ldx, g.ldw, (int)g.M, (int)g.N, (int)g.K, g.splits, g.sx, g.sw, 0, 0, 0, 0, 0, 0, part ? g.part : nullptr,
+                                    g.out_f32 ? (float*)g.out : nullptr, g.out_f32 ? nullptr : (bf16*)g.out, g.N});
 }

@@ -28,3 +28,27 @@ def test_gemm_bf16_few_rows(ctx, oracle, rng, M, N_, K):
     assert np.array_equal(half, oracle.f32_to_bf16(got).reshape(M, N_))
     for v in (dx, dw, dy):
         v.free()
+
+
+# the same of E4M3 weights: loads of 64 columns, 1024 columns per block, sums of several blocks per output
+@pytest.mark.parametrize("M,N_,K", [(1, 16, 64), (8, 48, 192), (9, 32, 1088), (16, 1024, 2048), (5, 1600, 4160), (8, 15984, 512), (13, 7600, 1024),
+                                    (3, 768, 14336), (4, 1024, 3072), (16, 2080, 4096)])
+def test_gemm_fp8_few_rows(ctx, oracle, rng, M, N_, K):
+    import torch
+    x = oracle.round_bf16((rng.standard_normal((M, K)) * np.exp2(rng.integers(-12, 3, (M, K)))).astype(np.float32))
+    q, s = oracle.split_rows_device_layout(x)
+    wq = rng.integers(0, 256, (N_, K)).astype(np.uint8)
+    wq[(wq & 127) == 127] = 0  # no NaN
+    f64 = lambda a: torch.from_numpy(a).view(torch.float8_e4m3fn).to(torch.float64).numpy()  # noqa: E731
+    terms = f64(q.reshape(-1, K)).reshape(-1, 2, 8, K)
+    xs = (terms[:, 0] + terms[:, 1] / 16).reshape(-1, K)[:M] * s[:, None].astype(np.float64)
+    sw = rng.uniform(0.5, 2, N_).astype(np.float32)
+    w = f64(wq)
+    want, size = xs @ w.T * sw, np.abs(xs) @ np.abs(w).T * sw
+    dq, ds, dw, dsw, dy = DV.of(ctx, q), DV.of(ctx, s), DV.of(ctx, wq), DV.of(ctx, sw), DV(ctx, M * N_)
+    N.check(L().strictb200_gemm_fp8(ctx.h, M, N_, K, dq.p, ds.p, dw.p, dsw.p, dy.p, 1, 0))
+    got = dy.to_host().reshape(M, N_)
+    # as above, eight more additions between blocks and the two scales
+    assert (np.abs(got - want) <= (K / 16 + 18) * 2.0 ** -23 * size).all()
+    for v in (dq, ds, dw, dsw, dy):
+        v.free()
