@@ -106,7 +106,7 @@ int strictb200_trace_end(strictb200_ctx* ctx, uint64_t* out_records, int max_rec
  * "attn_blocks_per_sm" (0), "split_target" (0), "tp_two_shot" (fused all-reduce in two shots,
  * -1: with more than four ranks), "wait_limit" (polls of a cross-rank wait before it gives up,
  * 4194304), "prefill_chunk" (token rows per prefill chunk, 16384), "fuse_rope" (decode attention applies
- * QK-norm and RoPE and appends to the cache itself, 0), "row_cluster" (blocks of one cluster that share a row in the decode row
+ * QK-norm and RoPE and appends to the cache itself, -1: with at most 16 sequences and an unsplit projection), "row_cluster" (blocks of one cluster that share a row in the decode row
  * kernels, 4), "attn_prefetch" (decode attention loads its first key/value
  * tiles before the dependency wait, 1), "blur_rows" (image rows per block of the
  * blur kernel, 0 = 8), "host_timeout_ms" (under tensor

@@ -698,7 +698,7 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
     resident_fused_of[ctx->device & 63] = r;
     return cudaSuccess;
   });
-  const int res0 = (ctx->opt.fuse_rope ? resident_fused_of : resident_of)[ctx->device & 63];
+  const int res0 = (ctx->opt.fuse_rope > 0 ? resident_fused_of : resident_of)[ctx->device & 63];
   const int resident = res0 > 0 ? res0 : 1;
   const int64_t slots = (int64_t)ctx->sm_count * resident, pairs = (int64_t)B * Hkv;
   int best = tiles;

@@ -59,7 +59,7 @@ struct SbOptions {
   int tp_two_shot = -1;        // fused all-reduce: 0 one shot, 1 two shots
   int wait_limit = 1 << 22;    // polls of a cross-rank wait before the kernel gives up and sets the error word
   int prefill_chunk = 16384;   // token rows per prefill chunk
-  int fuse_rope = 0;           // decode step: QK-norm, RoPE and the cache append inside the attention kernel (bit-identical; measured no faster)
+  int fuse_rope = -1;          // decode step: QK-norm, RoPE and the cache append inside the attention kernel (bit-identical); -1: at most 16 sequences
   int row_cluster = 4;         // blocks (one cluster) per row of the decode row kernels, where the row has 1024 columns per block; 0 or 1 = one block per row
   int attn_prefetch = 1;       // decode attention starts to load its first key/value tiles before the dependency wait
   int blur_rows = 0;           // rows of the image per block of the blur kernel; 0 = chosen from the image and the grid

@@ -197,7 +197,10 @@ int qwen_decode_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
     r.q_out = b.qb; r.kcache = kv_k(kv, l); r.vcache = kv_v(kv, l);
     // QK-norm, RoPE and the cache append inside the attention kernel (one kernel less per layer), or as a kernel of their own.
     // The merge kernel overwrites b.sa (the o_proj operand's scales) only after every attention block has read it.
-    const bool fuse_rope = ctx->opt.fuse_rope && s1 <= 8 && m->Hq_l / m->Hkv_l <= 16;
+    // By itself where a step is a chain of short kernels and the projection is one result that every key chunk's block may read: Qwen3-0.6B
+    // 713 -> 698 us (batch 1), 812 -> 789 (batch 8); Qwen3-8B at batch 32 (five partial results) 3986 -> 3964, within what two runs differ.
+    const int fuse = ctx->opt.fuse_rope;
+    const bool fuse_rope = (fuse < 0 ? B <= 16 && s1 == 1 : fuse > 0) && s1 <= 8 && m->Hq_l / m->Hkv_l <= 16;
     if (!fuse_rope) PROF(STRICTB200_K_ROPE, k_rope_qknorm_kvappend(ctx, r, B));
     // split-KV attention over len+1 keys; the combine emits the quantised o_proj input
     PROF(STRICTB200_K_ATTN, k_attn_decode(ctx, b.qb, kv_k(kv, l), kv_v(kv, l), kv->d_lens, 1, (int)B, m->Hq_l, m->Hkv_l, (int)D, kv->maxlen,
