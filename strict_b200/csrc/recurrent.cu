@@ -28,10 +28,41 @@ __global__ void __launch_bounds__(256) gated_conv_kernel(GatedArgs a, int64_t ro
   const int per_row = ch_blocks + act_blks;
   const int64_t t = blockIdx.x / per_row;
   const int blk = blockIdx.x % per_row, w = a.s.width, taps = a.s.taps;
+  // A decode row: its constants are loaded before the wait and its history in one round trip after it; one after the other they were most
+  // of the kernel (Morarax, 4 sequences: 5.9 -> 2.6 us exposed).
+  const int c0 = blk * 256 + (int)threadIdx.x;
+  const bool step = !a.seq && taps <= 4 && blk < ch_blocks && c0 < w;
+  float kx[4], xb0 = 0.f, cb0 = 0.f;
+  if (step) {
+    xb0 = a.x_bias[c0];
+    cb0 = a.conv_bias[c0];
+#pragma unroll
+    for (int j = 0; j < 4; j++) kx[j] = j < taps ? a.conv[(int64_t)c0 * taps + j] : 0.f;
+  }
   pdl_wait();
   SB_TRACE_WAITED();
   if (blk >= ch_blocks) {
     act_block<T>(a.act, a.p, rows, t, blk - ch_blocks);
+  } else if (step) {
+    float* hist = a.hist + t * (taps - 1) * w + c0;
+    float h[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) h[j] = j < taps - 1 ? hist[(int64_t)j * w] : 0.f;
+    const float now = proj(a.p, rows, t, w + c0) + xb0;
+    float acc = cb0;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (j < taps - 1) acc = fmaf(kx[j], h[j], acc);  // oldest first
+    acc = fmaf(taps == 1 ? kx[0] : taps == 2 ? kx[1] : taps == 3 ? kx[2] : kx[3], now, acc);
+    const int bs = a.s.bs(), g = c0 / bs;
+    T* u = (T*)a.u + t * a.s.ld_u() + (int64_t)g * a.s.bs_p() + c0 - g * bs;
+    *u = to_t<T>(acc);
+    if (c0 - g * bs == bs - 1)
+      for (int j = 1; j <= a.s.bs_p() - bs; j++) u[j] = to_t<T>(0.f);  // as below
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (j < taps - 2) hist[(int64_t)j * w] = h[j + 1];
+    if (taps > 1) hist[(int64_t)(taps - 2) * w] = now;
   } else {
     const int c = blk * 256 + (int)threadIdx.x;
     if (c < w) {
