@@ -311,6 +311,8 @@ int sb_gemm_pick_splits(strictb200_ctx*, int64_t M, int64_t N, int64_t K);
 // gemm_rows.cu: at most 16 rows
 bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished);
 int sb_gemm_rows_splits(strictb200_ctx*, int64_t N, int64_t K, bool f8);
+int k_gemm_rows_glu(strictb200_ctx*, const GemmArgs& g, float* ones);
+int k_gemm_rows_fp8_bf16(strictb200_ctx*, const GemmArgs& g);
 int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
 // gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
 // Where a finished value goes. Columns from n_switch on (0 = none) belong to a second product of the same launch: its

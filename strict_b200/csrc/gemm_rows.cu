@@ -9,8 +9,12 @@
 // The legacy tensor path is enough: one product of 32 channels x 16 columns per 1 KB of weights.
 // Where such blocks would not all be resident (two per SM hold 19 MB in registers) a block takes a second tile of 32 channels, whose weights
 // wait in shared memory, each thread's own where it put them: 38 MB are on their way before the wait (bf16 only).
+// (The two halves of W = [gate | up] of a SwiGLU may share a block, 16 channels of each, which then writes bf16 silu(gate) * up.)
 // E4M3: a load is 16 columns. Weights become fp16 pairs, and so does the sum of the two E4M3 terms of X, hi + lo / 16 (both without
-// rounding: the sum has at most 9 significant bits down to units of 2^-13), so one product serves both terms.
+// rounding: the sum has at most 9 significant bits down to units of 2^-13), so one product serves both terms. Rows of X that come as
+// bf16 are multiplied as they are, by weights that became bf16: no row maximum, no split, no launch for them.
+#include <cuda_fp16.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -25,6 +29,7 @@ struct RowsArgs {
   const void *x, *w;
   int64_t ldx, ldw;             // elements
   int M, N, K, splits;
+  int prefetch;                 // load the weights before the dependency wait
   const float *sx, *sw;         // E4M3: scales of the rows of X and of the channels (finished outputs)
   int kb_switch, splits0;       // in units of 64 columns, as in GemmBf16Args::k_switch
   int n_switch, x_row_off;      // rows of x of the channels from n_switch on (n_switch 0: all read the first rows)
@@ -34,6 +39,7 @@ struct RowsArgs {
   float* out_f32;
   bf16* out_bf16;
   int64_t ldo;
+  float* ones = nullptr;        // GLU: [M]
 };
 
 template <bool F16>
@@ -51,15 +57,26 @@ __device__ __forceinline__ void mma_rows(float* c, uint32_t a0, uint32_t a1, uin
 __device__ __forceinline__ void unpack4(uint32_t v, uint32_t* h) {
   asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;\n\t}" : "=r"(h[0]), "=r"(h[1]) : "r"(v));
 }
+// The same values as bf16 pairs (exact).
+__device__ __forceinline__ void unpack4_bf16(uint32_t v, uint32_t* h) {
+  unpack4(v, h);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const float2 f = __half22float2(*(const __half2*)&h[i]);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h[i]) : "f"(f.y), "f"(f.x));
+  }
+}
 __device__ __forceinline__ uint32_t join_terms(uint32_t hi, uint32_t lo) {  // hi + lo / 16
   uint32_t v;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(0x2C002C00u), "r"(hi));
   return v;
 }
 
-// NT: groups of 8 rows of X. TWO: a second tile of channels, through shared memory (for at most AHEAD steps per warp).
-template <bool F8, int NT, bool TWO>
+enum { ROWS_BF16 = 0, ROWS_F8 = 1, ROWS_F8_BF16 = 2 };  // weights and X bf16; E4M3 and two E4M3 terms; E4M3 and bf16
+// NT: groups of 8 rows of X. GLU: W = [gate | up], both of 16 channels. TWO: a second tile of channels, through shared memory (for at most AHEAD steps per warp).
+template <int KIND, int NT, bool TWO, bool GLU>
 __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
+  constexpr bool F8 = KIND != ROWS_BF16, TERMS2 = KIND == ROWS_F8;
   constexpr int TILES = TWO ? 2 : 1, CH = TILES * TILE;
   constexpr int AHEAD = ahead(F8), WORDS = F8 ? 8 : 4;  // words of a load, as operands
   constexpr int COLS = F8 ? 16 : 8, STEP = 4 * COLS;    // columns of a thread's load and of a warp's
@@ -69,7 +86,7 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
   SB_TRACE_BEGIN();
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * CH, z = blockIdx.y;
+  const int n0 = blockIdx.x * (GLU ? CH / 2 : CH), z = blockIdx.y, half = a.N / 2;
   const int units = (a.K + 63) / 64;
   int u0, u1;  // this block's columns, in units of 64
   if (a.splits0 > 0) {
@@ -87,11 +104,13 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
   const int steps_all = PER * (u1 - u0), s0 = PER * u0 + warp * steps_all / WARPS, s1 = PER * u0 + (warp + 1) * steps_all / WARPS;
   const T* wr = (const T*)a.w + (int64_t)(n0 + g) * a.ldw + COLS * t;
   const int64_t xk = a.group_n > 0 ? n0 / a.group_n * a.group_k : 0;
-  const T* xr = (const T*)a.x + (int64_t)((a.n_switch > 0 && n0 >= a.n_switch ? a.x_row_off : 0) + g) * a.ldx + xk + COLS * t;
+  using TX = std::conditional_t<TERMS2, uint8_t, bf16>;
+  const TX* xr = (const TX*)a.x + (int64_t)((a.n_switch > 0 && n0 >= a.n_switch ? a.x_row_off : 0) + g) * a.ldx + xk + COLS * t;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   uint32_t w[AHEAD][4][WORDS], x[AHEAD][NT][WORDS];
   auto unpack = [](const uint4& u, uint32_t* o) {
-    if constexpr (F8) { unpack4(u.x, o); unpack4(u.y, o + 2); unpack4(u.z, o + 4); unpack4(u.w, o + 6); }
+    if constexpr (KIND == ROWS_F8) { unpack4(u.x, o); unpack4(u.y, o + 2); unpack4(u.z, o + 4); unpack4(u.w, o + 6); }
+    else if constexpr (KIND == ROWS_F8_BF16) { unpack4_bf16(u.x, o); unpack4_bf16(u.y, o + 2); unpack4_bf16(u.z, o + 4); unpack4_bf16(u.w, o + 6); }
     else { o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w; }
   };
   auto load_w = [&](int s) {
@@ -101,13 +120,16 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int k = (s + i) * STEP;
-        raw[i][r] = s + i < s1 && k + COLS * t < a.K && n0 + g + 8 * r < a.N ? __ldcs((const uint4*)(wr + (int64_t)(8 * r) * a.ldw + k)) : zero;
+        const int row = GLU ? (r >> 1) * half + 8 * (r & 1) : 8 * r;  // from the thread's first
+        const bool in = GLU ? n0 + g + 8 * (r & 1) < half : n0 + g + row < a.N;
+        raw[i][r] = s + i < s1 && k + COLS * t < a.K && in ? __ldcs((const uint4*)(wr + (int64_t)row * a.ldw + k)) : zero;
       }
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int r = 0; r < 4; r++) unpack(raw[i][r], w[i][r]);
   };
+  if (!a.prefetch) pdl_wait();
   load_w(s0);  // weights are constants, and E4M3 ones are converted before the wait too (the conversions took longer than all that follows)
   if constexpr (TWO) {
 #pragma unroll
@@ -137,7 +159,7 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
         for (int h = 0; h < 2; h++)
 #pragma unroll
           for (int q = 0; q < WORDS; q += 2)
-            mma_rows<F8>(acc[2 * tile + h][j], w[i][2 * h][q], w[i][2 * h + 1][q], w[i][2 * h][q + 1], w[i][2 * h + 1][q + 1], x[i][j][q], x[i][j][q + 1]);
+            mma_rows<TERMS2>(acc[2 * tile + h][j], w[i][2 * h][q], w[i][2 * h + 1][q], w[i][2 * h][q + 1], w[i][2 * h + 1][q + 1], x[i][j][q], x[i][j][q + 1]);
   };
   constexpr int TERMS = F8 ? 2 : 1;
   for (int s = s0; s < s1; s += AHEAD) {
@@ -150,14 +172,22 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
 #pragma unroll
         for (int e = 0; e < TERMS; e++) {
           const int k = (s + i) * STEP;
-          raw[i][j][e] = s + i < s1 && k + COLS * t < a.K && g + 8 * j < a.M ? __ldcg((const uint4*)(xr + (int64_t)(8 * (TERMS * j + e)) * a.ldx + k)) : zero;
+          // the second load: the lo terms, eight rows further on, or (bf16 beside E4M3) the thread's other eight columns
+          const TX* from = xr + (int64_t)(8 * (TERMS2 ? 2 * j + e : j)) * a.ldx + k + (TERMS2 ? 0 : 8 * e);
+          raw[i][j][e] = s + i < s1 && k + COLS * t < a.K && g + 8 * j < a.M ? __ldcg((const uint4*)from) : zero;
         }
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int j = 0; j < NT; j++) {
+        if constexpr (KIND == ROWS_F8_BF16) {
+          const uint4 lo = raw[i][j][0], hi = raw[i][j][TERMS - 1];
+          x[i][j][0] = lo.x; x[i][j][1] = lo.y; x[i][j][2] = lo.z; x[i][j][3] = lo.w;
+          x[i][j][WORDS - 4] = hi.x; x[i][j][WORDS - 3] = hi.y; x[i][j][WORDS - 2] = hi.z; x[i][j][WORDS - 1] = hi.w;
+          continue;
+        }
         unpack(raw[i][j][0], x[i][j]);
-        if constexpr (F8) {
+        if constexpr (TERMS2) {
           uint32_t lo[WORDS];
           unpack(raw[i][j][1], lo);
 #pragma unroll
@@ -183,7 +213,18 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < TILES * NT; i++) {
-    const int m = 8 * (i / TILES) + warp, c = i % TILES * TILE + lane, n = n0 + c;
+    const int m = 8 * (i / TILES) + warp, c = i % TILES * TILE + lane, n = GLU ? (lane >> 4) * half + n0 + (lane & 15) : n0 + c;
+    if constexpr (GLU) {  // lanes 0..15 hold the gates, the others the up values of the same channels
+      if (m >= a.M) continue;
+      const bool in = n0 + (lane & 15) < half;
+      float v = red[0][m][c];
+#pragma unroll
+      for (int j = 1; j < WARPS; j++) v += red[j][m][c];
+      v = in ? __fmul_rn(__fmul_rn(v, a.sx[m]), a.sw[n]) : 0.f;
+      const float up = __shfl_down_sync(0xffffffffu, v, 16);
+      if (lane < 16 && in) a.out_bf16[m * a.ldo + n] = __float2bfloat16_rn(sb_silu_mul(v, up));
+      continue;
+    }
     if (m >= a.M || n >= a.N) continue;
     float v = red[0][m][c];
 #pragma unroll
@@ -193,28 +234,30 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
     else if (a.out_f32) a.out_f32[m * a.ldo + n] = v;
     else a.out_bf16[m * a.ldo + n] = __float2bfloat16_rn(v);
   }
+  if (GLU && blockIdx.x == 0 && (int)threadIdx.x < a.M) a.ones[threadIdx.x] = 1.f;  // scales of the rows it writes
   SB_TRACE_END(SB_K_GEMM, (uint32_t)a.N ^ ((uint32_t)a.K << 12));
 }
 
-template <bool F8, int NT, bool TWO>
+template <int KIND, int NT, bool TWO, bool GLU = false>
 int launch(strictb200_ctx* ctx, const RowsArgs& a) {
-  constexpr size_t smem = TWO ? ahead(F8) * 4 * 32 * WARPS * sizeof(uint4) : 0;
+  constexpr size_t smem = TWO ? ahead(KIND != ROWS_BF16) * 4 * 32 * WARPS * sizeof(uint4) : 0;
   static SbDeviceOnce once;  // one per instantiation
-  if (TWO) SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_rows_kernel<F8, NT, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
-  const int ch = TWO ? 2 * TILE : TILE;
-  SB_CUDA(sb_launch(ctx, gemm_rows_kernel<F8, NT, TWO>, dim3((unsigned)((a.N + ch - 1) / ch), (unsigned)a.splits), dim3(32 * WARPS), smem, a));
+  auto kernel = gemm_rows_kernel<KIND, NT, TWO, GLU>;
+  if (TWO) SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
+  const int ch = TWO ? 2 * TILE : GLU ? TILE / 2 : TILE, n = GLU ? a.N / 2 : a.N;
+  SB_CUDA(sb_launch(ctx, kernel, dim3((unsigned)((n + ch - 1) / ch), (unsigned)a.splits), dim3(32 * WARPS), smem, a));
   ctx->launches++;
   return STRICTB200_OK;
 }
-template <bool F8>
+template <int KIND>
 int launch(strictb200_ctx* ctx, const RowsArgs& a) {
-  if constexpr (!F8) {
+  if constexpr (KIND == ROWS_BF16) {
     // longest run of columns a block gets, in units of 64
     const int units = (a.K + 63) / 64, n0 = a.splits0, n1 = a.splits - n0;
     const int run = n0 ? std::max((a.kb_switch + n0 - 1) / n0, (units - a.kb_switch + n1 - 1) / n1) : (units + n1 - 1) / n1;
-    if ((int64_t)((a.N + TILE - 1) / TILE) * a.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= ahead(F8) * WARPS) return a.M <= 8 ? launch<F8, 1, true>(ctx, a) : launch<F8, 2, true>(ctx, a);
+    if ((int64_t)((a.N + TILE - 1) / TILE) * a.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= ahead(false) * WARPS) return a.M <= 8 ? launch<KIND, 1, true>(ctx, a) : launch<KIND, 2, true>(ctx, a);
   }
-  return a.M <= 8 ? launch<F8, 1, false>(ctx, a) : launch<F8, 2, false>(ctx, a);
+  return a.M <= 8 ? launch<KIND, 1, false>(ctx, a) : launch<KIND, 2, false>(ctx, a);
 }
 }  // namespace
 
@@ -246,11 +289,21 @@ int sb_gemm_rows_splits(strictb200_ctx* ctx, int64_t N, int64_t K, bool f8) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(s, 8));                       // eight results are what the consumers take
 }
 int k_gemm_rows_bf16(strictb200_ctx* ctx, const GemmBf16Args& b) {
-  return launch<false>(ctx, RowsArgs{b.x, b.w, b.ldx, b.ldw, (int)b.M, (int)b.N, (int)b.K, b.splits, nullptr, nullptr, (int)(b.k_switch / 64), b.k_switch ? b.splits0 : 0,
+  return launch<ROWS_BF16>(ctx, RowsArgs{b.x, b.w, b.ldx, b.ldw, (int)b.M, (int)b.N, (int)b.K, b.splits, ctx->opt.prefetch, nullptr, nullptr, (int)(b.k_switch / 64), b.k_switch ? b.splits0 : 0,
                                      b.e.n_switch, b.e.x_row_off, b.group_n, b.group_k, b.part, b.e.out_f32, b.e.out_bf16, b.e.ldo});
 }
 int k_gemm_rows_fp8(strictb200_ctx* ctx, const GemmArgs& g) {
   const bool part = g.raw || g.splits > 1;
-  return launch<true>(ctx, RowsArgs{g.xq, g.wq, g.ldx, g.ldw, (int)g.M, (int)g.N, (int)g.K, g.splits, g.sx, g.sw, 0, 0, 0, 0, 0, 0, part ? g.part : nullptr,
+  return launch<ROWS_F8>(ctx, RowsArgs{g.xq, g.wq, g.ldx, g.ldw, (int)g.M, (int)g.N, (int)g.K, g.splits, ctx->opt.prefetch, g.sx, g.sw, 0, 0, 0, 0, 0, 0, part ? g.part : nullptr,
                                     g.out_f32 ? (float*)g.out : nullptr, g.out_f32 ? nullptr : (bf16*)g.out, g.N});
+}
+// W = [gate | up] [N, K]: out_bf16 [M, N / 2] = silu(gate) * up, and ones[M] = 1, the rows' scales for the next product's consumer.
+int k_gemm_rows_glu(strictb200_ctx* ctx, const GemmArgs& g, float* ones) {
+  const RowsArgs a{g.xq, g.wq, g.ldx, g.ldw, (int)g.M, (int)g.N, (int)g.K, 1, ctx->opt.prefetch, g.sx, g.sw, 0, 0, 0, 0, 0, 0, nullptr, nullptr, (bf16*)g.out, g.N / 2, ones};
+  return g.M <= 8 ? launch<ROWS_F8, 1, false, true>(ctx, a) : launch<ROWS_F8, 2, false, true>(ctx, a);
+}
+// part [splits][M, N] = sums of X . W^T, X [M, K] bf16 (g.xq, row stride g.ldx elements) and E4M3 weights.
+int k_gemm_rows_fp8_bf16(strictb200_ctx* ctx, const GemmArgs& g) {
+  return launch<ROWS_F8_BF16>(ctx, RowsArgs{g.xq, g.wq, g.ldx, g.ldw, (int)g.M, (int)g.N, (int)g.K, g.splits, ctx->opt.prefetch, nullptr, nullptr, 0, 0, 0, 0, 0, 0, g.part,
+                                            nullptr, nullptr, g.N});
 }
