@@ -4,6 +4,8 @@ import pytest
 
 from strict_b200 import native as N
 from strict_b200.kernel import DeviceVariable as DV
+from conftest import TOL_FP8, logits_close
+from test_gpu_models import TINY_QWEN, _run_pair
 
 pytestmark = pytest.mark.gpu
 L = N.lib
@@ -52,3 +54,24 @@ def test_gemm_fp8_few_rows(ctx, oracle, rng, M, N_, K):
     assert (np.abs(got - want) <= (K / 16 + 18) * 2.0 ** -23 * size).all()
     for v in (dq, ds, dw, dsw, dy):
         v.free()
+
+
+# one and two groups of 8 sequences and one beyond them; feed-forwards that end inside a block of 16 channel pairs' run of columns, rows wider than
+# the 1024 columns a block holds; with the weights' loads behind the dependency wait
+@pytest.mark.parametrize("B,over,prefetch", [(1, {}, 1), (8, dict(d_ff=192), 1), (9, dict(d_ff=320), 1), (16, dict(d_model=1152, d_ff=1216), 1), (17, dict(d_ff=192), 1),
+                                             (3, dict(d_ff=320), 0)])
+def test_decode_of_few_rows_vs_oracle(ctx, oracle, B, over, prefetch):
+    cfg = dict(TINY_QWEN, n_layers=2, vocab=512, **over)
+    with ctx.option("prefetch", prefetch):
+        m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 5, B, 12, [12 - i % 5 for i in range(B)], 4, random_gains=True)
+        for _ in range(3):
+            ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+            assert ok, (mx, rel)
+            ids = oracle.argmax(want)
+            _, logits = kv.decode_step(ids, want_logits=True)
+            want = st.decode(ids)
+        ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+        assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
