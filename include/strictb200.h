@@ -10,6 +10,10 @@
  * Threading: a context is bound to one device and one stream; calls on one context must be
  * serialised by the caller; different contexts may be driven from different threads.
  * Pointers named d_* are device pointers of that context's device, h_* are host pointers.
+ * Stream order: calls take effect in the order in which they are made on the context's stream. One exception: the weights
+ * (and the biases and scales of channels) of a call that is one product, strictb200_gemm_fp8, _gemm_int8, _gemm_bf16 or
+ * _gemm_f32, may be read before the kernels in front of it have ended. Where one of those kernels writes them, put a copy, a
+ * memset or strictb200_synchronize in between. strictb200_gemm_fp8w and _gemm_int8w read them in order.
  */
 #ifndef STRICTB200_H
 #define STRICTB200_H

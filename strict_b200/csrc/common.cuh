@@ -683,6 +683,9 @@ __device__ __forceinline__ void sb_bf16_store16(const Bf16Epilogue& e, int M, in
 // pdl_wait() blocks until the predecessor has completed and its writes are visible. Every such
 // kernel calls pdl_wait() before it reads or writes anything another kernel touches (so the
 // ordering stays transitive along the stream); only reads of constants (weights) may precede it.
+// A kernel that an entry point puts in front of a product of the caller's weights (the splits of activation rows) triggers after its
+// own wait: the product reads weights before its wait, and so it starts only when all that came before the entry, which may
+// have written them, is complete.
 // Without the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -55,8 +55,8 @@ __device__ __forceinline__ void zero_pad_rows(int8_t* hi, int8_t* lo, int64_t ro
 // One block per token row.
 __global__ void __launch_bounds__(QT) quantize_rows_int8_kernel(const bf16* x, int64_t M, int64_t K, int8_t* q, float* scale) {
   __shared__ float red[QT / 32];
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();  // not before the wait: see pdl_wait
   const int64_t row = blockIdx.x;
   int8_t* hi = q + ((row >> 3) * 16 + (row & 7)) * K;
   int8_t* lo = hi + 8 * K;
@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(QT) quantize_rows_int8_kernel(const bf16* x, i
 template <int IT>
 __global__ void __launch_bounds__(QT) quantize_rows_int8_wide_kernel(const bf16* x, int M, int K, int8_t* q, float* scale) {
   __shared__ float red[QT / 32];
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();  // not before the wait: see pdl_wait
   const int row = blockIdx.x;
   int8_t* hi = q + ((int64_t)(row >> 3) * 16 + (row & 7)) * K;
   int8_t* lo = hi + (int64_t)8 * K;

@@ -48,8 +48,8 @@ __device__ __forceinline__ void store8_e4m3(uint8_t* p, const float* v, float in
 template <int IT>
 __global__ void __launch_bounds__(ROW_THREADS) quantize_rows_kernel(const bf16* x, int64_t K, int64_t ldx, uint8_t* __restrict__ q, float* __restrict__ scale) {
   __shared__ float red[32];
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();  // not before the wait: see pdl_wait
   const int64_t row = blockIdx.x;
   const bf16* xr = x + row * ldx;
   uint4 w[IT];

@@ -75,3 +75,21 @@ def test_decode_of_few_rows_vs_oracle(ctx, oracle, B, over, prefetch):
     for o in (kv, m):
         o.dispose()
     st.close(), om.close()
+
+
+# weights that the call in front has just written, again and again in the same place, through the row split and the product's early loads
+@pytest.mark.parametrize("M,N_,K", [(1, 4096, 1024), (16, 1024, 4096), (100, 4096, 2048)])
+def test_weights_written_just_before(ctx, oracle, rng, M, N_, K):
+    x = oracle.round_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    sources = [(rng.standard_normal((N_, K)) * 0.05).astype(np.float32) for _ in range(2)]
+    dx, dw, ds = DV.of(ctx, oracle.f32_to_bf16(x)), DV(ctx, N_ * K, np.int8), DV(ctx, N_)
+    df, dy = [DV.of(ctx, w) for w in sources], [DV(ctx, M * N_, np.uint16) for _ in range(8)]
+    for i, y in enumerate(dy):
+        N.check(L().strictb200_quantize_weights_int8(ctx.h, df[i % 2].p, N_, K, dw.p, ds.p))
+        N.check(L().strictb200_gemm_int8w(ctx.h, M, N_, K, dx.p, dw.p, ds.p, y.p))
+    for j, w in enumerate(sources):
+        want = oracle.gemm_int8w(x, *oracle.quantize_weights_int8(w))
+        for y in dy[j::2]:
+            assert np.array_equal(y.to_host().reshape(M, N_), want)
+    for v in (dx, dw, ds, *df, *dy):
+        v.free()
