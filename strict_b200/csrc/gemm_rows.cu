@@ -8,7 +8,8 @@
 // of two products (the columns of a fragment may come in any order as long as W and X agree), so no operand passes shared memory.
 // The legacy tensor path is enough: one product of 32 channels x 16 columns per 1 KB of weights.
 // Where such blocks would not all be resident (two per SM hold 19 MB in registers) a block takes a second tile of 32 channels, whose weights
-// wait in shared memory, each thread's own where it put them: 38 MB are on their way before the wait (bf16 only).
+// wait in shared memory, each thread's own where it put them: 38 MB are there or on their way before the wait (bf16 only). They come by plain
+// loads and stores, so that the form has no instruction that the form of one tile does not have.
 // (The two halves of W = [gate | up] of a SwiGLU may share a block, 16 channels of each, which then writes bf16 silu(gate) * up.)
 // E4M3: a load is 16 columns. Weights become fp16 pairs, and so does the sum of the two E4M3 terms of X, hi + lo / 16 (both without
 // rounding: the sum has at most 9 significant bits down to units of 2^-13), so one product serves both terms. Rows of X that come as
@@ -130,19 +131,22 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
       for (int r = 0; r < 4; r++) unpack(raw[i][r], w[i][r]);
   };
   if (!a.prefetch) pdl_wait();
-  load_w(s0);  // weights are constants, and E4M3 ones are converted before the wait too (the conversions took longer than all that follows)
-  if constexpr (TWO) {
+  if constexpr (TWO) {  // the second tile first: its registers are free again when the first one's loads begin
+    uint4 raw[AHEAD][4];
 #pragma unroll
     for (int i = 0; i < AHEAD; i++)
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int k = (s0 + i) * STEP;
         const bool in = s0 + i < s1 && k + COLS * t < a.K && n0 + TILE + g + 8 * r < a.N;
-        const T* from = in ? wr + (int64_t)(TILE + 8 * r) * a.ldw + k : (const T*)a.w;
-        const uint32_t to = (uint32_t)__cvta_generic_to_shared(second + (i * 4 + r) * 32 * WARPS + threadIdx.x);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(in ? 16 : 0) : "memory");
+        raw[i][r] = in ? __ldcs((const uint4*)(wr + (int64_t)(TILE + 8 * r) * a.ldw + k)) : zero;
       }
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) second[(i * 4 + r) * 32 * WARPS + threadIdx.x] = raw[i][r];
   }
+  load_w(s0);  // weights are constants, and E4M3 ones are converted before the wait too (the conversions took longer than all that follows)
   pdl_wait();
   SB_TRACE_WAITED();
   float acc[2 * TILES][NT][4];
@@ -196,7 +200,6 @@ __global__ void __launch_bounds__(32 * WARPS, 2) gemm_rows_kernel(RowsArgs a) {
       }
     multiply(0);
     if constexpr (TWO) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
       for (int i = 0; i < AHEAD; i++)
 #pragma unroll
@@ -255,7 +258,9 @@ int launch(strictb200_ctx* ctx, const RowsArgs& a) {
     // longest run of columns a block gets, in units of 64
     const int units = (a.K + 63) / 64, n0 = a.splits0, n1 = a.splits - n0;
     const int run = n0 ? std::max((a.kb_switch + n0 - 1) / n0, (units - a.kb_switch + n1 - 1) / n1) : (units + n1 - 1) / n1;
-    if ((int64_t)((a.N + TILE - 1) / TILE) * a.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= ahead(false) * WARPS) return a.M <= 8 ? launch<KIND, 1, true>(ctx, a) : launch<KIND, 2, true>(ctx, a);
+    // Two tiles per block against one, us, 8 / 16 rows: N 9600 K 1024 4.7 / 7.4 against 5.9 / 7.5, N 14336 5.8 / 9.6 against 6.7 / 8.1, N 16384 6.4 /
+    // 10.5 against 7.2 / 8.9: with two groups of rows the second tile's products come on top of a longer chain.
+    if (a.M <= 8 && (int64_t)((a.N + TILE - 1) / TILE) * a.splits > 2 * (int64_t)ctx->sm_count && 2 * run <= ahead(false) * WARPS) return launch<KIND, 1, true>(ctx, a);
   }
   return a.M <= 8 ? launch<KIND, 1, false>(ctx, a) : launch<KIND, 2, false>(ctx, a);
 }
