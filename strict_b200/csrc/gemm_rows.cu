@@ -275,15 +275,26 @@ SB_TRACE_TU(gemm_rows)
 // and error against 64 bits (K 1024 / 5120): 9.8e-7 / 5.6e-6 there (tcgen05 cuts off after every instruction), 1.3e-7 / 6.0e-7 here.
 // A decode step of 8 sequences (28 layers of latent attention, 1024 wide): 926 -> 763 us.
 // Beyond 32 MB of weights the rows of X, which every block reads, and the later rounds of blocks cost more than the K splits of the large
-// tiles; a finished product has no K splits there, and with few tiles it stays here (4096 x 14336: 66.8 -> 26.7 us with 8 rows, 38.3 with 16;
-// 14336 x 4096: 23.2 -> 21.1 with 8, but 28.2 with 16; 28672 x 4096 36.2 -> 37.7).
+// tiles; a finished product has no K splits there, and with few tiles it stays here (us, 8 / 16 rows here against the large tiles: 4096 x
+// 14336 26.9 / 37.4 against 66.5; 1024 x 28672 40.9 / 55.7 against 130; 8192 x 8192 21.8 / 27.5 against 39.3; 8192 x 28672 71.5 / 94.0 against 131).
+// Many channels of short rows run in rounds of blocks that each wait for a round trip, where the large tiles' ring goes on: up to one
+// round of blocks (one_round), two with two tiles per block and at most 8 rows. us, 8 / 16 rows against the large tiles:
+//   N 16384 K 256   4.1 / 5.9 against 4.6    N 18944 K 3072  18.9 against 20.1       N 9472 K 1024  4.9 / 5.4 against 7.6
+//   N 32768 K 256   7.7 / 11.2 against 5.1   N 32768 K 2048  23.8 against 20.6       N 9600 K 256 5.1 (16), K 768 6.4 against 4.4, 6.5
 // E4M3 weights, whose large tiles are half as long a stream and whose conversion is work here: 1 / 16 rows, us, the row split in front included,
 //   N 4096 K 1024  8.1 / 8.0 -> 5.9 / 5.9     N 1024 K 3072  8.1 / 8.4 -> 7.9 / 7.9     N 1024 K 14336  12.4 / 12.8 -> 10.8 / 12.6
 //   N 6144 K 1024  8.1 / 8.0 -> 5.8 / 5.8     N 4096 K 4096  9.6 / 10.6, 9.9 / 12.6 here; N 6144 K 4096  10.4 / 11.0, 13.1 / 16.9 here
+// and without it, 8 / 16 rows against the large tiles:
+//   N 16384 K 512  5.4 against 6.9    N 9600 K 256   4.4 / 5.3 against 4.7    N 12288 K 640  5.1 / 7.3 against 6.7
+//   N 16384 K 256  5.0 against 4.6    N 32768 K 256  9.6 / 12.0 against 4.7   N 6144 K 1280 (two splits)  6.6 / 8.6 against 6.7
 // A decode step of Qwen3-0.6B: 774 -> 711 us (batch 1).
 bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished) {
   if (M > 16 || K % (f8 ? 16 : 8)) return false;
+  constexpr int64_t one_round = 2 * 148 * TILE;  // channels whose blocks are resident at once
   const int64_t weights = N * K;
+  const bool short_rounds = M <= 8 ? N <= one_round || (N <= 2 * one_round && (!f8 || K >= 512))
+                                   : f8 ? N * std::min<int64_t>((K + 1023) / 1024, 8) <= one_round : N <= one_round || (N <= 2 * one_round && K >= 768);
+  if (!short_rounds) return false;
   if (f8) return weights <= (8 << 20) || (N <= 1024 && weights <= (16 << 20));
   return weights <= (16 << 20) || (finished && (N <= 8192 || (M <= 8 && weights <= (64 << 20))));
 }

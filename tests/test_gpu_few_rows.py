@@ -12,9 +12,9 @@ L = N.lib
 
 
 # one and two groups of 8 rows; channels around a block's 32 and 64; columns around a load's 32, a unit of 64, the 1024 a block holds ahead, and
-# more of them; grids beyond two blocks per SM (two tiles per block); the largest matrix of the kernel and one beyond
+# more of them; grids beyond two blocks per SM (two tiles per block, and one with more than 8 rows); the most channels of the kernel and one beyond
 @pytest.mark.parametrize("M,N_,K", [(1, 1, 8), (8, 31, 24), (9, 33, 40), (16, 64, 1024), (3, 100, 1032), (5, 40, 5000), (8, 9600, 136), (13, 9599, 1024),
-                                    (8, 16384, 1024), (2, 16385, 1024), (17, 64, 64)])
+                                    (8, 16384, 1024), (2, 16385, 1024), (17, 64, 64), (8, 18944, 72), (7, 18945, 72), (9, 9473, 776), (16, 9473, 72)])
 def test_gemm_bf16_few_rows(ctx, oracle, rng, M, N_, K):
     x = oracle.round_bf16(rng.standard_normal((M, K)).astype(np.float32))
     w = oracle.round_bf16((rng.standard_normal((N_, K)) * 0.05).astype(np.float32))
@@ -33,7 +33,7 @@ def test_gemm_bf16_few_rows(ctx, oracle, rng, M, N_, K):
 
 
 # the same of E4M3 weights: loads of 64 columns, 1024 columns per block, sums of several blocks per output
-@pytest.mark.parametrize("M,N_,K", [(1, 16, 64), (8, 48, 192), (9, 32, 1088), (16, 1024, 2048), (5, 1600, 4160), (8, 15984, 512), (13, 7600, 1024),
+@pytest.mark.parametrize("M,N_,K", [(1, 16, 64), (8, 48, 192), (9, 32, 1088), (16, 1024, 2048), (5, 1600, 4160), (8, 15984, 512), (13, 7600, 1024), (16, 9472, 128), (9, 9488, 128),
                                     (3, 768, 14336), (4, 1024, 3072), (16, 2080, 4096)])
 def test_gemm_fp8_few_rows(ctx, oracle, rng, M, N_, K):
     import torch

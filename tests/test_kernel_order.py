@@ -1,4 +1,4 @@
-"""What the kernels' sources must say about programmatic dependent launch: a wrong order of trigger, wait and loads is a race that a
+"""What can be told without a GPU about how kernels are chosen and ordered. What the kernels' sources must say about programmatic dependent launch: a wrong order of trigger, wait and loads is a race that a
 run on a GPU hardly ever shows."""
 import glob
 import os
@@ -36,3 +36,18 @@ def test_row_splits_trigger_after_their_wait(name):
     have written them, is complete."""
     body = KERNELS[name][2]
     assert 0 <= body.index("pdl_wait()") < body.index("pdl_trigger()")
+
+
+# M, N, K, E4M3 weights, finished product -> the kernel of few rows takes it: both sides of the lines that its rule draws, all measured
+@pytest.mark.parametrize("M,N,K,f8,finished,takes", [
+    (16, 9472, 64, False, True, True), (9, 9473, 64, False, True, False), (9, 9473, 768, False, True, True), (16, 18945, 768, False, False, False),
+    (8, 18944, 64, False, True, True), (8, 18945, 64, False, True, False), (8, 32768, 256, False, True, False), (8, 18944, 3072, False, True, True),
+    (16, 8192, 28672, False, True, True), (8, 4096, 4104, False, False, False), (17, 64, 64, False, True, False),
+    (16, 9472, 512, True, False, True), (16, 9488, 512, True, False, False), (16, 6144, 1280, True, False, False), (8, 6144, 1280, True, False, True),
+    (8, 16384, 512, True, True, True), (8, 16384, 256, True, True, False), (8, 9472, 64, True, True, True), (1, 32768, 128, True, True, False)])
+def test_rule_of_the_few_row_kernel(M, N, K, f8, finished, takes):
+    import ctypes as C
+    from strict_b200 import native
+    rule = native.lib()._Z18sb_gemm_rows_takeslllbb
+    rule.restype, rule.argtypes = C.c_bool, [C.c_int64] * 3 + [C.c_bool] * 2
+    assert rule(M, N, K, f8, finished) == takes
