@@ -673,7 +673,7 @@ SB_TRACE_TU(attention)
 // full cache): a cache that holds 2100 of 2432 keys in chunks of 512 runs four full chunks and a
 // stub per sequence, chunks of 448 run five even ones (14 % less attention time, measured). The
 // attn_blocks_per_sm option restores the plain "that many blocks per SM" rule.
-static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0) {
+static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool short_chunks = true) {
   const int per_sm = ctx->opt.attn_blocks_per_sm;
   const int tiles = (maxlen + KT - 1) / KT;
   const int tiles_plan = len_plan > 0 && len_plan < maxlen ? (len_plan + KT - 1) / KT : tiles;
@@ -706,9 +706,11 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
   // At most 8 chunks per sequence: that is what the fast merge kernel takes. 16 chunks for the few
   // (sequence, head) pairs of TP=8 shortened the attention kernel but the general merge kernel they
   // need cost more than that (21.9 against 17.0 us per layer for the pair, measured on eight GPUs).
-  // Short caches get chunks of one or two tiles while the grid stays in one wave (8 sequences of 544 keys, 8 KV heads: chunks of 256 keys
-  // walked four tiles one after the other on some SMs and one on others, 8.7 us; chunks of 128, 5.7 us).
+  // Less than four tiles (256 keys) only while all blocks are resident at once (8 sequences of 544 keys, 8 KV heads: chunks of 256 keys
+  // walked four tiles one after the other on some SMs and one on others, 8.7 us; chunks of 128, 5.7 us). In several waves short chunks gain nothing and
+  // multiply the partial results (`short_chunks` false: never).
   for (int c = (tiles + 7) / 8; c <= tiles; c++) {
+    if (c < 4 && c < tiles && (!short_chunks || pairs * ((tiles_plan + c - 1) / c) > slots)) continue;
     // (counting a stub as a whole block is deliberate: weighting blocks by their length made the rule pick three long
     // chunks where five short ones measured 47 us against 66)
     const int64_t blocks = pairs * ((tiles_plan + c - 1) / c), waves = (blocks + slots - 1) / slots;
@@ -717,10 +719,8 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
   }
   return best * KT;
 }
-int sb_attn_decode_splits(strictb200_ctx* ctx, int B, int Hkv, int maxlen) {
-  int c = decode_chunk(ctx, B, Hkv, maxlen);
-  return (maxlen + c - 1) / c;
-}
+static int splits_of(int maxlen, int chunk) { return (maxlen + chunk - 1) / chunk; }
+int sb_attn_decode_splits(strictb200_ctx* ctx, int B, int Hkv, int maxlen) { return splits_of(maxlen, decode_chunk(ctx, B, Hkv, maxlen)); }
 int sb_attn_decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan) { return decode_chunk(ctx, B, Hkv, maxlen, len_plan); }
 size_t sb_attn_decode_scratch(int B, int Hq, int Dh, int nsplit) { return (size_t)B * Hq * nsplit * (Dh + 2) * sizeof(float); }
 
@@ -826,8 +826,11 @@ extern "C" int strictb200_attn_decode_noalloc(strictb200_ctx* ctx, const uint16_
   SB_REQUIRE(B >= 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && Hq / Hkv <= 16 && maxlen > 0, "bad shape");
   if (!B) return STRICTB200_OK;
   SB_REQUIRE(q && kc && vc && lens && out, "null pointer");
-  int nsplit = sb_attn_decode_splits(ctx, B, Hkv, maxlen);
-  size_t need = sb_attn_decode_scratch(B, Hq, Dh, nsplit) / sizeof(float);
+  auto floats = [&](int chunk) { return sb_attn_decode_scratch(B, Hq, Dh, splits_of(maxlen, chunk)) / sizeof(float); };
+  int chunk = decode_chunk(ctx, B, Hkv, maxlen);
+  if (floats(chunk) > NOALLOC_SCRATCH_FLOATS) chunk = decode_chunk(ctx, B, Hkv, maxlen, 0, false);  // fewer partial results
+  const int nsplit = splits_of(maxlen, chunk);
+  const size_t need = floats(chunk);
   if (need > NOALLOC_SCRATCH_FLOATS)
     return sb_fail(STRICTB200_ERR_INVALID_ARG, "attn_decode_noalloc: batch " + std::to_string(B) + " x " + std::to_string(Hq) + " heads x " +
                                                    std::to_string(nsplit) + " key chunks needs " + std::to_string(need * sizeof(float)) +
@@ -838,5 +841,5 @@ extern "C" int strictb200_attn_decode_noalloc(strictb200_ctx* ctx, const uint16_
   // Nothing in the scratch has to start at zero: each key chunk a sequence owns is written in full
   // by its block before the combine kernel reads it, and chunks beyond a sequence's length are never read.
   return k_attn_decode(ctx, (const bf16*)q, (const bf16*)kc, (const bf16*)vc, lens, 0, B, Hq, Hkv, Dh, maxlen, scale, nsplit, scratch,
-                       (bf16*)out, nullptr, nullptr, nullptr);
+                       (bf16*)out, nullptr, nullptr, nullptr, chunk);
 }

@@ -54,6 +54,13 @@ def test_noalloc_matches_allocating_entry_twice_in_a_row(ctx, oracle):
     assert np.array_equal(a, b)
 
 
+# many sequences with short caches: key chunks below 256 keys would take more partial results than the built-in scratch holds
+@pytest.mark.parametrize("B,Hq,Hkv,maxlen", [(38, 32, 8, 1344), (28, 64, 8, 640), (112, 32, 8, 576), (75, 32, 2, 960)])
+def test_noalloc_takes_many_short_caches(ctx, oracle, B, Hq, Hkv, maxlen):
+    a, b = _case(ctx, oracle, 3, B, Hq, Hkv, maxlen, [1 + (i * 131) % maxlen for i in range(B - 1)] + [maxlen])
+    assert np.array_equal(a, b)
+
+
 def test_noalloc_rejects_what_does_not_fit(ctx):
     # 4096 sequences x 32 heads x 130 floats of partial results per key chunk is far beyond 4 MiB;
     # the size check comes before any pointer is touched
