@@ -672,8 +672,8 @@ SB_TRACE_TU(attention)
 // most 8 chunks for a full cache. The waves are counted for sequences of `len_plan` keys (0: a
 // full cache): a cache that holds 2100 of 2432 keys in chunks of 512 runs four full chunks and a
 // stub per sequence, chunks of 448 run five even ones (14 % less attention time, measured). The
-// attn_blocks_per_sm option restores the plain "that many blocks per SM" rule.
-static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool short_chunks = true) {
+// attn_blocks_per_sm option restores the plain "that many blocks per SM" rule. `fused`: the kernel with the RoPE prologue will run.
+static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool fused = false, bool short_chunks = true) {
   const int per_sm = ctx->opt.attn_blocks_per_sm;
   const int tiles = (maxlen + KT - 1) / KT;
   const int tiles_plan = len_plan > 0 && len_plan < maxlen ? (len_plan + KT - 1) / KT : tiles;
@@ -698,7 +698,7 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
     resident_fused_of[ctx->device & 63] = r;
     return cudaSuccess;
   });
-  const int res0 = (ctx->opt.fuse_rope > 0 ? resident_fused_of : resident_of)[ctx->device & 63];
+  const int res0 = (fused ? resident_fused_of : resident_of)[ctx->device & 63];
   const int resident = res0 > 0 ? res0 : 1;
   const int64_t slots = (int64_t)ctx->sm_count * resident, pairs = (int64_t)B * Hkv;
   int best = tiles;
@@ -721,7 +721,7 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
 }
 static int splits_of(int maxlen, int chunk) { return (maxlen + chunk - 1) / chunk; }
 int sb_attn_decode_splits(strictb200_ctx* ctx, int B, int Hkv, int maxlen) { return splits_of(maxlen, decode_chunk(ctx, B, Hkv, maxlen)); }
-int sb_attn_decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan) { return decode_chunk(ctx, B, Hkv, maxlen, len_plan); }
+int sb_attn_decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan, bool fused) { return decode_chunk(ctx, B, Hkv, maxlen, len_plan, fused); }
 size_t sb_attn_decode_scratch(int B, int Hq, int Dh, int nsplit) { return (size_t)B * Hq * nsplit * (Dh + 2) * sizeof(float); }
 
 // The key chunks alone, for a merge of the caller's: rows of HD = 64 or 128 dims, len_add = 1 (the new token's row is in the cache).
@@ -828,7 +828,7 @@ extern "C" int strictb200_attn_decode_noalloc(strictb200_ctx* ctx, const uint16_
   SB_REQUIRE(q && kc && vc && lens && out, "null pointer");
   auto floats = [&](int chunk) { return sb_attn_decode_scratch(B, Hq, Dh, splits_of(maxlen, chunk)) / sizeof(float); };
   int chunk = decode_chunk(ctx, B, Hkv, maxlen);
-  if (floats(chunk) > NOALLOC_SCRATCH_FLOATS) chunk = decode_chunk(ctx, B, Hkv, maxlen, 0, false);  // fewer partial results
+  if (floats(chunk) > NOALLOC_SCRATCH_FLOATS) chunk = decode_chunk(ctx, B, Hkv, maxlen, 0, false, false);  // fewer partial results
   const int nsplit = splits_of(maxlen, chunk);
   const size_t need = floats(chunk);
   if (need > NOALLOC_SCRATCH_FLOATS)

@@ -571,7 +571,7 @@ bool sb_retention_decode_fits(const HeadShape& s);
 int k_retention_decode(strictb200_ctx*, const RetentionArgs& a, int64_t B);
 size_t sb_attn_decode_scratch(int B, int Hq, int D, int nsplit);
 int sb_attn_decode_splits(strictb200_ctx*, int B, int Hkv, int maxlen);
-int sb_attn_decode_chunk(strictb200_ctx*, int B, int Hkv, int maxlen, int len_plan);  // keys per block for sequences of about len_plan keys (at most 8 chunks cover maxlen)
+int sb_attn_decode_chunk(strictb200_ctx*, int B, int Hkv, int maxlen, int len_plan, bool fused = false);  // keys per block for sequences of about len_plan keys (at most 8 chunks cover maxlen)
 // rope != null: the queries and the new token's key/value rows are computed inside the attention kernel from the qkv
 // projection's partial results (what k_rope_qknorm_kvappend would do in a kernel of its own); q is then unused
 int k_attn_decode(strictb200_ctx*, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, int len_add, int B, int Hq,

@@ -45,6 +45,14 @@ int plan_gate_up_splits(strictb200_model* m, int64_t M) {
   return s > 4 ? 4 : s;
 }
 
+// QK-norm, RoPE and the cache append inside the attention kernel? s1: K splits of the qkv projection.
+// By itself where a step is a chain of short kernels and the projection is one result that every key chunk's block may read: Qwen3-0.6B
+// 713 -> 698 us (batch 1), 812 -> 789 (batch 8); Qwen3-8B at batch 32 (five partial results) 3986 -> 3964, within what two runs differ.
+bool fuses_rope(strictb200_model* m, int64_t B, int s1) {
+  const int fuse = m->ctx->opt.fuse_rope;
+  return (fuse < 0 ? B <= 16 && s1 == 1 : fuse > 0) && s1 <= 8 && m->Hq_l / m->Hkv_l <= 16;
+}
+
 void carve_decode(strictb200_kv* kv, char* base, DecBuf* out, size_t* total) {
   strictb200_model* m = kv->m;
   const auto& c = m->c;
@@ -197,10 +205,7 @@ int qwen_decode_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
     r.q_out = b.qb; r.kcache = kv_k(kv, l); r.vcache = kv_v(kv, l);
     // QK-norm, RoPE and the cache append inside the attention kernel (one kernel less per layer), or as a kernel of their own.
     // The merge kernel overwrites b.sa (the o_proj operand's scales) only after every attention block has read it.
-    // By itself where a step is a chain of short kernels and the projection is one result that every key chunk's block may read: Qwen3-0.6B
-    // 713 -> 698 us (batch 1), 812 -> 789 (batch 8); Qwen3-8B at batch 32 (five partial results) 3986 -> 3964, within what two runs differ.
-    const int fuse = ctx->opt.fuse_rope;
-    const bool fuse_rope = (fuse < 0 ? B <= 16 && s1 == 1 : fuse > 0) && s1 <= 8 && m->Hq_l / m->Hkv_l <= 16;
+    const bool fuse_rope = fuses_rope(m, B, s1);
     if (!fuse_rope) PROF(STRICTB200_K_ROPE, k_rope_qknorm_kvappend(ctx, r, B));
     // split-KV attention over len+1 keys; the combine emits the quantised o_proj input
     PROF(STRICTB200_K_ATTN, k_attn_decode(ctx, b.qb, kv_k(kv, l), kv_v(kv, l), kv->d_lens, 1, (int)B, m->Hq_l, m->Hkv_l, (int)D, kv->maxlen,
@@ -340,7 +345,9 @@ int decode_enqueue(strictb200_model* m, strictb200_kv* kv) {
     int longest = 0;
     for (int b = 0; b < kv->B; b++) longest = std::max(longest, kv->h_lens[b] + 1);
     if (!kv->chunk || longest > kv->plan_until) {
-      const int chunk = sb_attn_decode_chunk(ctx, kv->B, m->Hkv_l, kv->maxlen, std::min(kv->maxlen, longest + 128));
+      const int64_t nqkv = ((int64_t)m->Hq_l + 2 * m->Hkv_l) * m->c.head_dim;
+      const bool fused = fuses_rope(m, kv->B, plan_splits(m, kv->B, nqkv, m->c.d_model));
+      const int chunk = sb_attn_decode_chunk(ctx, kv->B, m->Hkv_l, kv->maxlen, std::min(kv->maxlen, longest + 128), fused);
       if (chunk != kv->chunk) {
         kv->chunk = chunk;
         kv->nsplit = (kv->maxlen + chunk - 1) / chunk;
