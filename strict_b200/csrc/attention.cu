@@ -303,8 +303,8 @@ __device__ __forceinline__ int ld_volatile_i32(const int32_t* p) {
 // appends them to the cache and patches them into its own shared-memory tile (its tile load may
 // have read that row before the append). One kernel less per layer of the decode step.
 template <int HD, bool FUSED>
-__global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc, const bf16* __restrict__ vc,
-                                                          const int32_t* __restrict__ lens, int len_add, int B, int Hq, int Hkv, int maxlen,
+__global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const bf16* kc, const bf16* vc,
+                                                          const int32_t* lens, int len_add, int B, int Hq, int Hkv, int maxlen,
                                                           int chunk, int nsplit, float scale_log2, float* __restrict__ o_part,
                                                           float* __restrict__ ml_part, RopeFuseArgs rf, int prefetch) {
   static_assert(!FUSED || HD == D, "the RoPE prologue is for 128 dims");
@@ -527,8 +527,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* __restrict
 // consecutive dims of one head (two when Hq > 32) and keeps them in registers for the optional
 // two-term E4M3 split of the whole token row [Hq*128] (the o_proj input).
 constexpr int CB_THREADS = 512, CB_ITEMS = 2;
-__global__ void __launch_bounds__(CB_THREADS) attn_combine_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                                                                  const int32_t* __restrict__ lens, int len_add, int Hq, int maxlen, int chunk,
+__global__ void __launch_bounds__(CB_THREADS) attn_combine_kernel(const float* o_part, const float* ml_part,
+                                                                  const int32_t* lens, int len_add, int Hq, int maxlen, int chunk,
                                                                   int nsplit, bf16* __restrict__ out, uint8_t* __restrict__ q_out,
                                                                   float* __restrict__ qscale) {
   __shared__ float red[32];
@@ -584,8 +584,8 @@ __global__ void __launch_bounds__(CB_THREADS) attn_combine_kernel(const float* _
 // in flight. Every partial is loaded in one batch together with the sequence length (slots of
 // chunks beyond the length hold stale data and are masked out of the arithmetic, which is that
 // of the kernel above).
-__global__ void __launch_bounds__(1024) attn_combine_decode_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                                                                   const int32_t* __restrict__ lens, int len_add, int Hq, int maxlen, int chunk,
+__global__ void __launch_bounds__(1024) attn_combine_decode_kernel(const float* o_part, const float* ml_part,
+                                                                   const int32_t* lens, int len_add, int Hq, int maxlen, int chunk,
                                                                    int nsplit, bf16* __restrict__ out, uint8_t* __restrict__ q_out,
                                                                    float* __restrict__ qscale, int* __restrict__ status) {
   __shared__ float red[32];

@@ -1,11 +1,11 @@
 // fp32 attention of the GPT-2 path: prompts in tiles, decode rows with the keys spread over half-warps, and a kernel for any head width.
-// Inputs that another kernel of the chain writes are not declared __restrict__ in the kernels below: loads of invariant data may be
+// Inputs that another kernel of the chain writes are not declared const __restrict__ in these kernels: loads of invariant data may be
 // moved in front of the dependency wait.
 #include "common.cuh"
 
 namespace {
-__global__ void kv_append_f32_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
-                                     const int32_t* __restrict__ seq, const int32_t* __restrict__ pos, const int32_t* __restrict__ lens, int H,
+__global__ void kv_append_f32_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc,
+                                     const int32_t* seq, const int32_t* pos, const int32_t* lens, int H,
                                      int Dh, int maxlen) {
   pdl_trigger();
   pdl_wait();
@@ -22,9 +22,9 @@ __global__ void kv_append_f32_kernel(const float* __restrict__ qkv, float* __res
   }
 }
 // Any head width. grid (H, T), 256 threads; scores of one (token, head) live in shared memory.
-__global__ void __launch_bounds__(256) attn_f32_kernel(const float* __restrict__ qkv, const float* __restrict__ kc, const float* __restrict__ vc,
-                                                       const int32_t* __restrict__ seq, const int32_t* __restrict__ pos,
-                                                       const int32_t* __restrict__ lens, int H, int Dh, int maxlen, float scale,
+__global__ void __launch_bounds__(256) attn_f32_kernel(const float* qkv, const float* kc, const float* vc,
+                                                       const int32_t* seq, const int32_t* pos,
+                                                       const int32_t* lens, int H, int Dh, int maxlen, float scale,
                                                        float* __restrict__ out, float* kc_new, float* vc_new) {
   // kc_new/vc_new (decode: every row is its own sequence) make this block also append its head's
   // new key and value; it then takes position p from the projection output, not from the cache.
@@ -116,8 +116,8 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(const float* __restrict__
 constexpr int PT = 64, PD = 64, PS = PD + 4;  // queries and keys per tile, head dims, row stride in shared memory
 constexpr int PROMPT_SMEM = 4 * PT * PS * 4;
 __global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* qkv, const float* kc, const float* vc,
-                                                              const int32_t* __restrict__ qstart, const int32_t* __restrict__ past,
-                                                              const int32_t* __restrict__ after, int b0, int H, int maxlen, float scale,
+                                                              const int32_t* qstart, const int32_t* past,
+                                                              const int32_t* after, int b0, int H, int maxlen, float scale,
                                                               float* out) {
   extern __shared__ __align__(16) float ps[];
   float *qs = ps, *ks = ps + PT * PS, *vs = ks + PT * PS, *pr = vs + PT * PS;

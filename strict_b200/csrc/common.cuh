@@ -682,7 +682,8 @@ __device__ __forceinline__ void sb_bf16_store16(const Bf16Epilogue& e, int M, in
 // predecessor in the stream is still running: pdl_trigger() lets the successor start launching,
 // pdl_wait() blocks until the predecessor has completed and its writes are visible. Every such
 // kernel calls pdl_wait() before it reads or writes anything another kernel touches (so the
-// ordering stays transitive along the stream); only reads of constants (weights) may precede it.
+// ordering stays transitive along the stream); only reads of constants (weights) may precede it, and only constants are
+// declared const __restrict__: the compiler may move loads of invariant data in front of the wait.
 // A kernel that an entry point puts in front of a product of the caller's weights (the splits of activation rows) triggers after its
 // own wait: the product reads weights before its wait, and so it starts only when all that came before the entry, which may
 // have written them, is complete.

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(QT) quantize_weights_int8_kernel(const float* 
 }
 
 // Sum of the K splits' integer partials, [split][hi, lo][M, N], joined and scaled.
-__global__ void finish_int8_kernel(const int32_t* __restrict__ part, int splits, int64_t M, int64_t N, const float* __restrict__ sx,
+__global__ void finish_int8_kernel(const int32_t* part, int splits, int64_t M, int64_t N, const float* sx,
                                    const float* __restrict__ sw, bf16* __restrict__ y) {
   pdl_trigger();
   pdl_wait();

@@ -163,9 +163,9 @@ __global__ void __launch_bounds__(256) act_rows_kernel(ProjRows p, ActArgs a, in
 
 // grid (H, T), 256 threads; 256 keys per step, fp32 arithmetic throughout.
 template <typename T>
-__global__ void __launch_bounds__(256) head_attn_any_kernel(HeadShape s, const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc,
-                                                            const float* __restrict__ gate, const int32_t* __restrict__ seq, const int32_t* __restrict__ pos,
-                                                            const int32_t* __restrict__ lens, int maxlen, T* __restrict__ out, int64_t ldo) {
+__global__ void __launch_bounds__(256) head_attn_any_kernel(HeadShape s, const T* q, const T* kc, const T* vc,
+                                                            const float* gate, const int32_t* seq, const int32_t* pos,
+                                                            const int32_t* lens, int maxlen, T* __restrict__ out, int64_t ldo) {
   extern __shared__ float sm[];
   __shared__ float red[32];
   pdl_trigger();
@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(256) head_attn_any_kernel(HeadShape s, const T
 
 // grid (B, heads in groups of 8), 256 threads: a warp merges the key chunks of one head (at most 8), a lane owns HD / 32 dims.
 template <int HD>
-__global__ void __launch_bounds__(256) head_combine_kernel(HeadShape s, const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                                                           const float* __restrict__ gate, const int32_t* __restrict__ lens, int maxlen, int chunk, int nsplit,
+__global__ void __launch_bounds__(256) head_combine_kernel(HeadShape s, const float* o_part, const float* ml_part,
+                                                           const float* gate, const int32_t* lens, int maxlen, int chunk, int nsplit,
                                                            bf16* __restrict__ out, int64_t ldo) {
   constexpr int PER = HD / 32;
   SB_TRACE_BEGIN();

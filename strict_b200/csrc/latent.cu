@@ -901,9 +901,9 @@ __global__ void __launch_bounds__(256) latent_value_kernel(ValueDev a) {
 // ------------------------------------------------------------------ any width, bf16 or fp32
 // grid (H, T), 256 threads; 256 keys per step, fp32 arithmetic throughout.
 template <typename T>
-__global__ void __launch_bounds__(256) latent_attn_any_kernel(LatentShape s, const T* __restrict__ q, const T* __restrict__ cache, const T* __restrict__ wkv,
-                                                              const int32_t* __restrict__ seq, const int32_t* __restrict__ pos,
-                                                              const int32_t* __restrict__ lens, int maxlen, T* __restrict__ out, int64_t ldo) {
+__global__ void __launch_bounds__(256) latent_attn_any_kernel(LatentShape s, const T* q, const T* cache, const T* __restrict__ wkv,
+                                                              const int32_t* seq, const int32_t* pos,
+                                                              const int32_t* lens, int maxlen, T* __restrict__ out, int64_t ldo) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[32];
   pdl_trigger();

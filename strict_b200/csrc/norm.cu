@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(1024) rownorm_decode_kernel(RowNormDev a, int6
 }
 
 
-__global__ void __launch_bounds__(ROW_THREADS) layernorm_kernel(const float* __restrict__ x, const float* __restrict__ g,
+__global__ void __launch_bounds__(ROW_THREADS) layernorm_kernel(const float* x, const float* __restrict__ g,
                                                                 const float* __restrict__ b, float eps, int64_t d, float* __restrict__ y) {
   pdl_trigger();
   __shared__ float red[32];
@@ -566,7 +566,7 @@ __global__ void add_f32_kernel(float* __restrict__ x, const float* __restrict__ 
 // two-term E4M3 split of h per row. 512 threads; a thread owns up to 4 groups of 8 columns and
 // keeps h in registers between the absmax pass and the split (rows wider than 16384 recompute).
 constexpr int SW_THREADS = 512, SW_ITEMS = 4;
-__global__ void __launch_bounds__(SW_THREADS) swiglu_kernel(const bf16* __restrict__ gu, const float* __restrict__ gu32, int64_t I,
+__global__ void __launch_bounds__(SW_THREADS) swiglu_kernel(const bf16* gu, const float* gu32, int64_t I,
                                                             bf16* __restrict__ y, uint8_t* __restrict__ q, float* __restrict__ qscale) {
   __shared__ float red[32];
   pdl_trigger();
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(SW_THREADS) swiglu_kernel(const bf16* __restri
 // The decode-step shape of the above: a row of I columns is shared by a cluster of gridDim.y
 // blocks, one 8-column group per thread (I == gridDim.y * blockDim.x * 8), fp32 input, split
 // output. The blocks of a row push their absolute maxima to each other.
-__global__ void __launch_bounds__(512) swiglu_decode_kernel(const float* __restrict__ gu32, int64_t I, bf16* __restrict__ y,
+__global__ void __launch_bounds__(512) swiglu_decode_kernel(const float* gu32, int64_t I, bf16* __restrict__ y,
                                                             uint8_t* __restrict__ q, float* __restrict__ qscale, int* __restrict__ status) {
   __shared__ float red[32];
   __shared__ __align__(8) ClusterExchange xch;
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(512) swiglu_decode_kernel(const float* __restr
 // The same for a gate/up projection that arrives as at most 4 raw split-K partials
 // [splits][M][2I] with the scales still to apply (the narrow shards of tensor parallelism, whose
 // GEMM needs K splits to cover the GPU): 4 columns per thread, so 2 x splits loads in flight.
-__global__ void __launch_bounds__(512) swiglu_decode_part_kernel(const float* __restrict__ part, int splits, const float* __restrict__ sx,
+__global__ void __launch_bounds__(512) swiglu_decode_part_kernel(const float* part, int splits, const float* sx,
                                                                  const float* __restrict__ sw, int64_t M, int64_t I, uint8_t* __restrict__ q,
                                                                  float* __restrict__ qscale, int* __restrict__ status) {
   __shared__ float red[32];
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(512) swiglu_decode_part_kernel(const float* __
   SB_TRACE_END(SB_K_SWIGLU, 0);
 }
 
-__global__ void gelu_tanh_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ y) {
+__global__ void gelu_tanh_kernel(const float* x, int64_t n, float* __restrict__ y) {
   pdl_trigger();
   pdl_wait();
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -843,7 +843,7 @@ int k_gelu_tanh(strictb200_ctx* ctx, const float* x, int64_t n, float* y) {
 
 // out[m,n] = (sum_s part[s][m,n]) * sx[m] * sw[n], fp32 (the input of a cross-rank all-reduce) or bf16
 namespace {
-__global__ void reduce_scale_kernel(const float* __restrict__ part, int splits, const float* __restrict__ sx, const float* __restrict__ sw,
+__global__ void reduce_scale_kernel(const float* part, int splits, const float* sx, const float* __restrict__ sw,
                                     int64_t M, int64_t N, float* __restrict__ out, bf16* __restrict__ out_bf16) {
   pdl_trigger();
   pdl_wait();

@@ -13,7 +13,7 @@ __global__ void embedding_bf16_kernel(const bf16* __restrict__ table, const int3
   for (int64_t i = threadIdx.x; i < d / 8; i += blockDim.x) dst[i] = src[i];
 }
 
-__global__ void embedding_bf16_f32_kernel(const bf16* __restrict__ table, const int32_t* __restrict__ ids, int64_t d, int64_t vocab,
+__global__ void embedding_bf16_f32_kernel(const bf16* __restrict__ table, const int32_t* ids, int64_t d, int64_t vocab,
                                           float* __restrict__ out) {
   pdl_trigger();
   pdl_wait();
@@ -29,8 +29,8 @@ __global__ void embedding_bf16_f32_kernel(const bf16* __restrict__ table, const 
   }
 }
 
-__global__ void embedding_f32_kernel(const float* __restrict__ wte, const float* __restrict__ wpe, const int32_t* __restrict__ ids,
-                                     const int32_t* __restrict__ pos, const int32_t* __restrict__ lens, int64_t d, int64_t vocab, int max_pos,
+__global__ void embedding_f32_kernel(const float* __restrict__ wte, const float* __restrict__ wpe, const int32_t* ids,
+                                     const int32_t* pos, const int32_t* lens, int64_t d, int64_t vocab, int max_pos,
                                      float* __restrict__ out) {
   pdl_trigger();
   pdl_wait();
@@ -133,7 +133,7 @@ int k_embedding_f32(strictb200_ctx* ctx, const float* wte, const float* wpe, con
 // per row merges the chunk winners (chunks ascend, ties keep the lower index).
 namespace {
 constexpr int AM_CHUNK = 4096;
-__global__ void __launch_bounds__(256) argmax_chunk_kernel(const float* __restrict__ x, int64_t N, int64_t ldx, float* __restrict__ cval,
+__global__ void __launch_bounds__(256) argmax_chunk_kernel(const float* x, int64_t N, int64_t ldx, float* __restrict__ cval,
                                                            int32_t* __restrict__ cidx, int nchunks) {
   __shared__ float sv[8];
   __shared__ int si[8];
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256) argmax_chunk_kernel(const float* __restri
     cidx[row * nchunks + blockIdx.x] = bi;
   }
 }
-__global__ void argmax_merge_kernel(const float* __restrict__ cval, const int32_t* __restrict__ cidx, int nchunks, int32_t* __restrict__ out,
+__global__ void argmax_merge_kernel(const float* cval, const int32_t* cidx, int nchunks, int32_t* __restrict__ out,
                                     float* __restrict__ val_out) {
   pdl_trigger();
   pdl_wait();

@@ -38,6 +38,18 @@ def test_row_splits_trigger_after_their_wait(name):
     assert 0 <= body.index("pdl_wait()") < body.index("pdl_trigger()")
 
 
+# Inputs that no kernel of a step's chain writes. Loads through a const __restrict__ pointer may be moved in front of the dependency wait.
+CONSTANTS = {"w", "sw", "bias", "col_scale", "gain", "g", "b", "ln_gain", "ln_bias", "table", "wte", "wpe", "wkv"}
+
+
+@pytest.mark.parametrize("name", [n for n in KERNELS if "pdl_wait()" in KERNELS[n][2]])
+def test_chain_inputs_are_not_declared_invariant(name):
+    declared = set(re.findall(r"const \w+\s*\*\s*__restrict__ (\w+)", KERNELS[name][1]))
+    assert declared <= CONSTANTS
+    loads = re.findall(r"__ldg\(\(const \w+\*\)\(?(\w+)", KERNELS[name][2])
+    assert set(loads) <= {"wrow"}
+
+
 # M, N, K, E4M3 weights, finished product -> the kernel of few rows takes it: both sides of the lines that its rule draws, all measured
 @pytest.mark.parametrize("M,N,K,f8,finished,takes", [
     (16, 9472, 64, False, True, True), (9, 9473, 64, False, True, False), (9, 9473, 768, False, True, True), (16, 18945, 768, False, False, False),
