@@ -167,6 +167,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
     if (lane == 0) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(CH >> 4) << 24);
       const uint32_t big = tmem, small = tmem + 2 * BT;
+      // The operand tiles cannot arrive before the feeders' dependency wait has returned: the same wait here keeps the bounded ones below for
+      // progress inside this kernel, however long its predecessor takes.
+      pdl_wait();
       for (int kb = 0; kb < nkb; kb++) {
         const int s = kb % NSTAGE;
         if (!mbar_wait(smem_u32(&bar_full[s]), (kb / NSTAGE) & 1)) { set_status(a.status, 2); abort_flag = 1; break; }

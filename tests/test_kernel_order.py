@@ -50,6 +50,14 @@ def test_chain_inputs_are_not_declared_invariant(name):
     assert set(loads) <= {"wrow"}
 
 
+@pytest.mark.parametrize("name", ["gemm_f32_tc_kernel", "gemm_pair_kernel", "gemm_tmem_kernel"])
+def test_bounded_waits_follow_the_dependency_wait(name):
+    """The lane that issues products waits for operands with a bound; a long predecessor must not use the bound up."""
+    body = KERNELS[name][2]
+    issue = body[body.index("constexpr uint32_t idesc"):]
+    assert 0 <= issue.index("pdl_wait()") < issue.index("mbar_wait(")
+
+
 # M, N, K, E4M3 weights, finished product -> the kernel of few rows takes it: both sides of the lines that its rule draws, all measured
 @pytest.mark.parametrize("M,N,K,f8,finished,takes", [
     (16, 9472, 64, False, True, True), (9, 9473, 64, False, True, False), (9, 9473, 768, False, True, True), (16, 18945, 768, False, False, False),
