@@ -43,7 +43,8 @@ template <int MT, int NC, bool STAGED, bool LN>
 __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, const float* x, int64_t ldx, const float* __restrict__ w,
                                                        int64_t ldw, const float* __restrict__ bias, float* y, int64_t ldy, int accumulate, int ks,
                                                        float act_pos, float act_neg, const float* __restrict__ col_scale, float alpha,
-                                                       const float* __restrict__ ln_gain, const float* __restrict__ ln_bias, float ln_eps) {
+                                                       const float* __restrict__ ln_gain, const float* __restrict__ ln_bias, float ln_eps,
+                                                       int prefetch) {
   extern __shared__ __align__(16) float xs[];
   __shared__ float part[8][MT * NC];
   pdl_trigger();
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
   const int k4_lo = slice * per, k4_hi = min(nk4, k4_lo + per);
   // the weights are constants: the slice streams in while the previous kernel still runs (streaming loads: a step reads its
   // 0.5 GB of weights once each, and they should not push the kernels' code and the activations out of L2)
+  if (!prefetch) pdl_wait();
   float4 wpre[NC][F32_PRE];
 #pragma unroll
   for (int c = 0; c < NC; c++)
@@ -156,7 +158,7 @@ int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
   static SbDeviceOnce once;  // one per instantiation
   SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(gemm_f32_kernel<MT, NC, STAGED, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X_SMEM); }));
   SB_CUDA(sb_launch(ctx, gemm_f32_kernel<MT, NC, STAGED, LN>, grid, dim3(256), smem, (int)g.M, (int)g.N, (int)g.K, g.x, g.ldx, g.w, g.ldw, g.bias, g.y, g.ldy, g.mode, ks,
-                    g.act_pos, g.act_neg, g.col_scale, g.alpha, g.ln_gain, g.ln_bias, g.ln_eps));
+                    g.act_pos, g.act_neg, g.col_scale, g.alpha, g.ln_gain, g.ln_bias, g.ln_eps, ctx->opt.prefetch));
   ctx->launches++;
   return STRICTB200_OK;
 }

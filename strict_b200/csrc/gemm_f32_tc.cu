@@ -36,6 +36,7 @@ struct F32TcArgs {
   GemmF32Args g;
   int ks;       // blocks of a cluster that share K
   int* status;
+  int prefetch; // load the first weights before the dependency wait
 };
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -137,6 +138,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
       for (int h = 0; h < 2; h++)
         rx[i][h] = k + 4 * h < g.K && t0 + r + 32 * i < g.M ? *(const float4*)(xrow + (int64_t)(32 * i) * g.ldx + k + 4 * h) : zero;
     };
+    if (!a.prefetch) pdl_wait();
 #pragma unroll
     for (int i = 0; i < WR; i++) load_w(0, i);  // weights are constants
     pdl_wait();
@@ -274,7 +276,7 @@ int launch(strictb200_ctx* ctx, const GemmF32Args& g) {
   int ks = 1;
   while (ks < 8 && ks * 2 <= nkb && g.K > 1024 * (int64_t)ks) ks *= 2;                          // precision: short running sums
   while (ks < 8 && nkb >= 4 * (int64_t)ks && tn * tt * ks * 2 <= ctx->sm_count) ks *= 2;  // fill the GPU
-  F32TcArgs a{g, ks, ctx->d_status};
+  F32TcArgs a{g, ks, ctx->d_status, ctx->opt.prefetch};
   SB_CUDA(sb_launch_cluster(ctx, gemm_f32_tc_kernel<BT>, dim3((unsigned)tn, (unsigned)tt, (unsigned)ks), dim3(THREADS), smem, dim3(1, 1, (unsigned)ks), a));
   ctx->launches++;
   return STRICTB200_OK;

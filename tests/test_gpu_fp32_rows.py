@@ -59,6 +59,14 @@ def test_gemm_f32_few_rows(ctx, rng, M, N_, K):
     assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
 
 
+@pytest.mark.parametrize("M", [1, 3, 40])
+def test_gemm_f32_without_early_weights(ctx, rng, M):
+    x, w = rng.standard_normal((M, 772)).astype(np.float32), rng.standard_normal((300, 772)).astype(np.float32)
+    want = _gemm(ctx, x, w, None)
+    with ctx.option("prefetch", 0):
+        assert np.array_equal(_gemm(ctx, x, w, None), want)
+
+
 def test_gemm_f32_many_rows_not_finite(ctx, rng):
     """Infinities and NaN reach exactly the results they reach in a plain sum; an operand row at the end of the fp32 range is computed."""
     x, w = rng.standard_normal((40, 200)).astype(np.float32), rng.standard_normal((70, 200)).astype(np.float32)

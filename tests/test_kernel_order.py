@@ -58,6 +58,15 @@ def test_bounded_waits_follow_the_dependency_wait(name):
     assert 0 <= issue.index("pdl_wait()") < issue.index("mbar_wait(")
 
 
+# the option `prefetch` = 0: no weight is requested before the dependency wait. The first request of each product kernel:
+@pytest.mark.parametrize("name,request_", [("gemm_f32_kernel", "__ldcs("), ("gemm_f32_tc_kernel", "load_w(0, i)"), ("gemm_rows_kernel", "= in ? __ldcs("),
+                                           ("gemm_rows_kernel", "load_w(s0)"), ("gemm_tmem_kernel", "tma_load_2d_hint(")])
+def test_weights_wait_where_the_option_says_so(name, request_):
+    body = KERNELS[name][2]
+    wait = re.search(r"if \(!(a\.)?prefetch\) pdl_wait\(\);", body)
+    assert wait and wait.start() < body.index(request_)
+
+
 # M, N, K, E4M3 weights, finished product -> the kernel of few rows takes it: both sides of the lines that its rule draws, all measured
 @pytest.mark.parametrize("M,N,K,f8,finished,takes", [
     (16, 9472, 64, False, True, True), (9, 9473, 64, False, True, False), (9, 9473, 768, False, True, True), (16, 18945, 768, False, False, False),
