@@ -187,6 +187,7 @@ int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float
 int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   const int64_t M = g.M, N = g.N, K = g.K;
   if (K % 4 || g.ldx % 4 || g.ldw % 4) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: K and the row strides must be multiples of 4");
+  if (g.ln_gain && !sb_gemm_f32_takes_norm(M, K)) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: rows for the layer norm in front are at most 8 of 1024");
   // One pass over the weights per eight rows (this kernel) or per 32 to 128 (the tensor cores). Measured, us, rows = 9 / 16 / 32 / 128 / 4700:
   //   N 768  K 768    7.1 / 7.1 / 13.0 /  37.8 / 1197   against   8.5 / 8.5 /  8.7 / 13.9 /  62
   //   N 3072 K 768   13.2 / 19.8 / 33.1 / 119.8 / 6240            9.3 / 9.3 /  9.5 / 14.9 / 192
@@ -196,7 +197,6 @@ int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   // 9.6e-8..1.0e-7 / 1.3e-7 there.
   const bool few = M <= 4 || (M <= F32_MT && (g.ln_gain || N * K <= (8 << 20))) || (M <= 2 * F32_MT && N * K <= (1 << 20));
   if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) return k_gemm_f32_tc(ctx, g);
-  if (g.ln_gain && !sb_gemm_f32_takes_norm(M, K)) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: rows for the layer norm in front are at most 8 of 1024");
   // Warps per output channel: slices of at most 1024 columns, and two for a long enough row, while all blocks are resident at once (two
   // per SM with the norm in front or several rows, else four); two channels per warp where they would not be. With the norm in front
   // 3072 channels of 768 columns took 6.6 us as 384 blocks of two waves, 3.0 us as 192.

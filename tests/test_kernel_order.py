@@ -67,6 +67,25 @@ def test_weights_wait_where_the_option_says_so(name, request_):
     assert wait and wait.start() < body.index(request_)
 
 
+# a layer norm in front of the product is refused beyond the rows and columns that the row kernel norms, not left out
+@pytest.mark.parametrize("M,K", [(9, 768), (4700, 768), (8, 1028)])
+def test_norm_in_front_is_not_dropped(M, K):
+    import ctypes as C
+    from strict_b200 import native
+
+    class Args(C.Structure):
+        _fields_ = [("M", C.c_int64), ("N", C.c_int64), ("K", C.c_int64), ("x", C.c_void_p), ("ldx", C.c_int64), ("w", C.c_void_p), ("ldw", C.c_int64),
+                    ("bias", C.c_void_p), ("y", C.c_void_p), ("ldy", C.c_int64), ("mode", C.c_int), ("act_pos", C.c_float), ("act_neg", C.c_float),
+                    ("col_scale", C.c_void_p), ("alpha", C.c_float), ("ln_gain", C.c_void_p), ("ln_bias", C.c_void_p), ("ln_eps", C.c_float)]
+
+    here = C.create_string_buffer(4096)  # stands for a context and for data: a refused call reads neither
+    p = C.addressof(here)
+    f = native.lib()._Z10k_gemm_f32P14strictb200_ctxRK11GemmF32Args
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_void_p]
+    a = Args(M=M, N=3072, K=K, x=p, ldx=K, w=p, ldw=K, y=p, ldy=3072, alpha=1, ln_gain=p, ln_bias=p, ln_eps=1e-5)
+    assert f(p, C.addressof(a)) == native.ERR_INVALID_ARG
+
+
 # M, N, K, E4M3 weights, finished product -> the kernel of few rows takes it: both sides of the lines that its rule draws, all measured
 @pytest.mark.parametrize("M,N,K,f8,finished,takes", [
     (16, 9472, 64, False, True, True), (9, 9473, 64, False, True, False), (9, 9473, 768, False, True, True), (16, 18945, 768, False, False, False),
