@@ -193,8 +193,8 @@ int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   //   N 3072 K 768   13.2 / 19.8 / 33.1 / 119.8 / 6240            9.3 / 9.3 /  9.5 / 14.9 / 192
   //   N 1000 K 100    4.3 / 4.4 /  6.2 /  19.8 /  676            6.2 / 7.1 /  7.2 / 13.7 /  28
   // so two passes over a small matrix stay here, and five to eight rows over a large one go there (4096 x 4096: 46.8 us against 26.4).
-  // Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336): 9.2e-8 / 1.0e-7 / 1.6e-7 here, 8.0e-8..9.1e-8 /
-  // 9.6e-8..1.0e-7 / 1.3e-7 there.
+  // Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336): 9.2e-8 / 1.0e-7 / 1.6e-7 here, 7.6e-8..8.7e-8 /
+  // 9.6e-8 / 1.3e-7 there.
   const bool few = M <= 4 || (M <= F32_MT && (g.ln_gain || N * K <= (8 << 20))) || (M <= 2 * F32_MT && N * K <= (1 << 20));
   if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) return k_gemm_f32_tc(ctx, g);
   // Warps per output channel: slices of at most 1024 columns, and two for a long enough row, while all blocks are resident at once (two

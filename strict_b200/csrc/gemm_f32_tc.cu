@@ -1,14 +1,19 @@
 // fp32 linear layers of many rows on the tcgen05 tensor cores, without giving up fp32 results: Y[M,N] = X[M,K] . W[N,K]^T + bias.
 //
-// Every fp32 value is the exact sum of three bf16 terms, x = x0 + x1 + x2 (8 + 8 + 8 significant bits, each remainder exact).
-// Of the nine products of two values the six largest are computed, w0x0 + (w0x1 + w1x0) + (w0x2 + w1x1 + w2x0); the rest lies
-// below 2^-25 of the product, as far down as fp32's own rounding. A tensor core multiplies bf16 exactly, but it cuts its fp32
+// Every fp32 value is the exact sum of three bf16 terms, x = x0 + 2^-8 x1 + 2^-16 x2 (8 + 8 + 8 significant bits, each remainder exact).
+// The factors keep the terms where bf16 has bits: without them a value below 2^-110 would lose bits of its last term, one below 2^-118 of two.
+// (Below 2^-126, where fp32 itself ends in units of 2^-149, the terms no longer shrink by 2^-8, and the products left out amount to at
+// most half of such a unit of the value.)
+// Of the nine products of two values the six largest are computed, w0x0 + 2^-8 (w0x1 + w1x0) + 2^-16 (w0x2 + w1x1 + w2x0); the rest lies
+// below 2^-24 of the product, as far down as the rounding of an fp32 product. A tensor core multiplies bf16 exactly, but it cuts its fp32
 // sum off after every instruction (measured: 1e-8 of the result towards zero per 16 columns, 6e-7 after 768), so
 //   - the large product w0x0 is summed over 32 columns at a time in tensor memory; two such sums are added and then added to the
 //     running sum in registers, where fp32 addition rounds to nearest;
-//   - the five small ones stay in one tensor-memory accumulator for all of K: what is cut off there is 2^-8 times smaller;
-//   - no block walks more than about 1024 columns: longer rows are shared by the blocks of a cluster, whose sums are added in
-//     block order through distributed shared memory (and few tiles are shared the same way to fill the GPU).
+//   - the small ones stay in tensor memory for all of a block's columns, a sum for each factor: what is cut off there is 2^-8 times
+//     smaller or less;
+//   - no block walks more than about 1024 columns, or an eighth of K where that is more: longer rows are shared by the up to eight
+//     blocks of a cluster, whose sums are added in block order through distributed shared memory (and few tiles are shared the same
+//     way to fill the GPU).
 // Measured error against 64 bits (2-norm, normal operands; in brackets the row kernel of gemm_f32.cu, all plain fp32 FMAs):
 // see the table at k_gemm_f32 in gemm_f32.cu.
 //
@@ -50,12 +55,12 @@ __device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-// Two values -> their bf16 terms, packed (the first value in the low half); u and v become the remainders.
+// Two values -> their bf16 terms, packed (the first value in the low half); u and v become 2^8 times the remainders.
 __device__ __forceinline__ uint32_t take_term(float& u, float& v) {
   uint32_t t;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t) : "f"(v), "f"(u));
-  u = __fsub_rn(u, __uint_as_float(t << 16));
-  v = __fsub_rn(v, __uint_as_float(t & 0xFFFF0000u));
+  u = __fmul_rn(256.f, __fsub_rn(u, __uint_as_float(t << 16)));
+  v = __fmul_rn(256.f, __fsub_rn(v, __uint_as_float(t & 0xFFFF0000u)));
   return t;
 }
 // Eight columns of one row into the three planes at this shared-memory address.
@@ -88,7 +93,7 @@ __device__ __forceinline__ void finish(const GemmF32Args& g, int tok, int n, flo
 template <int BT>
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
   constexpr int X_PLANE = BT * 128, STAGE = 3 * (W_PLANE + X_PLANE);
-  constexpr int COLS = 3 * BT <= 128 ? 128 : 3 * BT <= 256 ? 256 : 512;  // two partial sums of the large product, one of the small ones
+  constexpr int COLS = 4 * BT;  // two partial sums of the large product, the sums of the small ones
   constexpr int HALF = BT / 2;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[NSTAGE], bar_empty[NSTAGE], bar_sum_full, bar_sum_empty;
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
   } else if (warp == FEEDERS) {
     if (lane == 0) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(CH >> 4) << 24);
-      const uint32_t big = tmem, small = tmem + 2 * BT;
+      const uint32_t big = tmem, small1 = tmem + 2 * BT, small2 = tmem + 3 * BT;
       // The operand tiles cannot arrive before the feeders' dependency wait has returned: the same wait here keeps the bounded ones below for
       // progress inside this kernel, however long its predecessor takes.
       pdl_wait();
@@ -183,11 +188,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint64_t o = (uint64_t)(2 * j);  // 16 columns = 32 bytes inside the swizzle atom
-          tc_mma_ss(small, w[0] + o, x[1] + o, idesc, (kb | j) ? 1u : 0u);
-          tc_mma_ss(small, w[0] + o, x[2] + o, idesc, 1u);
-          tc_mma_ss(small, w[1] + o, x[0] + o, idesc, 1u);
-          tc_mma_ss(small, w[1] + o, x[1] + o, idesc, 1u);
-          tc_mma_ss(small, w[2] + o, x[0] + o, idesc, 1u);
+          tc_mma_ss(small1, w[0] + o, x[1] + o, idesc, (kb | j) ? 1u : 0u);
+          tc_mma_ss(small1, w[1] + o, x[0] + o, idesc, 1u);
+          tc_mma_ss(small2, w[0] + o, x[2] + o, idesc, (kb | j) ? 1u : 0u);
+          tc_mma_ss(small2, w[1] + o, x[1] + o, idesc, 1u);
+          tc_mma_ss(small2, w[2] + o, x[0] + o, idesc, 1u);
         }
         if (kb && !mbar_wait(smem_u32(&bar_sum_empty), (kb - 1) & 1)) { set_status(a.status, 4); abort_flag = 1; break; }
         tc_fence_after();
@@ -225,12 +230,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(F32TcArgs a) {
     }
     if (ok) {
 #pragma unroll
-      for (int q = 0; q < HALF; q += 16) {
-        uint32_t u[16];
-        tc_ld16(at + 2 * BT + q, u);
+      for (int q = 0; q < HALF; q += 8) {
+        uint32_t u[8], v[8];
+        tc_ld8(at + 2 * BT + q, u);
+        tc_ld8(at + 3 * BT + q, v);
         tc_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; i++) sum[q + i] = __fadd_rn(sum[q + i], __uint_as_float(u[i]));
+        for (int i = 0; i < 8; i++) sum[q + i] = __fmaf_rn(0x1p-8f, __fmaf_rn(0x1p-8f, __uint_as_float(v[i]), __uint_as_float(u[i])), sum[q + i]);
       }
       // the stages have been read by every product: they become [token][channel] sums of this block
       const uint32_t to = smem + (uint32_t)((half * HALF * CH + lg * 32 + lane) * 4);

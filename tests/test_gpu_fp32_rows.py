@@ -59,6 +59,22 @@ def test_gemm_f32_few_rows(ctx, rng, M, N_, K):
     assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
 
 
+# operands down to the end of the fp32 range, of one side or both, next to ones that bring the products back: the terms of a value below 2^-110
+# would end in bits that bf16 does not have
+@pytest.mark.parametrize("ex,ew", [(-112, 60), (-118, 100), (-125, 0), (-125, 120), (120, -124), (-60, -60), (-135, 126), (-147, 126)])
+def test_gemm_f32_many_rows_small_operands(ctx, rng, ex, ew):
+    M, N_, K = 48, 136, 260
+    x = np.ldexp(rng.uniform(1, 2, (M, K)) * rng.choice([-1, 1], (M, K)), ex).astype(np.float32)
+    w = np.ldexp(rng.uniform(1, 2, (N_, K)) * rng.choice([-1, 1], (N_, K)), ew).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm(ctx, x, w, None)
+    # as above, and one unit at the end of the fp32 range per instruction and addition; of a value below 2^-126 the products left out are w1 x2 and
+    # w2 x1, 2^-9 and 2^-17 of w times what lies below 2^-141 and 2^-133: half a unit of the value
+    left_out = 2.0 ** -150 * np.abs(w).astype(np.float64).sum(1) if ex < -126 else 0
+    assert (np.abs(got - want) <= (6 + 1024 / 64 + 8) * 2.0 ** -24 * size + (K / 16 + 16) * 2.0 ** -149 + left_out).all()
+
+
 @pytest.mark.parametrize("M", [1, 3, 40])
 def test_gemm_f32_without_early_weights(ctx, rng, M):
     x, w = rng.standard_normal((M, 772)).astype(np.float32), rng.standard_normal((300, 772)).astype(np.float32)
