@@ -130,3 +130,59 @@ def test_gpt2_prompts_and_decode(ctx, oracle, head_dim, lens, d_ff):
     for o in (kv, m):
         o.dispose()
     st.close(), om.close()
+
+
+@pytest.mark.parametrize("head_dim", [64, 48])
+def test_gpt2_infinite_token_does_not_reach_earlier_rows(ctx, oracle, head_dim):
+    """Rows of a prompt in front of a token with an infinite embedding, of the same 64 keys and of others, are what they are without it."""
+    cfg = dict(TINY_GPT2, d_model=2 * head_dim, head_dim=head_dim, d_ff=4 * head_dim, max_pos=256, vocab=300)
+    m = sb.Model(ctx, cfg).init_random(3)
+    toks = oracle.gen_tokens(3, 1, 150, 299).reshape(1, 150)
+    kv = m.new_cache(1, 200)
+    _, clean = kv.prefill_rows(toks, [range(150)])
+    embed = m.get_tensor("embed", np.float32, 300 * cfg["d_model"]).reshape(300, -1)
+    embed[299, 5] = np.inf
+    m.set_tensor("embed", embed)
+    for at in (1, 50, 63, 64, 130):
+        toks2 = toks.copy()
+        toks2[0, at] = 299
+        kv.reset()
+        _, rows = kv.prefill_rows(toks2, [range(150)])
+        assert np.array_equal(rows[:at, :299], clean[:at, :299]) and np.isnan(rows[at:, :299]).all()
+    kv.dispose(), m.dispose()
+
+
+@pytest.mark.parametrize("head_dim", [32, 64, 128, 48])
+def test_gpt2_scores_of_minus_infinity(ctx, oracle, head_dim):
+    """The first 70 keys of every sequence score -inf, more than a tile of a prompt and more than every group of a decode row sees first: they weigh
+    nothing, and the others all the same. Rows with no other key are NaN."""
+    d = 2 * head_dim
+    cfg = dict(TINY_GPT2, n_layers=1, d_model=d, head_dim=head_dim, d_ff=4 * head_dim, max_pos=256, vocab=300)
+    m, om = sb.Model(ctx, cfg).init_random(7), oracle.Model(cfg, 7)
+    t = {n: np.array(om.tensor(n, np.float32)) for n in ("embed", "wpe", "layers.0.wqkv.w", "layers.0.wqkv.b")}
+    embed, wpe, w, b = t["embed"].reshape(300, d), t["wpe"].reshape(256, d), t["layers.0.wqkv.w"].reshape(3 * d, d), t["layers.0.wqkv.b"]
+    embed[:10], wpe[:] = 0, 0                       # ids 0..9 add nothing to the position
+    wpe[:70, 0], wpe[:70, 1] = 1, -1                # a normed column 0 that is not zero for the first 70 positions only
+    for p in range(70, 256):
+        wpe[p, 2 + 2 * (p % 5)], wpe[p, 3 + 2 * (p % 5)] = 1, -1
+    w[:2 * d], b[:2 * d] = 0, 0
+    b[0:d:head_dim], w[d:2 * d:head_dim, 0] = 1e20, -1e30
+    for n, v in t.items():
+        m.set_tensor(n, v)
+        om.tensor(n, np.float32)[:] = v
+    om.retie()
+    lens = np.array([71, 70, 128, 150], np.int32)
+    toks = np.random.default_rng(1).integers(0, 10, (4, 150)).astype(np.int32)
+    kv, st = m.new_cache(4, 200), om.new_state(4, 200)
+    _, logits = kv.prefill(toks, lens, want_logits=True)
+    want = st.prefill(toks, lens)
+    assert np.isnan(want[1]).all() and np.isfinite(want[[0, 2, 3]]).all()
+    for step in range(3):
+        assert np.allclose(logits, want, rtol=0, atol=2e-5, equal_nan=True)
+        ids = np.full(4, step, np.int32)
+        _, logits = kv.decode_step(ids, want_logits=True)
+        want = st.decode(ids)
+    assert np.isfinite(want).all() and np.allclose(logits, want, rtol=0, atol=2e-5)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
