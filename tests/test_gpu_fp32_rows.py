@@ -24,9 +24,9 @@ def _gemm(ctx, x, w, b):
 
 
 # rows around the token tiles (32, 64, 128), channels around a block's 128, columns around the 64 of a stage, the 1024 of a block and
-# two and eight blocks of a cluster
-@pytest.mark.parametrize("M,N_,K", [(9, 1, 4), (31, 127, 60), (32, 128, 64), (33, 129, 68), (64, 130, 1024), (65, 257, 1028), (128, 768, 3072),
-                                    (129, 300, 772), (300, 96, 8200), (1000, 40, 14336)])
+# two and eight blocks of a cluster; the fewest rows that come here, with a large matrix
+@pytest.mark.parametrize("M,N_,K", [(17, 1, 4), (31, 127, 60), (32, 128, 64), (33, 129, 68), (64, 130, 1024), (65, 257, 1028), (128, 768, 3072),
+                                    (129, 300, 772), (300, 96, 8200), (1000, 40, 14336), (5, 2800, 3072), (9, 1366, 772)])
 def test_gemm_f32_many_rows(ctx, rng, M, N_, K):
     x = (rng.standard_normal((M, K)) * np.exp2(rng.integers(-6, 7, (M, K)))).astype(np.float32)
     w = (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
@@ -44,8 +44,9 @@ def test_gemm_f32_many_rows(ctx, rng, M, N_, K):
     assert np.allclose(_gemm(ctx, x, w, b), got + b, rtol=1e-6, atol=1e-6 * np.abs(got).max())
 
 
-# the row kernel's instances: one to eight rows, one or two channels per warp, rows split over warps, rows of X that do not fit shared memory
-@pytest.mark.parametrize("M,N_,K", [(1, 9600, 300), (2, 2500, 768), (3, 4999, 1028), (4, 2400, 2048), (4, 40, 6200), (7, 500, 512), (8, 6001, 64),
+# the row kernel's instances: one to eight rows, one or two channels per warp, rows split over warps, rows of X that do not fit shared memory,
+# two passes over a small matrix
+@pytest.mark.parametrize("M,N_,K", [(9, 1, 4), (1, 9600, 300), (2, 2500, 768), (3, 4999, 1028), (4, 2400, 2048), (4, 40, 6200), (7, 500, 512), (8, 6001, 64),
                                     (8, 300, 12000), (16, 700, 1200)])
 def test_gemm_f32_few_rows(ctx, rng, M, N_, K):
     x, w = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)

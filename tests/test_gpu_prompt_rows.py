@@ -12,11 +12,13 @@ pytestmark = pytest.mark.gpu
 L = N.lib
 
 
-# feed-forwards that end inside a tile of 128 channels; more than eight token tiles of 128 and an odd rest of them; norms of one, two and
-# eight column groups per thread (the last with a width that is no multiple of 128 and takes other products); more than 32 and fewer heads
+# feed-forwards that end inside a tile of 128 channels; more than eight token tiles of 128 and an odd rest of them; more than 32 and fewer heads; the
+# norm of whole rows (more than 1024 of them, or a width that is no multiple of 128 and takes other products) with one, two, four and
+# eight column groups per thread
 @pytest.mark.parametrize("over,lens", [(dict(d_ff=192), [100, 77, 40]), (dict(d_ff=320, n_q_heads=36, n_kv_heads=3, head_dim=128), [90, 211]),
-                                       (dict(d_model=1152, d_ff=128), [700, 520]), (dict(d_model=4160, d_ff=128), [12, 9]), (dict(d_model=2048, d_ff=256), [1100])],
-                         ids=["ff192", "heads42", "d1152", "d4160", "d2048"])
+                                       (dict(d_model=1152, d_ff=128), [700, 520]), (dict(d_model=4160, d_ff=128), [12, 9]), (dict(d_model=2048, d_ff=256), [1100]),
+                                       (dict(d_model=640, d_ff=128), [1030]), (dict(d_model=2176, d_ff=128), [600, 430])],
+                         ids=["ff192", "heads42", "d1152", "d4160", "d2048", "d640", "d2176"])
 def test_prompts_vs_oracle(ctx, oracle, over, lens):
     cfg = dict(TINY_QWEN, n_layers=2, vocab=512, max_pos=1200, **over)
     m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 7, len(lens), max(lens), lens, 1, random_gains=True)
