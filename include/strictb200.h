@@ -107,7 +107,7 @@ int strictb200_trace_end(strictb200_ctx* ctx, uint64_t* out_records, int max_rec
  * library's own choice. Names: "pdl" (programmatic dependent launch, 1), "attn_tc" (prefill
  * attention kernel: 0 mma.sync, 1 tcgen05 one query tile per block, 2 two tiles per block, -1),
  * "gemm_pair" (many-token GEMM on SM pairs, 1), "prefetch" (1), "deep_ring" (1),
- * "attn_blocks_per_sm" (0), "split_target" (0), "tp_two_shot" (fused all-reduce in two shots,
+ * "attn_blocks_per_sm" (0), "split_target" (0; products of 128-channel tiles), "tp_two_shot" (fused all-reduce in two shots,
  * -1: with more than four ranks), "wait_limit" (polls of a cross-rank wait before it gives up,
  * 4194304), "prefill_chunk" (token rows per prefill chunk, 16384), "fuse_rope" (decode attention applies
  * QK-norm and RoPE and appends to the cache itself, -1: with at most 16 sequences and an unsplit projection), "row_cluster" (blocks of one cluster that share a row in the decode row

@@ -175,7 +175,7 @@ int k_gemm_int8w(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const int
   g.wq = (const uint8_t*)wq; g.ldw = K; g.sw = sw;
   g.out = y; g.out_f32 = 0; g.part = (float*)part; g.splits = splits; g.raw = 0; g.kernel = 3; g.i8 = 1;
   // More than one tile of tokens: SM pairs and 256 x 256 tiles, the line of the E4M3 path (k_gemm_fp8_tmem). Linear layer of 2048 tokens,
-  // 4096 x 4096: 110 us with 128 x 256 tiles of one SM each, one launch of blocks per tile, and a quantiser of two-byte loads; 75 us so.
+  // 4096 x 4096: 110 us with 128 x 256 tiles of one SM each, one launch of blocks per tile, and a quantiser of two-byte loads; 77 us so.
   const int64_t rows = sb_qrows(M);
   if (splits == 1 && ctx->opt.gemm_pair && rows > 256 && rows <= 65535 * 256 && N >= 256 && ctx->sm_count >= 2) return k_gemm_int8_tmem_pair(ctx, g);
   SB_TRY(k_gemm_fp8_tmem_split(ctx, g));

@@ -281,10 +281,11 @@ SB_TRACE_TU(gemm_rows)
 // round of blocks (one_round), two with two tiles per block and at most 8 rows. us, 8 / 16 rows against the large tiles:
 //   N 16384 K 256   4.1 / 5.9 against 4.6    N 18944 K 3072  18.9 against 20.1       N 9472 K 1024  4.9 / 5.4 against 7.6
 //   N 32768 K 256   7.7 / 11.2 against 5.1   N 32768 K 2048  23.8 against 20.6       N 9600 K 256 5.1 (16), K 768 6.4 against 4.4, 6.5
-// E4M3 weights, whose large tiles are half as long a stream and whose conversion is work here: 1 / 16 rows, us, the row split in front included,
-//   N 4096 K 1024  8.1 / 8.0 -> 5.9 / 5.9     N 1024 K 3072  8.1 / 8.4 -> 7.9 / 7.9     N 1024 K 14336  12.4 / 12.8 -> 10.8 / 12.6
-//   N 6144 K 1024  8.1 / 8.0 -> 5.8 / 5.8     N 4096 K 4096  9.6 / 10.6, 9.9 / 12.6 here; N 6144 K 4096  10.4 / 11.0, 13.1 / 16.9 here
-// and without it, 8 / 16 rows against the large tiles:
+// E4M3 weights, whose large tiles are half as long a stream and whose conversion is work here. Whole calls on bf16 rows (the row split in front
+// included, weights from HBM), 1 / 16 rows, us, before and with this kernel (2 to 3 us of it the split's overlap):
+//   N 4096 K 1024  10.2 / 10.4 -> 6.3 / 6.5   N 1024 K 3072  10.4 / 11.4 -> 8.3 / 8.4   N 1024 K 14336  16.5 / 16.5 -> 10.5 / 13.0
+//   N 6144 K 1024  10.3 / 10.4 -> 6.3 / 6.3   N 4096 K 4096  9.6 / 10.6 on the large tiles, 9.9 / 12.6 here; N 6144 K 4096  10.4 / 11.0, 13.1 / 16.9 here
+// and without the split, 8 / 16 rows against the large tiles:
 //   N 16384 K 512  5.4 against 6.9    N 9600 K 256   4.4 / 5.3 against 4.7    N 12288 K 640  5.1 / 7.3 against 6.7
 //   N 16384 K 256  5.0 against 4.6    N 32768 K 256  9.6 / 12.0 against 4.7   N 6144 K 1280 (two splits)  6.6 / 8.6 against 6.7
 // A decode step of Qwen3-0.6B: 774 -> 711 us (batch 1).
