@@ -261,11 +261,13 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
   constexpr int D = 4 * LANES, GROUPS = 512 / LANES, BATCH = 8;
   __shared__ float red_m[GROUPS], red_l[GROUPS];
   __shared__ __align__(16) float red_o[GROUPS][D];
+  SB_TRACE_BEGIN();
   pdl_trigger();
   const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x % LANES, grp = threadIdx.x / LANES, hd = H * D;
   float* kb = kc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
   float* vb = vc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
   pdl_wait();
+  SB_TRACE_WAITED();
   const int p = lens[b];
   if (p < 0 || p >= maxlen) return;
   const float* row = qkv + (int64_t)b * 3 * hd + h * D + 4 * c;
@@ -313,6 +315,7 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
       }
     }
   }
+  SB_TRACE_MARK(0);
   if (c == 0) { red_m[grp] = m; red_l[grp] = l; }
   *(float4*)&red_o[grp][4 * c] = o;
   __syncthreads();
@@ -328,8 +331,11 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
     }
     out[(int64_t)b * hd + h * D + threadIdx.x] = acc * (1.0f / sum);
   }
+  SB_TRACE_END(SB_K_ATTN, 0);
 }
 }  // namespace
+
+SB_TRACE_TU(attention_f32)
 
 int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, const int32_t* seq, const int32_t* pos, const int32_t* lens,
                int64_t T, int H, int Dh, int maxlen, float scale, float* out, const F32Prompts* prompts) {

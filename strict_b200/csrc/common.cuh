@@ -316,6 +316,28 @@ int k_gemm_rows_fp8_bf16(strictb200_ctx*, const GemmArgs& g);
 int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
 // gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
 // Where a finished value goes. Columns from n_switch on (0 = none) belong to a second product of the same launch: its
+// gemm_rows_chain.cu: the same rows, the norm of the residual in front of a product, and a product added to the residual
+struct NormRowsGemm {
+  int64_t M = 0, N = 0, K = 0;  // out [M,N] = norm(x) . w^T, x [M,K] fp32, rounded to bf16 after the norm; w [N,K] E4M3
+  const float *x = nullptr, *gain = nullptr;
+  float eps = 0.f;
+  const uint8_t* w = nullptr;
+  const float* sw = nullptr;    // [N] scales of the channels (out_glu only: out takes the raw sums)
+  float* out = nullptr;
+  bf16* out_glu = nullptr;      // w = [gate | up]: [M, N / 2] silu(gate) * up instead
+  float* ones = nullptr;        // [M] = 1 (may be null)
+};
+bool sb_norm_rows_takes(int64_t M, int64_t N, int64_t K);
+int k_norm_rows(strictb200_ctx*, const NormRowsGemm& g);
+struct ResidualRowsGemm {
+  int64_t M = 0, N = 0, K = 0;  // res [M,N] += (x . w^T) * sw, x [M,K] bf16, w [N,K] E4M3
+  const bf16* x = nullptr;
+  const uint8_t* w = nullptr;
+  const float* sw = nullptr;
+  float* res = nullptr;
+};
+bool sb_residual_rows_takes(int64_t M, int64_t N, int64_t K);
+int k_residual_rows(strictb200_ctx*, const ResidualRowsGemm& g);
 // operand rows are x_row_off + m, and with act_out set the value leaves through the activation.
 struct Bf16Epilogue {
   float* out_f32 = nullptr;   // [M, ldo]
@@ -573,10 +595,11 @@ size_t sb_attn_decode_scratch(int B, int Hq, int D, int nsplit);
 int sb_attn_decode_splits(strictb200_ctx*, int B, int Hkv, int maxlen);
 int sb_attn_decode_chunk(strictb200_ctx*, int B, int Hkv, int maxlen, int len_plan, bool fused = false);  // keys per block for sequences of about len_plan keys (at most 8 chunks cover maxlen)
 // rope != null: the queries and the new token's key/value rows are computed inside the attention kernel from the qkv
-// projection's partial results (what k_rope_qknorm_kvappend would do in a kernel of its own); q is then unused
+// projection's partial results (what k_rope_qknorm_kvappend would do in a kernel of its own); q is then unused.
+// cluster_merge: at most 8 key chunks, merged inside a cluster straight to bf16 rows (no q_out, no scratch)
 int k_attn_decode(strictb200_ctx*, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, int len_add, int B, int Hq,
                   int Hkv, int D, int maxlen, float scale, int nsplit, float* scratch, bf16* out, uint8_t* q_out, float* qscale_out,
-                  const RopeArgs* rope = nullptr, int chunk = 0);
+                  const RopeArgs* rope = nullptr, int chunk = 0, bool cluster_merge = false);
 int k_attn_decode_chunks(strictb200_ctx*, int HD, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* lens, int B, int Hq, int Hkv, int maxlen,
                          float scale, int nsplit, int chunk, float* o_part, float* ml_part);
 // attention_f32.cu. `prompts` (with seq and pos): the rows as sequences b0.. of the cache, one after the other

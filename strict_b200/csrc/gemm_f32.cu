@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
   extern __shared__ __align__(16) float xs[];
   __shared__ float part[8][MT * NC];
   pdl_trigger();
+  SB_TRACE_BEGIN();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = 8 / ks, slice = warp % ks;
   const int n0 = (blockIdx.x * groups + warp / ks) * NC;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
   const float bn = bias && lane < NC && oc < N ? bias[oc] : 0.f;
   pdl_wait();
   if (LN) {
+  SB_TRACE_WAITED();
     if (warp < mt) {  // a warp per row
       const float4* xr = (const float4*)(x + (int64_t)(m0 + warp) * ldx);
       float4 v[F32_PRE];
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
     __syncthreads();
   }
   float acc[NC * MT];
+  SB_TRACE_MARK(0);
 #pragma unroll
   for (int i = 0; i < NC * MT; i++) acc[i] = 0.f;
   auto fma_rows = [&](int k4, const float4* wv) {
@@ -134,6 +137,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
     fma_rows(k4, wv);
   }
   constexpr int VALS = NC * MT, STEP = 32 / VALS;
+  SB_TRACE_MARK(1);
   const float sum = fold_sums<VALS>(acc, lane);
   if (lane % STEP == 0) part[warp][lane / STEP] = sum;
   __syncthreads();
@@ -148,6 +152,7 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
     }
   }
 }
+  SB_TRACE_END(SB_K_GEMM, (uint32_t)N ^ ((uint32_t)K << 12));
 
 template <int MT, int NC, bool STAGED, bool LN>
 int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
@@ -176,6 +181,8 @@ int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks, bool two) {
 }  // namespace
 
 bool sb_gemm_f32_takes_norm(int64_t M, int64_t K) { return M <= F32_MT && K <= LN_K; }
+SB_TRACE_TU(gemm_f32)
+
 
 int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float* x, const float* w, const float* bias, float* y,
                int accumulate) {

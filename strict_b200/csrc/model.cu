@@ -53,6 +53,15 @@ bool fuses_rope(strictb200_model* m, int64_t B, int s1) {
   return (fuse < 0 ? B <= 16 && s1 == 1 : fuse > 0) && s1 <= 8 && m->Hq_l / m->Hkv_l <= 16;
 }
 
+// A step of few sequences of a narrow model: norms in front of the products, sums straight into the residual, key chunks merged inside
+// their cluster (gemm_rows_chain.cu): 5 launches per layer instead of 8.
+bool chained_step(strictb200_model* m, int64_t B) {
+  const auto& c = m->c;
+  const int64_t d = c.d_model, nq = (int64_t)m->Hq_l * c.head_dim, nqkv = nq + 2 * (int64_t)m->Hkv_l * c.head_dim;
+  return m->world == 1 && m->I_l % 16 == 0 && m->Hq_l / m->Hkv_l <= 16 && sb_norm_rows_takes(B, nqkv, d) && sb_norm_rows_takes(B, 2 * (int64_t)m->I_l, d) &&
+         sb_residual_rows_takes(B, d, nq) && sb_residual_rows_takes(B, d, m->I_l);
+}
+
 void carve_decode(strictb200_kv* kv, char* base, DecBuf* out, size_t* total) {
   strictb200_model* m = kv->m;
   const auto& c = m->c;
@@ -180,7 +189,46 @@ namespace {
 // ------------------------------------------------------------------ Qwen3 decode step body
 // Everything below is enqueued on the stream with device-resident state only, so the whole
 // body can be captured into a CUDA graph.
+int qwen_chained_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
+  strictb200_ctx* ctx = m->ctx;
+  const auto& c = m->c;
+  const int64_t B = kv->B, d = c.d_model, D = c.head_dim, nq = (int64_t)m->Hq_l * D, nqkv = nq + 2 * (int64_t)m->Hkv_l * D;
+  PROF(STRICTB200_K_EMBED, k_embedding_bf16_f32(ctx, m->embed, kv->d_ids, B, d, c.vocab, b.x));
+  NormRowsGemm in;
+  in.M = B; in.K = d; in.x = b.x; in.eps = c.eps;
+  ResidualRowsGemm out;
+  out.M = B; out.N = d; out.res = b.x;
+  bf16* glu = (bf16*)b.gu;
+  for (int l = 0; l < c.n_layers; l++) {
+    LayerW& w = m->L[l];
+    in.N = nqkv; in.gain = w.norm1_g; in.w = w.wqkv.q; in.out = b.part; in.out_glu = nullptr; in.ones = b.red;
+    PROF(STRICTB200_K_GEMM_QKV, k_norm_rows(ctx, in));
+    RopeArgs r;
+    r.part = b.part; r.splits = 1; r.sx = b.red; r.sw = w.wqkv.s; r.lens = kv->d_lens;
+    r.cos_t = m->rope_cos; r.sin_t = m->rope_sin; r.qgain = w.qn_g; r.kgain = w.kn_g; r.eps = c.eps;
+    r.Hq = m->Hq_l; r.Hkv = m->Hkv_l; r.D = (int)D; r.maxlen = kv->maxlen; r.max_pos = c.max_pos;
+    r.q_out = b.qb; r.kcache = kv_k(kv, l); r.vcache = kv_v(kv, l);
+    const bool fuse_rope = fuses_rope(m, B, 1);
+    if (!fuse_rope) PROF(STRICTB200_K_ROPE, k_rope_qknorm_kvappend(ctx, r, B));
+    PROF(STRICTB200_K_ATTN, k_attn_decode(ctx, b.qb, kv_k(kv, l), kv_v(kv, l), kv->d_lens, 1, (int)B, m->Hq_l, m->Hkv_l, (int)D, kv->maxlen, 1.0f / sqrtf((float)D),
+                                          kv->nsplit, b.attn_ws, b.att, nullptr, nullptr, fuse_rope ? &r : nullptr, kv->chunk, true));
+    out.K = nq; out.x = b.att; out.w = w.wo.q; out.sw = w.wo.s;
+    PROF(STRICTB200_K_GEMM_O, k_residual_rows(ctx, out));
+    in.N = w.wgu.N; in.gain = w.norm2_g; in.w = w.wgu.q; in.sw = w.wgu.s; in.out = nullptr; in.out_glu = glu; in.ones = nullptr;
+    PROF(STRICTB200_K_GEMM_GU, k_norm_rows(ctx, in));
+    out.K = m->I_l; out.x = glu; out.w = w.wdown.q; out.sw = w.wdown.s;
+    PROF(STRICTB200_K_GEMM_DOWN, k_residual_rows(ctx, out));
+  }
+  RowNormArgs a;
+  a.x_f32 = b.x; a.gain = m->normf_g; a.eps = c.eps; a.q = b.aq; a.qscale = b.sa;
+  PROF(STRICTB200_K_ROWNORM, k_rownorm(ctx, a, B, d));
+  PROF(STRICTB200_K_HEAD, head_and_pick(m, B, b.aq, b.sa, b, kv->d_next, nullptr, (int)B));
+  PROF(STRICTB200_K_EMBED, k_add_i32(ctx, kv->d_lens, nullptr, 1, B));
+  return STRICTB200_OK;
+}
+
 int qwen_decode_body(strictb200_model* m, strictb200_kv* kv, DecBuf& b) {
+  if (kv->nsplit <= 8 && chained_step(m, kv->B)) return qwen_chained_body(m, kv, b);
   strictb200_ctx* ctx = m->ctx;
   const auto& c = m->c;
   const int64_t B = kv->B, d = c.d_model, D = c.head_dim;
@@ -346,7 +394,7 @@ int decode_enqueue(strictb200_model* m, strictb200_kv* kv) {
     for (int b = 0; b < kv->B; b++) longest = std::max(longest, kv->h_lens[b] + 1);
     if (!kv->chunk || longest > kv->plan_until) {
       const int64_t nqkv = ((int64_t)m->Hq_l + 2 * m->Hkv_l) * m->c.head_dim;
-      const bool fused = fuses_rope(m, kv->B, plan_splits(m, kv->B, nqkv, m->c.d_model));
+      const bool fused = fuses_rope(m, kv->B, chained_step(m, kv->B) ? 1 : plan_splits(m, kv->B, nqkv, m->c.d_model));
       const int chunk = sb_attn_decode_chunk(ctx, kv->B, m->Hkv_l, kv->maxlen, std::min(kv->maxlen, longest + 128), fused);
       if (chunk != kv->chunk) {
         kv->chunk = chunk;
