@@ -216,6 +216,7 @@ int strictb200_destroy(strictb200_ctx* ctx) {
   if (ctx->gemm_ws) cudaFree(ctx->gemm_ws);
   if (ctx->ws2) cudaFree(ctx->ws2);
   if (ctx->prefill_ws) cudaFree(ctx->prefill_ws);
+  if (ctx->planes) cudaFree(ctx->planes);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);

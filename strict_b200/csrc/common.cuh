@@ -111,6 +111,9 @@ struct strictb200_ctx {
   // scratch of the prefill chunks (activations of up to opt.prefill_chunk token rows), grow-only
   void* prefill_ws = nullptr;
   size_t prefill_ws_bytes = 0;
+  // bf16 planes of the operands of a large fp32 product (gemm_f32_pair.cu), grow-only and bounded
+  void* planes = nullptr;
+  size_t planes_bytes = 0;
   uint64_t ws_generation = 0;  // advanced whenever a scratch buffer is re-allocated (recorded sequences check it)
 };
 

@@ -7,7 +7,8 @@
 // Rows of X, W and Y may be wider than the product (ldx, ldw, ldy).
 #include "common.cuh"
 
-int k_gemm_f32_tc(strictb200_ctx* ctx, const GemmF32Args& g);  // gemm_f32_tc.cu
+int k_gemm_f32_tc(strictb200_ctx* ctx, const GemmF32Args& g);    // gemm_f32_tc.cu
+int k_gemm_f32_pair(strictb200_ctx* ctx, const GemmF32Args& g);  // gemm_f32_pair.cu
 
 namespace {
 constexpr int F32_MT = 8;
@@ -47,8 +48,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
                                                        int prefetch) {
   extern __shared__ __align__(16) float xs[];
   __shared__ float part[8][MT * NC];
-  pdl_trigger();
   SB_TRACE_BEGIN();
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = 8 / ks, slice = warp % ks;
   const int n0 = (blockIdx.x * groups + warp / ks) * NC;
@@ -75,8 +76,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
   const int oc = n0 + lane;  // lanes that will finish a channel
   const float bn = bias && lane < NC && oc < N ? bias[oc] : 0.f;
   pdl_wait();
-  if (LN) {
   SB_TRACE_WAITED();
+  if (LN) {
     if (warp < mt) {  // a warp per row
       const float4* xr = (const float4*)(x + (int64_t)(m0 + warp) * ldx);
       float4 v[F32_PRE];
@@ -107,8 +108,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
     for (int i = threadIdx.x; i < mt * nk4; i += 256) ((float4*)xs)[i] = __ldcg((const float4*)(x + (int64_t)(m0 + i / nk4) * ldx) + i % nk4);
     __syncthreads();
   }
-  float acc[NC * MT];
   SB_TRACE_MARK(0);
+  float acc[NC * MT];
 #pragma unroll
   for (int i = 0; i < NC * MT; i++) acc[i] = 0.f;
   auto fma_rows = [&](int k4, const float4* wv) {
@@ -136,8 +137,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
     for (int c = 0; c < NC; c++) wv[c] = n0 + c < N ? __ldcs((const float4*)(w + (int64_t)(n0 + c) * ldw) + k4) : make_float4(0.f, 0.f, 0.f, 0.f);
     fma_rows(k4, wv);
   }
-  constexpr int VALS = NC * MT, STEP = 32 / VALS;
   SB_TRACE_MARK(1);
+  constexpr int VALS = NC * MT, STEP = 32 / VALS;
   const float sum = fold_sums<VALS>(acc, lane);
   if (lane % STEP == 0) part[warp][lane / STEP] = sum;
   __syncthreads();
@@ -151,8 +152,8 @@ __global__ void __launch_bounds__(256, 2) gemm_f32_kernel(int M, int N, int K, c
       else y[o] = accumulate == 1 ? y[o] + v : accumulate == 2 ? sb_gelu_tanh(v) : accumulate == 3 ? sb_xielu(v, act_pos, act_neg) : v;
     }
   }
-}
   SB_TRACE_END(SB_K_GEMM, (uint32_t)N ^ ((uint32_t)K << 12));
+}
 
 template <int MT, int NC, bool STAGED, bool LN>
 int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
@@ -180,9 +181,9 @@ int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks, bool two) {
 }
 }  // namespace
 
-bool sb_gemm_f32_takes_norm(int64_t M, int64_t K) { return M <= F32_MT && K <= LN_K; }
 SB_TRACE_TU(gemm_f32)
 
+bool sb_gemm_f32_takes_norm(int64_t M, int64_t K) { return M <= F32_MT && K <= LN_K; }
 
 int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float* x, const float* w, const float* bias, float* y,
                int accumulate) {
@@ -203,7 +204,10 @@ int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   // Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336): 9.2e-8 / 1.0e-7 / 1.6e-7 here, 7.6e-8..8.7e-8 /
   // 9.6e-8 / 1.3e-7 there.
   const bool few = M <= 4 || (M <= F32_MT && (g.ln_gain || N * K <= (8 << 20))) || (M <= 2 * F32_MT && N * K <= (1 << 20));
-  if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) return k_gemm_f32_tc(ctx, g);
+  if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) {
+    const int st = k_gemm_f32_pair(ctx, g);
+    return st == STRICTB200_ERR_UNSUPPORTED ? k_gemm_f32_tc(ctx, g) : st;
+  }
   // Warps per output channel: slices of at most 1024 columns, and two for a long enough row, while all blocks are resident at once (two
   // per SM with the norm in front or several rows, else four); two channels per warp where they would not be. With the norm in front
   // 3072 channels of 768 columns took 6.6 us as 384 blocks of two waves, 3.0 us as 192.

@@ -25,7 +25,7 @@
 //   warps 9..16   running sums: half of the token columns each, thread = channel
 // A result that is not finite is computed again as a plain fp32 sum (an infinity has no bf16 remainder), so infinities, NaN and
 // overflow come out as they do from the row kernel. Every mbarrier wait is bounded and reports through the context's error word.
-#include "tcgen05.cuh"
+#include "gemm_f32_terms.cuh"
 
 namespace {
 using namespace tc;
@@ -55,14 +55,6 @@ __device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-// Two values -> their bf16 terms, packed (the first value in the low half); u and v become 2^8 times the remainders.
-__device__ __forceinline__ uint32_t take_term(float& u, float& v) {
-  uint32_t t;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t) : "f"(v), "f"(u));
-  u = __fmul_rn(256.f, __fsub_rn(u, __uint_as_float(t << 16)));
-  v = __fmul_rn(256.f, __fsub_rn(v, __uint_as_float(t & 0xFFFF0000u)));
-  return t;
-}
 // Eight columns of one row into the three planes at this shared-memory address.
 __device__ __forceinline__ void store_terms(uint32_t addr, uint32_t plane_bytes, float4 a, float4 b) {
 #pragma unroll
@@ -71,23 +63,18 @@ __device__ __forceinline__ void store_terms(uint32_t addr, uint32_t plane_bytes,
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr + p * plane_bytes), "r"(t0), "r"(t1), "r"(t2), "r"(t3) : "memory");
   }
 }
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; k++) s = fmaf(x[k], w[k], s);
-  return s;
-}
 __device__ __forceinline__ void finish(const GemmF32Args& g, int tok, int n, float v) {
   if (tok >= g.M || n >= g.N) return;
-  if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot(g.x + (int64_t)tok * g.ldx, g.w + (int64_t)n * g.ldw, (int)g.K);
-  if (g.bias) v += g.bias[n];
   float* y = g.y + (int64_t)tok * g.ldy + n;
-  if (g.mode == 4) *y += g.alpha * (g.col_scale ? g.col_scale[n] : 1.f) * v;
-  else *y = g.mode == 1 ? *y + v : g.mode == 2 ? sb_gelu_tanh(v) : g.mode == 3 ? sb_xielu(v, g.act_pos, g.act_neg) : v;
+  if (not_finite(v)) v = plain_dot(g.x + (int64_t)tok * g.ldx, g.w + (int64_t)n * g.ldw, (int)g.K);
+  if (g.bias) v += g.bias[n];
+  switch (g.mode) {
+    case 1: *y = finished<1>(g, 1.f, v, *y); break;
+    case 2: *y = finished<2>(g, 1.f, v, 0.f); break;
+    case 3: *y = finished<3>(g, 1.f, v, 0.f); break;
+    case 4: *y = finished<4>(g, g.alpha * (g.col_scale ? g.col_scale[n] : 1.f), v, *y); break;
+    default: *y = v;
+  }
 }
 
 template <int BT>
