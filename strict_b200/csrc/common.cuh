@@ -316,9 +316,6 @@ bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished)
 int sb_gemm_rows_splits(strictb200_ctx*, int64_t N, int64_t K, bool f8);
 int k_gemm_rows_glu(strictb200_ctx*, const GemmArgs& g, float* ones);
 int k_gemm_rows_fp8_bf16(strictb200_ctx*, const GemmArgs& g);
-int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
-// gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
-// Where a finished value goes. Columns from n_switch on (0 = none) belong to a second product of the same launch: its
 // gemm_rows_chain.cu: the same rows, the norm of the residual in front of a product, and a product added to the residual
 struct NormRowsGemm {
   int64_t M = 0, N = 0, K = 0;  // out [M,N] = norm(x) . w^T, x [M,K] fp32, rounded to bf16 after the norm; w [N,K] E4M3
@@ -341,6 +338,9 @@ struct ResidualRowsGemm {
 };
 bool sb_residual_rows_takes(int64_t M, int64_t N, int64_t K);
 int k_residual_rows(strictb200_ctx*, const ResidualRowsGemm& g);
+int sb_pick_splits_kb(strictb200_ctx*, int64_t M, int64_t N, int64_t nkb);  // the same rule for nkb K blocks of 128 bytes
+// gemm_bf16.cu: Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands on the kernels of the E4M3 path (tcgen05 kind::f16), fp32 accumulation.
+// Where a finished value goes. Columns from n_switch on (0 = none) belong to a second product of the same launch: its
 // operand rows are x_row_off + m, and with act_out set the value leaves through the activation.
 struct Bf16Epilogue {
   float* out_f32 = nullptr;   // [M, ldo]

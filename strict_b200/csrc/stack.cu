@@ -342,6 +342,20 @@ int norm_rows(strictb200_model* m, const StackLayer* w, int64_t M, float* x, con
   return k_group_norm(m->ctx, a, M, m->c.d_model);
 }
 
+// ... where no norm follows: into the residual
+int add_pending(strictb200_model* m, int64_t M, float* x, const Pending& p) {
+  const SbStack& st = *m->stack;
+  if (!p.from) return STRICTB200_OK;
+  GroupNormArgs a;
+  a.x = x; a.ldx = st.dp; a.part = p.part; a.ldp = m->c.d_model; a.splits = p.splits; a.splits0 = p.splits0; a.mult = st.mult;
+  a.scale0 = p.from->ls1; a.scale1 = p.from->ls2;
+  return k_group_norm(m->ctx, a, M, m->c.d_model);
+}
+// Rows of a prompt chunk whose output products leave their sums to the next norm, as a decode step's do: finished, the few channel tiles of so
+// few rows would each come through one SM's path to memory. Whole prefills of 12 / 37 / 100 tokens, us: 28 layers of latent attention 1648 / 1769 / 1958 ->
+// 1039 / 1242 / 1434, recurrent, retention and attention layers 1778 / 1917 / 2152 -> 1129 / 1271 / 1433.
+bool few_prompt_rows(const SbStack& st, int64_t T) { return !st.f32 && T <= 128; }
+
 int embed_rows(strictb200_model* m, const int32_t* ids, int64_t M, float* x) {
   SbStack& st = *m->stack;
   if (st.f32) return k_embedding_f32(m->ctx, (const float*)st.embed, nullptr, ids, nullptr, nullptr, M, st.dp, m->c.vocab, 0, x);
@@ -548,6 +562,7 @@ struct StackPre {
   float* x;
   char* h;
   float* in;
+  float* part2;    // sums of the output product (few_prompt_rows)
   char *q, *oa, *mix;
   bf16 *kvx, *lat;
   int32_t* keys;   // [layers][2][nb]: row and position of every sequence's first key
@@ -566,9 +581,14 @@ int64_t key_rows(const StackLayer& w, const PrefillChunk& c) {
 void carve_pre(strictb200_model* m, const PrefillChunk& c, char* base, StackPre* o, size_t* total) {
   SbStack& st = *m->stack;
   const int64_t T = c.T;
-  size_t in = 1, q = 1, oa = 1, kvx = 1, lat = 1, mix = 1;
+  size_t in = 1, part2 = 1, q = 1, oa = 1, kvx = 1, lat = 1, mix = 1;
   for (const StackLayer& w : st.L) {
     in = std::max(in, (size_t)T * ld_in_of(st, w));
+    if (few_prompt_rows(st, T)) {
+      int first, all;
+      out_splits(m->ctx, st, w, T, m->c.d_model, &first, &all);
+      part2 = std::max(part2, (size_t)all * T * m->c.d_model);
+    }
     oa = std::max(oa, (size_t)T * w.ldo);
     if (w.kind != STRICTB200_MIXER_LATENT) {
       MixBufs t;
@@ -588,6 +608,7 @@ void carve_pre(strictb200_model* m, const PrefillChunk& c, char* base, StackPre*
   o->x = cv.take<float>(T * st.dp);
   o->h = cv.take<char>(2 * T * st.dp * st.esz());
   o->in = cv.take<float>(in);
+  o->part2 = cv.take<float>(part2);
   o->q = cv.take<char>(q * st.esz());
   o->oa = cv.take<char>(oa * st.esz());
   o->kvx = cv.take<bf16>(kvx);
@@ -762,15 +783,18 @@ int sb_stack_prefill_chunk(strictb200_model* m, strictb200_kv* kv, const Prefill
   MixRows rows;
   rows.T = T; rows.b0 = c.b0; rows.nb = c.nb; rows.max_new = c.max_new; rows.seq = c.ix.seq; rows.pos = c.ix.pos; rows.qstart = c.ix.qs; rows.past = c.ix.past;
   rows.lens = c.ix.la;
+  Pending pend;
   for (int l = 0; l < (int)st.L.size(); l++) {
     const StackLayer& w = st.L[l];
     const LatentShape& s = w.s;
     const int64_t ld_in = ld_in_of(st, w);
-    SB_TRY(norm_rows(m, &w, T, b.x, Pending(), b.h));
+    SB_TRY(norm_rows(m, &w, T, b.x, pend, b.h));
+    pend = Pending();
+    auto add_out = [&] { return few_prompt_rows(st, T) ? out_parts(m, w, T, b.oa, b.part2, &pend) : project_out(m, w, T, b.oa, b.x); };
     SB_TRY(project_in(m, w, T, b.h, b.in, ld_in, b.oa));
     if (w.kind != STRICTB200_MIXER_LATENT) {
       SB_TRY(mix_rows(m, kv, l, rows, ProjRows{b.in, ld_in, 1}, ActArgs(), b.mix, b.oa));
-      SB_TRY(project_out(m, w, T, b.oa, b.x));
+      SB_TRY(add_out());
       continue;
     }
     LatentSplitArgs a = split_args(m, kv, l, c.b0);
@@ -802,8 +826,9 @@ int sb_stack_prefill_chunk(strictb200_model* m, strictb200_kv* kv, const Prefill
       p.out = (bf16*)b.oa; p.ldo = w.ldo;
       SB_TRY(k_attn_prefill_latent(ctx, p));
     }
-    SB_TRY(project_out(m, w, T, b.oa, b.x));
+    SB_TRY(add_out());
   }
+  SB_TRY(add_pending(m, T, b.x, pend));
   SB_TRY(k_gather_rows(ctx, b.x, c.ix.last, c.n_rows, st.dp * 4, b.last));
   SB_TRY(norm_rows(m, nullptr, c.n_rows, b.last, Pending(), b.lasth));
   SB_TRY(head_rows(m, c.n_rows, b.lasth, b.logits));
