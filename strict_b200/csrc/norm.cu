@@ -921,13 +921,16 @@ __global__ void __launch_bounds__(NI == 1 ? 1024 : 512) group_norm_kernel(GroupN
   const int64_t row = blockIdx.x;
   const int n = a.gw / a.cb, c0 = (int)blockIdx.y / a.cb * a.gw + (int)blockIdx.y % a.cb * n;
   pdl_trigger();
-  float4 g1[NI], g2[NI], v[NI];
+  float4 g1[NI], g2[NI], v[NI], sc0[NI], sc1[NI];
 #pragma unroll
   for (int i = 0; i < NI; i++) {
     const int k = (i * (int)blockDim.x + (int)threadIdx.x) * 4;
-    if (k < n && a.g1) {
-      g1[i] = *(const float4*)(a.g1 + c0 + k);
+    sc0[i] = sc1[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (k < n) {
+      if (a.g1) g1[i] = *(const float4*)(a.g1 + c0 + k);
       if (a.g2) g2[i] = *(const float4*)(a.g2 + c0 + k);
+      if (a.scale0) sc0[i] = *(const float4*)(a.scale0 + c0 + k);
+      if (a.scale1) sc1[i] = *(const float4*)(a.scale1 + c0 + k);
     }
   }
   pdl_wait();
@@ -950,9 +953,11 @@ __global__ void __launch_bounds__(NI == 1 ? 1024 : 512) group_norm_kernel(GroupN
             float4& o = s < a.splits0 ? t : u;
             o.x += p[s].x; o.y += p[s].y; o.z += p[s].z; o.w += p[s].w;
           }
-        if (a.scale0) { const float4 c = *(const float4*)(a.scale0 + c0 + k); t.x *= c.x; t.y *= c.y; t.z *= c.z; t.w *= c.w; }
-        if (a.scale1) { const float4 c = *(const float4*)(a.scale1 + c0 + k); u.x *= c.x; u.y *= c.y; u.z *= c.z; u.w *= c.w; }
-        x.x = fmaf(a.mult, t.x + u.x, x.x); x.y = fmaf(a.mult, t.y + u.y, x.y); x.z = fmaf(a.mult, t.z + u.z, x.z); x.w = fmaf(a.mult, t.w + u.w, x.w);
+        const float4 c = sc0[i], e = sc1[i];
+        t = make_float4(__fmul_rn(t.x, c.x), __fmul_rn(t.y, c.y), __fmul_rn(t.z, c.z), __fmul_rn(t.w, c.w));
+        u = make_float4(__fmul_rn(u.x, e.x), __fmul_rn(u.y, e.y), __fmul_rn(u.z, e.z), __fmul_rn(u.w, e.w));
+        x.x = fmaf(a.mult, __fadd_rn(t.x, u.x), x.x); x.y = fmaf(a.mult, __fadd_rn(t.y, u.y), x.y);
+        x.z = fmaf(a.mult, __fadd_rn(t.z, u.z), x.z); x.w = fmaf(a.mult, __fadd_rn(t.w, u.w), x.w);
         *(float4*)xp = x;
       }
       v[i] = x;
