@@ -133,12 +133,9 @@ int sb_trace_set_heads(const SbTraceDev&);
 int sb_trace_set_recurrent(const SbTraceDev&);
 int sb_trace_set_gemm_rows(const SbTraceDev&);
 int sb_trace_set_gemm_rows_chain(const SbTraceDev&);
-int sb_trace_set_gemm_f32(const SbTraceDev&);
-int sb_trace_set_attention_f32(const SbTraceDev&);
 static int trace_set_all(const SbTraceDev& t) {
   return sb_trace_set_gemm_split(t) | sb_trace_set_norm(t) | sb_trace_set_rope(t) | sb_trace_set_attention(t) | sb_trace_set_latent(t) |
-         sb_trace_set_heads(t) | sb_trace_set_recurrent(t) | sb_trace_set_gemm_rows(t) | sb_trace_set_gemm_rows_chain(t) | sb_trace_set_gemm_f32(t) |
-         sb_trace_set_attention_f32(t);
+         sb_trace_set_heads(t) | sb_trace_set_recurrent(t) | sb_trace_set_gemm_rows(t) | sb_trace_set_gemm_rows_chain(t);
 }
 
 extern "C" {

@@ -254,24 +254,42 @@ __global__ void __launch_bounds__(256) attn_f32_prompt_kernel(const float* qkv, 
 // One block per row and head, and it appends the row's key and value to the cache. LANES lanes share a key (one 128-bit load of the
 // key and one of the value per lane), each such group walks every GROUPS-th key with a running maximum and its own sum, eight keys'
 // loads in flight; the groups meet in shared memory. Bound by the latency of those loads: 144 keys on average took 13.6 us of a GPT-2 step
-// with a key per thread and a second pass for the values, 3.7 us here.
+// with a key per thread and a second pass for the values, 3.7 us with batches behind the dependency wait. The first batch (rows of earlier steps) is
+// requested in front of it; the length it is derived from is read again after the wait, and the batch with it if it changed.
 template <int LANES>
 __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, float* kc, float* vc, const int32_t* lens, int H,
-                                                              int maxlen, float scale, float* out) {
+                                                              int maxlen, float scale, float* out, int prefetch) {
   constexpr int D = 4 * LANES, GROUPS = 512 / LANES, BATCH = 8;
   __shared__ float red_m[GROUPS], red_l[GROUPS];
   __shared__ __align__(16) float red_o[GROUPS][D];
-  SB_TRACE_BEGIN();
   pdl_trigger();
   const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x % LANES, grp = threadIdx.x / LANES, hd = H * D;
   float* kb = kc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
   float* vb = vc + ((int64_t)b * H + h) * maxlen * D + 4 * c;
+  float4 k[BATCH], v[BATCH];
+  auto load = [&](int base, int len) {
+#pragma unroll
+    for (int i = 0; i < BATCH; i++) {
+      const int j = base + grp + i * GROUPS;
+      if (j < len) {
+        k[i] = *(const float4*)(kb + (int64_t)j * D);
+        v[i] = *(const float4*)(vb + (int64_t)j * D);
+      }
+    }
+  };
+  auto ld_len = [&] {
+    int n;
+    asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(n) : "l"(lens + b) : "memory");
+    return n;
+  };
+  const int early = prefetch ? min(ld_len(), maxlen) : -1;
+  load(0, early);
   pdl_wait();
-  SB_TRACE_WAITED();
-  const int p = lens[b];
-  if (p < 0 || p >= maxlen) return;
   const float* row = qkv + (int64_t)b * 3 * hd + h * D + 4 * c;
   const float4 q = *(const float4*)row, k_own = *(const float4*)(row + hd), v_own = *(const float4*)(row + 2 * hd);
+  const int p = ld_len();
+  if (p < 0 || p >= maxlen) return;
+  if (p != early) load(0, p);
   if (grp == 0) {
     *(float4*)(kb + (int64_t)p * D) = k_own;
     *(float4*)(vb + (int64_t)p * D) = v_own;
@@ -280,18 +298,10 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int base = 0; base <= p; base += BATCH * GROUPS) {  // the same number of rounds for every group: their lanes share warps, and shuffles
     const int j0 = base + grp;
-    float4 k[BATCH], v[BATCH];
+    if (base) load(base, p);
 #pragma unroll
-    for (int i = 0; i < BATCH; i++) {
-      const int j = j0 + i * GROUPS;
-      if (j < p) {
-        k[i] = *(const float4*)(kb + (int64_t)j * D);
-        v[i] = *(const float4*)(vb + (int64_t)j * D);
-      } else {
-        k[i] = k_own;
-        v[i] = v_own;
-      }
-    }
+    for (int i = 0; i < BATCH; i++)
+      if (j0 + i * GROUPS >= p) { k[i] = k_own; v[i] = v_own; }
     float s[BATCH], mx = m;
 #pragma unroll
     for (int i = 0; i < BATCH; i++) {
@@ -315,7 +325,6 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
       }
     }
   }
-  SB_TRACE_MARK(0);
   if (c == 0) { red_m[grp] = m; red_l[grp] = l; }
   *(float4*)&red_o[grp][4 * c] = o;
   __syncthreads();
@@ -331,11 +340,8 @@ __global__ void __launch_bounds__(512) attn_f32_decode_kernel(const float* qkv, 
     }
     out[(int64_t)b * hd + h * D + threadIdx.x] = acc * (1.0f / sum);
   }
-  SB_TRACE_END(SB_K_ATTN, 0);
 }
 }  // namespace
-
-SB_TRACE_TU(attention_f32)
 
 int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, const int32_t* seq, const int32_t* pos, const int32_t* lens,
                int64_t T, int H, int Dh, int maxlen, float scale, float* out, const F32Prompts* prompts) {
@@ -343,7 +349,7 @@ int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, cons
   const bool rows16 = (((uintptr_t)qkv | (uintptr_t)kc | (uintptr_t)vc | (uintptr_t)out) & 15) == 0;
   if (!seq && rows16 && (Dh == 32 || Dh == 64 || Dh == 128) && T <= 65535) {  // rows that are sequences of their own
     auto kernel = Dh == 32 ? attn_f32_decode_kernel<8> : Dh == 64 ? attn_f32_decode_kernel<16> : attn_f32_decode_kernel<32>;
-    SB_CUDA(sb_launch(ctx, kernel, dim3((unsigned)H, (unsigned)T), dim3(512), 0, qkv, kc, vc, lens, H, maxlen, scale, out));
+    SB_CUDA(sb_launch(ctx, kernel, dim3((unsigned)H, (unsigned)T), dim3(512), 0, qkv, kc, vc, lens, H, maxlen, scale, out, ctx->opt.attn_prefetch));
     ctx->launches++;
     return STRICTB200_OK;
   }
