@@ -639,46 +639,57 @@ void sb_tp_abort(strictb200_ctx*);       // ncclCommAbort: stops the communicato
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t f32_to_bf16_bits(float f);
 // Sixteen tokens m0.. of one output channel n per lane (channels of a warp are consecutive, the first one even, all on the
-// same side of n_switch). bf16 rows: neighbouring lanes trade tokens so that each stores two channels at a time.
-__device__ __forceinline__ void sb_bf16_store16(const Bf16Epilogue& e, int M, int N, int m0, int n, const uint32_t* r) {
+// same side of n_switch), one function per kind of output, so that a loop over tokens holds the code of one kind only.
+enum { SB_OUT_F32 = 0, SB_OUT_BF16 = 1, SB_OUT_GLU = 2 };
+__device__ __forceinline__ int sb_bf16_out_kind(const Bf16Epilogue& e, int n) {
   const bool act = e.act_out && n >= e.n_switch;
-  if (act && e.glu) {
-    // The lanes of a pair hold the gate and the up value of one channel. Each takes eight tokens, then the lanes of two
-    // neighbouring channels trade so that each stores both channels of four tokens.
-    const int odd = n & 1, second = (n >> 1) & 1, j = (n - e.n_switch) >> 1, nf = (N - e.n_switch) >> 1;
-    float p[8];
+  return act && e.glu ? SB_OUT_GLU : !act && e.out_f32 ? SB_OUT_F32 : SB_OUT_BF16;
+}
+// Gated activation: the lanes of a pair hold the gate and the up value of one channel. Each takes eight tokens, then the lanes of two
+// neighbouring channels trade so that each stores both channels of four tokens.
+__device__ __forceinline__ void sb_bf16_store16_glu(const Bf16Epilogue& e, int M, int N, int m0, int n, const uint32_t* r) {
+  const int odd = n & 1, second = (n >> 1) & 1, j = (n - e.n_switch) >> 1, nf = (N - e.n_switch) >> 1;
+  float p[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const float got = __uint_as_float(__shfl_xor_sync(0xffffffffu, odd ? r[i] : r[8 + i], 1));
-      const float gate = odd ? got : __uint_as_float(r[i]), up = odd ? __uint_as_float(r[8 + i]) : got;
-      p[i] = fmaxf(gate, 0.f) * up;
-    }
-    bf16* o = e.act_out + (int64_t)(m0 + odd * 8 + second * 4) * e.ld_act + (j - second);
-#pragma unroll
-    for (int i = 0; i < 4; i++, o += e.ld_act) {
-      const float got = __shfl_xor_sync(0xffffffffu, second ? p[i] : p[4 + i], 2);
-      const float lo = second ? got : p[i], hi = second ? p[4 + i] : got;
-      if (m0 + odd * 8 + second * 4 + i < M && j - second < nf) {
-        if (j - second + 1 < nf) *(uint32_t*)o = f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
-        else *o = __float2bfloat16_rn(lo);
-      }
-    }
-    return;
+  for (int i = 0; i < 8; i++) {
+    const float got = __uint_as_float(__shfl_xor_sync(0xffffffffu, odd ? r[i] : r[8 + i], 1));
+    const float gate = odd ? got : __uint_as_float(r[i]), up = odd ? __uint_as_float(r[8 + i]) : got;
+    p[i] = fmaxf(gate, 0.f) * up;
   }
-  if (!act && e.out_f32) {
-    if (n >= N) return;
-    const float cs = e.col_scale ? e.alpha * e.col_scale[n] : e.alpha;
-    float* o = e.out_f32 + (int64_t)m0 * e.ldo + n;
-    float old[16];  // all read before the first store, so that the sixteen reads overlap
-    if (e.accumulate) {
+  bf16* o = e.act_out + (int64_t)(m0 + odd * 8 + second * 4) * e.ld_act + (j - second);
 #pragma unroll
-      for (int j = 0; j < 16; j++) old[j] = m0 + j < M ? o[j * e.ldo] : 0.f;
+  for (int i = 0; i < 4; i++, o += e.ld_act) {
+    const float got = __shfl_xor_sync(0xffffffffu, second ? p[i] : p[4 + i], 2);
+    const float lo = second ? got : p[i], hi = second ? p[4 + i] : got;
+    if (m0 + odd * 8 + second * 4 + i < M && j - second < nf) {
+      if (j - second + 1 < nf) *(uint32_t*)o = f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
+      else *o = __float2bfloat16_rn(lo);
     }
+  }
+}
+// fp32 rows; old: what is there (accumulate), read by sb_f32_read16 well before, so that the reads overlap
+__device__ __forceinline__ void sb_f32_read16(const Bf16Epilogue& e, int M, int N, int m0, int n, float* old) {
+  const float* o = e.out_f32 + (int64_t)m0 * e.ldo + n;
+#pragma unroll
+  for (int j = 0; j < 16; j++, o += e.ldo) old[j] = n < N && m0 + j < M ? *o : 0.f;
+}
+__device__ __forceinline__ void sb_f32_store16(const Bf16Epilogue& e, int M, int N, int m0, int n, const uint32_t* r, const float* old, float cs) {
+  if (n >= N) return;
+  float* o = e.out_f32 + (int64_t)m0 * e.ldo + n;
+  if (old) {
 #pragma unroll
     for (int j = 0; j < 16; j++, o += e.ldo)
-      if (m0 + j < M) *o = e.accumulate ? fmaf(cs, __uint_as_float(r[j]), old[j]) : __uint_as_float(r[j]);
-    return;
+      if (m0 + j < M) *o = fmaf(cs, __uint_as_float(r[j]), old[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; j++, o += e.ldo)
+      if (m0 + j < M) *o = __uint_as_float(r[j]);
   }
+}
+__device__ __forceinline__ float sb_f32_scale(const Bf16Epilogue& e, int N, int n) { return e.col_scale && n < N ? e.alpha * e.col_scale[n] : e.alpha; }
+// bf16 rows, through xIELU where they are a feed-forward's: neighbouring lanes trade tokens so that each stores two channels at a time
+__device__ __forceinline__ void sb_bf16_store16_rows(const Bf16Epilogue& e, int M, int N, int m0, int n, const uint32_t* r) {
+  const bool act = e.act_out && n >= e.n_switch;
   const int64_t ld = act ? e.ld_act : e.ldo;
   bf16* o = act ? e.act_out + (n - e.n_switch) : e.out_bf16 + n;
   float v[16];
@@ -703,6 +714,14 @@ __device__ __forceinline__ void sb_bf16_store16(const Bf16Epilogue& e, int M, in
     for (int j = 0; j < 16; j++, o += ld)
       if (m0 + j < M) *o = __float2bfloat16_rn(v[j]);
   }
+}
+__device__ __forceinline__ void sb_bf16_store16(const Bf16Epilogue& e, int M, int N, int m0, int n, const uint32_t* r) {
+  const int kind = sb_bf16_out_kind(e, n);
+  if (kind == SB_OUT_GLU) return sb_bf16_store16_glu(e, M, N, m0, n, r);
+  if (kind == SB_OUT_BF16) return sb_bf16_store16_rows(e, M, N, m0, n, r);
+  float old[16];  // all read before the first store, so that the sixteen reads overlap
+  if (e.accumulate) sb_f32_read16(e, M, N, m0, n, old);
+  sb_f32_store16(e, M, N, m0, n, r, e.accumulate ? old : nullptr, sb_f32_scale(e, N, n));
 }
 // Programmatic dependent launch. A kernel launched through sb_launch may begin while its
 // predecessor in the stream is still running: pdl_trigger() lets the successor start launching,

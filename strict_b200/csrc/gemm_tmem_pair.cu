@@ -294,6 +294,12 @@ __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constan
     for (int seg = 0; seg < my_tiles; seg++) {
       int tn, tt;
       tile_at(a, c + seg * pairs, tn, tt);
+      float sx0 = 0.f, sx1 = 0.f;  // scales of the warp's 64 tokens, two per lane
+      if constexpr (!BF16) {
+        const int tok = tt * BTH + half * (HALF / 2) + lane;
+        if (tok < a.M) sx0 = a.sx[tok];
+        if (tok + 32 < a.M) sx1 = a.sx[tok + 32];
+      }
       bool bad = !mbar_wait(smem_u32(&bar_acc_full[seg & 1]), (seg >> 1) & 1);
       if (bad && lane == 0) set_status(a.status, 3);
       if (epi_any(bad)) break;
@@ -303,53 +309,106 @@ __global__ void __launch_bounds__(THREADS) gemm_pair_kernel(const __grid_constan
       const int n = GLU ? tn * BN + (int)rank * (BN / 2) + lg * 16 + (lane & 15) : tn * 2 * BN + (int)rank * BN + ch;
       const int n_end = GLU ? a.N / 2 : a.N;
       const float swn = !BF16 && n < n_end ? a.sw[GLU && lane >= 16 ? n_end + n : n] : 0.f;
+      // 32 operand rows at a time. One loop per kind of output, each with little code, and nothing inside it waits for memory: with the scales of
+      // the tokens loaded one by one between the stores (which might have been to the same place) a tile's epilogue took 8.4 us, four times the products
+      // of a tile of K = 1024, and the last one of every launch is not overlapped. Figures at k_gemm_fp8_tmem_pair.
+      auto each = [&](auto&& before, auto&& store) {
 #pragma unroll 1
-      for (int grp = 0; grp < HALF / 16; grp += 2) {  // 32 operand rows at a time
-        uint32_t r[32];
-        tc_ld16(acc + (uint32_t)(grp * 16), r);
-        tc_ld16(acc + (uint32_t)(grp * 16 + 16), r + 16);
-        tc_wait_ld16(r);
-        tc_wait_ld16(r + 16);
-        if constexpr (BF16) {
-          const int tok = tt * 2 * BTH + half * HALF + grp * 16;
-          sb_bf16_store16(a.e, a.M, a.N, tok, n, r);
-          sb_bf16_store16(a.e, a.M, a.N, tok + 16, n, r + 16);
+        for (int grp = 0; grp < HALF / 16; grp += 2) {
+          uint32_t r[32];
+          before(grp);
+          tc_ld16(acc + (uint32_t)(grp * 16), r);
+          tc_ld16(acc + (uint32_t)(grp * 16 + 16), r + 16);
+          tc_wait_ld16(r);
+          tc_wait_ld16(r + 16);
+          store(grp, r);
+        }
+      };
+      auto nothing = [](int) {};
+      if constexpr (BF16) {
+        const int tok = tt * 2 * BTH + half * HALF;
+        const int kind = sb_bf16_out_kind(a.e, n);  // the same for the whole tile
+        if (kind == SB_OUT_GLU) {
+          each(nothing, [&](int grp, const uint32_t* r) {
+            sb_bf16_store16_glu(a.e, a.M, a.N, tok + grp * 16, n, r);
+            sb_bf16_store16_glu(a.e, a.M, a.N, tok + grp * 16 + 16, n, r + 16);
+          });
+        } else if (kind == SB_OUT_BF16) {
+          each(nothing, [&](int grp, const uint32_t* r) {
+            sb_bf16_store16_rows(a.e, a.M, a.N, tok + grp * 16, n, r);
+            sb_bf16_store16_rows(a.e, a.M, a.N, tok + grp * 16 + 16, n, r + 16);
+          });
+        } else if (a.e.accumulate) {
+          float old[32];
+          const float cs = sb_f32_scale(a.e, a.N, n);
+          each(
+              [&](int grp) {
+                sb_f32_read16(a.e, a.M, a.N, tok + grp * 16, n, old);
+                sb_f32_read16(a.e, a.M, a.N, tok + grp * 16 + 16, n, old + 16);
+              },
+              [&](int grp, const uint32_t* r) {
+                sb_f32_store16(a.e, a.M, a.N, tok + grp * 16, n, r, old, cs);
+                sb_f32_store16(a.e, a.M, a.N, tok + grp * 16 + 16, n, r + 16, old + 16, cs);
+              });
         } else {
-          const int tok0 = tt * BTH + half * (HALF / 2) + grp * 8;  // operand rows 16g.. hold tokens 8g..
-          if constexpr (GLU) {
-            const bool up = lane >= 16;
-            float y[16];
+          each(nothing, [&](int grp, const uint32_t* r) {
+            sb_f32_store16(a.e, a.M, a.N, tok + grp * 16, n, r, nullptr, 1.f);
+            sb_f32_store16(a.e, a.M, a.N, tok + grp * 16 + 16, n, r + 16, nullptr, 1.f);
+          });
+        }
+      } else {
+        const int tok = tt * BTH + half * (HALF / 2);  // operand rows 16 g.. hold tokens 8 g..
+        // finished values of the sixteen tokens of 32 operand rows
+        auto values = [&](int grp, const uint32_t* r, float* y) {
+          const float s = grp < 4 ? sx0 : sx1;
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-              const int k = (j & 8) * 2 + (j & 7);
-              const float v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
-              y[j] = __fmul_rn(__fmul_rn(v, tok0 + j < a.M ? a.sx[tok0 + j] : 0.f), swn);
+          for (int j = 0; j < 16; j++) {
+            const int k = (j & 8) * 2 + (j & 7);
+            float v;
+            if constexpr (I8) {
+              const int hi = (int)r[k], lo = (int)r[k + 8];
+              // 128 * hi + lo stays below 2^31 up to here (lo <= 64 * 127 * K <= 2^30); larger sums in 64 bits
+              v = abs(hi) < (1 << 23) ? __int2float_rn(hi * 128 + lo) : __ll2float_rn((int64_t)hi * 128 + (int64_t)lo);
+            } else {
+              v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
             }
-            bf16* o = (bf16*)a.out + (int64_t)(tok0 + (up ? 8 : 0)) * n_end + n;
+            y[j] = __fmul_rn(__fmul_rn(v, __shfl_sync(0xffffffffu, s, (grp & 3) * 8 + j)), swn);
+          }
+        };
+        if constexpr (GLU) {
+          const bool up = lane >= 16;
+          each(nothing, [&](int grp, const uint32_t* r) {
+            float y[16];
+            values(grp, r, y);
+            const int t0 = tok + grp * 8 + (up ? 8 : 0), left = n < n_end ? a.M - t0 : 0;
+            bf16* o = (bf16*)a.out + (int64_t)t0 * n_end + n;
 #pragma unroll
             for (int j = 0; j < 8; j++, o += n_end) {
               const float got = __shfl_xor_sync(0xffffffffu, up ? y[j] : y[8 + j], 16);
-              if (n < n_end && tok0 + (up ? 8 : 0) + j < a.M) *o = __float2bfloat16_rn(sb_silu_mul(up ? got : y[j], up ? y[8 + j] : got));
+              const float v = sb_silu_mul(up ? got : y[j], up ? y[8 + j] : got);
+              if (j < left) *o = __float2bfloat16_rn(v);
             }
-            continue;
-          }
+          });
+        } else if (a.out_f32) {
+          each(nothing, [&](int grp, const uint32_t* r) {
+            float y[16];
+            values(grp, r, y);
+            const int t0 = tok + grp * 8, left = n < a.N ? a.M - t0 : 0;
+            float* o = (float*)a.out + (int64_t)t0 * a.N + n;
 #pragma unroll
-          for (int j = 0; j < 16; j++) {
-            const int tok = tok0 + j, k = (j & 8) * 2 + (j & 7);
-            if (tok < a.M && n < a.N) {
-              float v;
-              if constexpr (I8) {
-                const int hi = (int)r[k], lo = (int)r[k + 8];
-                // 128 * hi + lo stays below 2^31 up to here (lo <= 64 * 127 * K <= 2^30); larger sums in 64 bits
-                v = abs(hi) < (1 << 23) ? __int2float_rn(hi * 128 + lo) : __ll2float_rn((int64_t)hi * 128 + (int64_t)lo);
-              } else {
-                v = __fadd_rn(__uint_as_float(r[k]), __fmul_rn(0.0625f, __uint_as_float(r[k + 8])));
-              }
-              const float y = __fmul_rn(__fmul_rn(v, a.sx[tok]), swn);
-              if (a.out_f32) ((float*)a.out)[(int64_t)tok * a.N + n] = y;
-              else ((bf16*)a.out)[(int64_t)tok * a.N + n] = __float2bfloat16_rn(y);
-            }
-          }
+            for (int j = 0; j < 16; j++, o += a.N)
+              if (j < left) *o = y[j];
+          });
+        } else {
+          each(nothing, [&](int grp, const uint32_t* r) {
+            float y[16];
+            values(grp, r, y);
+            const int t0 = tok + grp * 8, left = n < a.N ? a.M - t0 : 0;
+            bf16* o = (bf16*)a.out + (int64_t)t0 * a.N + n;
+#pragma unroll
+            for (int j = 0; j < 16; j++, o += a.N)
+              if (j < left) *o = __float2bfloat16_rn(y[j]);
+          });
         }
       }
       // the accumulator is drained by this warp: tell the leader's MMA warp
