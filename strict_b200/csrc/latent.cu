@@ -87,9 +87,8 @@ __device__ __forceinline__ float2 ld_cluster2(uint32_t addr) {
   asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // not volatile: the compiler may move fragment loads ahead of products that do not need them
 __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm(
@@ -783,6 +782,13 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   tc_fence_after();
   SB_TRACE_MARK(1);
   __syncthreads();  // the ring is free: it holds this block's sums now
+  if (threadIdx.x < LHEADS) {
+    const float l = (mx_s[0][0][threadIdx.x] + mx_s[0][1][threadIdx.x]) + (mx_s[0][2][threadIdx.x] + mx_s[0][3][threadIdx.x]);
+    ml_s[threadIdx.x].y = l;  // without keys: (-inf, 0)
+  }
+  // The two barriers of the cluster are announced as early as they may be and waited for as late: this one says that the ring may be written by the
+  // others and that the maxima and sums over the keys stand.
+  cluster_arrive();
   float* so = (float*)smem;  // [32][rank_p + 4]
   const int so_ld = a.rank_p + 4;
   if (ntiles > 0) {
@@ -802,10 +808,6 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
       }
     }
   }
-  if (threadIdx.x < LHEADS) {
-    const float l = (mx_s[0][0][threadIdx.x] + mx_s[0][1][threadIdx.x]) + (mx_s[0][2][threadIdx.x] + mx_s[0][3][threadIdx.x]);
-    ml_s[threadIdx.x].y = l;  // without keys: (-inf, 0)
-  }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies below read what the stores above wrote
   tc_fence_before();
   __syncthreads();
@@ -818,7 +820,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   const uint32_t slot_bytes = (uint32_t)(own * so_ld * 4);
   uint8_t* recv = smem + LHEADS * so_ld * 4;
   if (threadIdx.x == 0 && a.nsplit > 1) mbar_expect_tx(smem_u32(&bar_m), (uint32_t)((a.nsplit - 1) * n_own * so_ld * 4));
-  cluster_sync();  // every block's sums are complete and every ring is free
+  cluster_wait();
   if (threadIdx.x < a.nsplit && (int)threadIdx.x != split) {
     const int to = threadIdx.x, n = max(0, min(own, LHEADS - to * own));
     if (n > 0)
@@ -841,6 +843,8 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   }
   __syncthreads();
   if (a.nsplit > 1) wait(&bar_m, 0, 27);
+  __syncwarp();
+  cluster_arrive();  // nothing of another block's is read from here on
   SB_TRACE_MARK(2);
   const int c4n = a.rank_p / 4, heads = min(n_own, a.H - h0 - first);
   for (int i = threadIdx.x; i < heads * c4n; i += 256) {
@@ -859,7 +863,8 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     *(uint2*)(a.out + ((int64_t)b * a.H + h0 + first + h) * a.rank_p + c) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
   }
   if (err) { *(volatile int*)a.status = err; __threadfence_system(); }
-  cluster_sync();  // nobody leaves while another block may still read its shared memory
+  __syncwarp();
+  cluster_wait();  // nobody leaves while another block may still read its shared memory
   SB_TRACE_END(SB_K_ATTN, 0);
 }
 
