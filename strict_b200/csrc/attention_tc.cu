@@ -56,6 +56,23 @@ struct TcAttnArgs {
   const float* gate;     // [rows, Hq] factor of a head's output; may be null
 };
 
+// Which block this is. The tile of queries is the slowest index of the grid and counts down: the blocks with the most keys start first, those of all sequences
+// and heads, and the short ones fill the SMs at the end. (With ascending tiles as the fastest index the last block to start was one of the longest.) A grid
+// has 65535 tiles that way; longer prompts keep the tiles in x. Qwen3-8B, four prompts
+// of up to 2048 tokens of uneven length: 97.0 to 99.8 -> 84.1 to 85.5 ms; 4 x 8192 tokens, 32 heads: 3.36 -> 3.31 ms.
+struct TcBlock {
+  int tile, h, b;
+};
+constexpr int64_t TILES_Z = 65535;
+__device__ __forceinline__ TcBlock tc_block(const TcAttnArgs& a, int q) {
+  if (((int64_t)a.S + q - 1) / q > TILES_Z) return {(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
+  return {(int)(gridDim.z - 1 - blockIdx.z), (int)blockIdx.x, (int)blockIdx.y};
+}
+dim3 tc_grid(int64_t S, int64_t q, int Hq, int B) {
+  const int64_t tiles = (S + q - 1) / q;
+  return tiles > TILES_Z ? dim3((unsigned)tiles, (unsigned)Hq, (unsigned)B) : dim3((unsigned)Hq, (unsigned)B, (unsigned)tiles);
+}
+
 __global__ void __launch_bounds__(128) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                                               const __grid_constant__ CUtensorMap map_v, TcAttnArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -64,7 +81,8 @@ __global__ void __launch_bounds__(128) attn_prefill_tc_kernel(const __grid_const
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * BQ;
+  const TcBlock at = tc_block(a, BQ);
+  const int b = at.b, h = at.h, q0 = at.tile * BQ;
   const int len = a.lens[b], pst = a.past ? a.past[b] : 0;
   const int n_new = len - pst;
   if (q0 >= n_new) return;  // whole block, before anything is allocated
@@ -316,7 +334,8 @@ __global__ void __launch_bounds__(TC2_THREADS) attn_prefill_tc2_kernel(const __g
   __shared__ uint32_t tmem_base_slot;
   __shared__ float x_max[2][2][BQ], x_sum[2][BQ];  // [tile][column half][row]: exchange between the two threads of a row
 
-  const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * 2 * BQ;
+  const TcBlock at = tc_block(a, 2 * BQ);
+  const int b = at.b, h = at.h, q0 = at.tile * 2 * BQ;
   const int len = a.lens[b], pst = a.past ? a.past[b] : 0;
   const int n_new = len - pst;
   if (q0 >= n_new) return;  // whole block, before anything is allocated
@@ -579,8 +598,7 @@ int launch_tc2(strictb200_ctx* ctx, const CUtensorMap* m, const TcAttnArgs& a, i
   const size_t smem = tc2_tile_bytes<QA, RA, VA, KST>() + 1024;
   static SbDeviceOnce once;  // one per instantiation
   SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(attn_prefill_tc2_kernel<QA, RA, VA, KST, WIN, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
-  dim3 grid((unsigned)((S + 2 * BQ - 1) / (2 * BQ)), (unsigned)a.Hq, (unsigned)B);
-  attn_prefill_tc2_kernel<QA, RA, VA, KST, WIN, PLAIN><<<grid, TC2_THREADS, smem, ctx->stream>>>(m[0], m[1], m[2], m[3], m[4], a);
+  attn_prefill_tc2_kernel<QA, RA, VA, KST, WIN, PLAIN><<<tc_grid(S, 2 * BQ, a.Hq, B), TC2_THREADS, smem, ctx->stream>>>(m[0], m[1], m[2], m[3], m[4], a);
   SB_LAUNCHED(ctx);
   return STRICTB200_OK;
 }
@@ -611,8 +629,7 @@ int k_attn_prefill_tc(strictb200_ctx* ctx, const bf16* q, const bf16* kc, const 
   const size_t smem = 3 * TILE_BYTES + 1024;
   static SbDeviceOnce once;
   SB_CUDA(once.run(ctx->device, [&] { return cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }));
-  dim3 grid((unsigned)((S + BQ - 1) / BQ), (unsigned)Hq, (unsigned)B);
-  attn_prefill_tc_kernel<<<grid, 128, smem, ctx->stream>>>(mq, mk, mv, a);
+  attn_prefill_tc_kernel<<<tc_grid(S, BQ, Hq, B), 128, smem, ctx->stream>>>(mq, mk, mv, a);
   SB_LAUNCHED(ctx);
   return STRICTB200_OK;
 }
