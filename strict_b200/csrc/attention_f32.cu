@@ -23,6 +23,23 @@ __global__ void kv_append_f32_kernel(const float* qkv, float* __restrict__ kc, f
     vc[dst] = qkv[t * 3 * hd + 2 * hd + e];
   }
 }
+// Head widths that are multiples of four, 16-byte aligned: four columns of a key and of its value per thread. 4800 tokens of 768 columns: 9.6 us,
+// 19.5 with a thread per column.
+__global__ void __launch_bounds__(256) kv_append_f32_vec_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc, const int32_t* seq, const int32_t* pos,
+                                                                const int32_t* lens, uint32_t n, uint32_t hd, uint32_t Dh, int H, int maxlen) {
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x, per = hd / 4;
+  if (i >= n) return;
+  const uint32_t t = i / per, e = (i - t * per) * 4, h = e / Dh;
+  const float* row = qkv + (int64_t)t * 3 * hd + hd + e;
+  const float4 k = *(const float4*)row, v = *(const float4*)(row + hd);
+  const int b = seq ? seq[t] : (int)t, p = pos ? pos[t] : lens[b];
+  if (p < 0 || p >= maxlen) return;
+  const int64_t dst = (((int64_t)b * H + h) * maxlen + p) * Dh + (e - h * Dh);
+  *(float4*)(kc + dst) = k;
+  *(float4*)(vc + dst) = v;
+}
 // Any head width. grid (H, T), 256 threads; scores of one (token, head) live in shared memory.
 __global__ void __launch_bounds__(256) attn_f32_kernel(const float* qkv, const float* kc, const float* vc,
                                                        const int32_t* seq, const int32_t* pos,
@@ -372,7 +389,9 @@ int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, cons
     return STRICTB200_OK;
   }
   if (seq && prompts && rows16 && Dh == PD && T <= 65535 && prompts->nb <= 65535 && H <= 65535) {
-    SB_CUDA(sb_launch(ctx, kv_append_f32_kernel, dim3((unsigned)T), dim3(256), 0, qkv, kc, vc, seq, pos, lens, H, Dh, maxlen));
+    const int hd = H * Dh;
+    const uint32_t n = (uint32_t)(T * (hd / 4));  // fits: qkv alone has 48 bytes per item
+    SB_CUDA(sb_launch(ctx, kv_append_f32_vec_kernel, dim3((n + 255) / 256), dim3(256), 0, qkv, kc, vc, seq, pos, lens, n, (uint32_t)hd, (uint32_t)Dh, H, maxlen));
     ctx->launches++;
     // Blocks of 16 queries while those of 32 would all be resident (four per SM): 1 x 901 tokens 3.80 -> 3.60 ms for a GPT-2 prompt, 4 x 300 the same; with
     // more blocks those of 32 read the keys half as often (8 x 600: 9.05 ms against 9.41, and 9.17 with 64).
