@@ -1,0 +1,199 @@
+"""Decode steps of at most 16 sequences as a chain (norm in front of a product, product into the residual, key chunks merged in a cluster), the fp32
+products (many rows on pairs of SMs, many channels as a stream) and fp32 attention over prompts in blocks of 16 and 32 queries."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from strict_b200 import native as N
+from strict_b200.kernel import DeviceVariable as DV
+from conftest import TOL_F32, TOL_FP8, logits_close
+from test_gpu_models import TINY_GPT2, TINY_QWEN, _run_pair
+
+pytestmark = pytest.mark.gpu
+L = N.lib
+
+
+# one and two groups of 8 rows; widths of one to eight groups of 128 columns; products into the residual of at most 2048, 3072 and 4096 columns, ending inside
+# a warp's steps; gated channels that end inside a block's 16; weights behind the dependency wait; a width beyond the chain
+@pytest.mark.parametrize("B,over,prefetch", [(2, dict(d_model=1024, d_ff=1088), 1), (16, dict(d_model=640, d_ff=2112), 1), (8, dict(d_model=128, d_ff=3136), 1),
+                                             (9, dict(d_model=896, d_ff=64), 0), (1, dict(d_model=1024, d_ff=4096), 1), (3, dict(d_model=1088, d_ff=1088), 1)])
+def test_chained_step_vs_oracle(ctx, oracle, B, over, prefetch):
+    cfg = dict(TINY_QWEN, n_layers=1, vocab=512, **over)
+    with ctx.option("prefetch", prefetch):
+        m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 7, B, 9, [9 - i % 4 for i in range(B)], 4, random_gains=True)
+        for _ in range(2):
+            ids = oracle.argmax(want)
+            _, logits = kv.decode_step(ids, want_logits=True)
+            want = st.decode(ids)
+            ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+            assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
+
+
+# key chunks of one (sequence, head) in one cluster: one chunk, several, sequences that leave the cluster's other blocks without keys, a
+# new token that opens a chunk; with the first tiles behind the dependency wait
+@pytest.mark.parametrize("lens,prefetch", [([300, 3], 1), ([64, 63, 127, 128], 1), ([190, 1, 65], 0)])
+def test_chunks_merged_in_a_cluster_vs_oracle(ctx, oracle, lens, prefetch):
+    cfg = dict(TINY_QWEN, n_layers=2, vocab=512, max_pos=512)
+    with ctx.option("attn_prefetch", prefetch):
+        m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 3, len(lens), max(lens), lens, 4, random_gains=True)
+        for _ in range(3):
+            ids = oracle.argmax(want)
+            _, logits = kv.decode_step(ids, want_logits=True)
+            want = st.decode(ids)
+            ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+            assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
+
+
+class GemmF32Args(C.Structure):
+    _fields_ = [("M", C.c_int64), ("N", C.c_int64), ("K", C.c_int64), ("x", C.c_void_p), ("ldx", C.c_int64), ("w", C.c_void_p), ("ldw", C.c_int64),
+                ("bias", C.c_void_p), ("y", C.c_void_p), ("ldy", C.c_int64), ("mode", C.c_int), ("act_pos", C.c_float), ("act_neg", C.c_float),
+                ("col_scale", C.c_void_p), ("alpha", C.c_float), ("ln_gain", C.c_void_p), ("ln_bias", C.c_void_p), ("ln_eps", C.c_float)]
+
+
+def _gemm_f32(ctx, x, w, y, **over):
+    f = L()._Z10k_gemm_f32P14strictb200_ctxRK11GemmF32Args
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_void_p]
+    d = {k: DV.of(ctx, v) for k, v in dict(x=x, w=w, y=y, **{k: v for k, v in over.items() if isinstance(v, np.ndarray)}).items()}
+    a = GemmF32Args(M=len(x), N=len(w), K=x.shape[1], ldx=x.shape[1], ldw=w.shape[1], ldy=y.shape[1], alpha=1)
+    for k, v in over.items():
+        if not isinstance(v, np.ndarray):
+            setattr(a, k, v)
+    for k, v in d.items():
+        setattr(a, k, v.p)
+    N.check(f(ctx.h, C.addressof(a)))
+    out = d["y"].to_host().reshape(y.shape)
+    for v in d.values():
+        v.free()
+    return out
+
+
+# 44 tiles of 256 channels x 128 tokens and more, ending inside a tile of either kind and inside a stage of 64 columns; rows of one stage, of several parts
+# of four stages, and beyond the 16 stages after which the small products are taken out
+@pytest.mark.parametrize("M,N_,K", [(129, 5633, 4), (1400, 901, 68), (1409, 1000, 260), (5505, 100, 1028), (300, 4097, 2052)])
+def test_gemm_f32_on_pairs_vs_fp64(ctx, rng, M, N_, K):
+    x = (rng.standard_normal((M, K)) * np.exp2(rng.integers(-6, 7, (M, K)))).astype(np.float32)
+    w = (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(N_).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32))
+    # of the magnitudes' sum: two cut-off instructions (2 * 2^-23) and the addition of a stage's two sums, four additions in a part, one per part, two for the
+    # small products of 1024 columns, one unit for what is left out
+    bound = (4 + 1 + 4 + (K + 255) // 256 + 2 * ((K + 1023) // 1024) + 1) * 2.0 ** -24
+    assert (np.abs(got - want) <= bound * size).all()
+    assert np.sqrt(np.mean((got - want) ** 2) / np.mean(want ** 2)) < 2e-7
+    old = rng.standard_normal((M, N_)).astype(np.float32)
+    unit = 2.0 ** -22 * (np.abs(got) + np.abs(old) + np.abs(b) + 1)  # a few roundings of the values involved
+    assert (np.abs(_gemm_f32(ctx, x, w, old.copy(), bias=b, mode=1) - (old + (got + b))) <= unit).all()
+    s = rng.uniform(0.5, 2, N_).astype(np.float32)
+    assert (np.abs(_gemm_f32(ctx, x, w, old.copy(), col_scale=s, alpha=0.5, mode=4) - (old + 0.5 * s * got)) <= 2 * unit).all()
+    z = (got + b).astype(np.float64)
+    gelu = 0.5 * z * (1 + np.tanh(0.797884583 * (z + 0.044715 * z ** 3)))
+    assert (np.abs(_gemm_f32(ctx, x, w, old.copy(), bias=b, mode=2) - gelu) <= 4 * unit).all()
+
+
+# an infinity, a NaN and a sum beyond the range: the values they touch come out as plain fp32 sums give them, every other as without them
+def test_gemm_f32_on_pairs_not_finite(ctx, rng):
+    M, N_, K = 1400, 1000, 132
+    x, w = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N_, K)).astype(np.float32)
+    clean = _gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32))
+    x2, w2 = x.copy(), w.copy()
+    x2[5, 7], x2[1399, 131], w2[999, 3] = np.inf, np.nan, -np.inf
+    x2[700, :], w2[20, :] = 1e30, 1e30
+    old = np.ones((M, N_), np.float32)
+    got = _gemm_f32(ctx, x2, w2, old.copy(), mode=1) - 1
+    with np.errstate(all="ignore"):
+        want = (x2.astype(np.float64) @ w2.astype(np.float64).T).astype(np.float32)
+    rows, cols = np.ones(M, bool), np.ones(N_, bool)
+    rows[[5, 700, 1399]], cols[[20, 999]] = False, False
+    assert np.allclose(got[np.ix_(rows, cols)], clean[np.ix_(rows, cols)], rtol=1e-5, atol=1e-5)
+    for part in (np.s_[5, :], np.s_[1399, :], np.s_[:, 999]):
+        assert np.array_equal(np.isnan(got[part]), np.isnan(want[part])) and np.array_equal(np.isinf(got[part]), np.isinf(want[part]))
+    assert np.isinf(got[700, 20]) and np.isfinite(got[700, cols]).all()
+
+
+# operands of the ends of the fp32 range, as the kernel of fewer rows takes them
+@pytest.mark.parametrize("ex,ew", [(-118, 100), (-125, 120), (120, -124), (-147, 126)])
+def test_gemm_f32_on_pairs_small_operands(ctx, rng, ex, ew):
+    M, N_, K = 1400, 1000, 132
+    x = np.ldexp(rng.uniform(1, 2, (M, K)) * rng.choice([-1, 1], (M, K)), ex).astype(np.float32)
+    w = np.ldexp(rng.uniform(1, 2, (N_, K)) * rng.choice([-1, 1], (N_, K)), ew).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32))
+    # as above, and a unit at the end of the range per instruction and addition; of a value below 2^-126 half a unit is left out
+    left_out = 2.0 ** -150 * np.abs(w).astype(np.float64).sum(1) if ex < -126 else 0
+    assert (np.abs(got - want) <= 13 * 2.0 ** -24 * size + (K / 16 + 16) * 2.0 ** -149 + left_out).all()
+
+
+# a recorded call keeps its kernel and replays after larger calls have moved the scratch
+def test_gemm_f32_recorded_does_not_depend_on_scratch(ctx, rng):
+    x, w = rng.standard_normal((1400, 64)).astype(np.float32), rng.standard_normal((1000, 64)).astype(np.float32)
+    dx, dw, dy = DV.of(ctx, x), DV.of(ctx, w), DV(ctx, 1400 * 1000)
+    with ctx.record():
+        N.check(L().strictb200_gemm_f32(ctx.h, 1400, 1000, 64, dx.p, dw.p, None, dy.p))
+    _gemm_f32(ctx, rng.standard_normal((4000, 512)).astype(np.float32), rng.standard_normal((2000, 512)).astype(np.float32), np.zeros((4000, 2000), np.float32))
+    ctx.replay(ctx.last_graph)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    assert np.allclose(dy.to_host().reshape(want.shape), want, rtol=1e-5, atol=1e-5)
+    ctx.free_graph(ctx.last_graph)
+    for v in (dx, dw, dy):
+        v.free()
+
+
+# eight channels for every warp of two blocks per SM and one more, one to four rows, rows that end inside a load of a warp
+@pytest.mark.parametrize("M,N_,K", [(1, 18944, 768), (2, 18945, 4), (3, 20001, 772), (4, 19000, 1024), (1, 50257, 132)])
+def test_gemm_f32_stream_vs_fp64(ctx, rng, M, N_, K):
+    x, w = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
+    b = rng.standard_normal(N_).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).astype(np.float64).T
+    got = _gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32))
+    # a lane adds its part of at most K columns four at a time, then five folds: each addition at most 2^-24 of the magnitudes
+    assert (np.abs(got - want) <= (K / 32 + 4 + 5) * 2.0 ** -24 * size).all()
+    assert np.array_equal(_gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32), bias=b), got + b)
+
+
+# two heads and 7 tiles of 32 queries: 42 sequences are the last that take blocks of 16 queries, 43 the first with 32; lengths that end inside a warp's 8 rows, a block
+# and a tile of keys; a step over the keys they leave
+@pytest.mark.parametrize("B", [3, 42, 43])
+def test_gpt2_prompts_in_blocks_vs_oracle(ctx, oracle, B):
+    cfg = dict(TINY_GPT2, max_pos=256)
+    lens = [200 - (i * 37) % 200 for i in range(B)]
+    m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 5, B, 200, lens, 2, random_gains=True)
+    ok, mx, rel = logits_close(logits, want, **TOL_F32)
+    assert ok, (mx, rel)
+    ids = oracle.argmax(want)
+    _, logits = kv.decode_step(ids, want_logits=True)
+    ok, mx, rel = logits_close(logits, st.decode(ids), **TOL_F32)
+    assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
+
+
+# rows of a warp each (2368 rows and more) and of a block each; the narrowest and the widest of a warp, rows that end inside a lane's loads, wider ones
+@pytest.mark.parametrize("M,d", [(2368, 768), (2367, 768), (2375, 4), (2369, 772), (2370, 1024), (2368, 1028), (2400, 257)])
+def test_layer_norm_of_many_rows_vs_fp64(ctx, rng, M, d):
+    x = (rng.standard_normal((M, d)) + rng.uniform(-2, 2, (M, 1))).astype(np.float32)
+    g, b = rng.uniform(0.5, 1.5, d).astype(np.float32), rng.standard_normal(d).astype(np.float32)
+    dx, dg, db, dy = DV.of(ctx, x), DV.of(ctx, g), DV.of(ctx, b), DV(ctx, M * d)
+    N.check(L().strictb200_layernorm(ctx.h, dx.p, dg.p, db.p, 1e-5, M, d, dy.p))
+    got = dy.to_host().reshape(M, d)
+    x64 = x.astype(np.float64)
+    mean, var = x64.mean(1, keepdims=True), x64.var(1, keepdims=True)
+    r = 1 / np.sqrt(var + 1e-5)
+    # at most 16 additions in a row for each sum; of the mean that is 16 * 2^-24 of the magnitudes, of the variance half of it again in the root; a few roundings of the result
+    unit = 2.0 ** -24
+    bound = (20 * unit * (np.abs(x64).mean(1, keepdims=True) + np.abs(x64 - mean)) * r) * np.abs(g) + 4 * unit * (np.abs(b) + np.abs((x64 - mean) * r * g))
+    # a mean that is off moves the deviations together: its square enters the variance
+    assert (np.abs(got - ((x64 - mean) * r * g + b)) <= bound).all()
+    for v in (dx, dg, db, dy):
+        v.free()

@@ -99,3 +99,24 @@ def test_rule_of_the_few_row_kernel(M, N, K, f8, finished, takes):
     rule = native.lib()._Z18sb_gemm_rows_takeslllbb
     rule.restype, rule.argtypes = C.c_bool, [C.c_int64] * 3 + [C.c_bool] * 2
     assert rule(M, N, K, f8, finished) == takes
+
+
+# the same of the products of a decode chain and of the stream over many channels
+@pytest.mark.parametrize("name,request_", [("norm_rows_kernel", "__ldcs("), ("residual_rows_kernel", "__ldcs("), ("gemm_f32_stream_kernel", "request(n)")])
+def test_chained_weights_wait_where_the_option_says_so(name, request_):
+    body = KERNELS[name][2]
+    wait = re.search(r"if \(!(a\.)?prefetch\) pdl_wait\(\);", body)
+    assert wait and wait.start() < body.index(request_)
+
+
+# both sides of the lines that the rules of the chain draw
+@pytest.mark.parametrize("rule,M,N,K,takes", [
+    ("norm", 1, 4096, 1024, True), ("norm", 16, 9472, 128, True), ("norm", 17, 4096, 1024, False), ("norm", 16, 9473, 128, False), ("norm", 8, 4096, 1152, False),
+    ("norm", 8, 4096, 1000, False), ("residual", 16, 1024, 4096, True), ("residual", 1, 1184, 16, True), ("residual", 17, 1024, 2048, False),
+    ("residual", 8, 1185, 2048, False), ("residual", 8, 1024, 4112, False), ("residual", 8, 1024, 2056, False)])
+def test_rules_of_the_chain(rule, M, N, K, takes):
+    import ctypes as C
+    from strict_b200 import native
+    f = getattr(native.lib(), {"norm": "_Z18sb_norm_rows_takeslll", "residual": "_Z22sb_residual_rows_takeslll"}[rule])
+    f.restype, f.argtypes = C.c_bool, [C.c_int64] * 3
+    assert f(M, N, K) == takes
