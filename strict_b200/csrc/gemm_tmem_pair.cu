@@ -9,7 +9,7 @@
 // Operand layout, numerics and epilogue are those of gemm_tmem.cu (weights = A operand = TMEM
 // lanes, operand rows = B operand = TMEM columns, acc_hi + acc_lo/16, scales, bf16/fp32 stores).
 //
-// Roles (both blocks of a pair run the same code, 192 threads each; rank 0 is the leader):
+// Roles (both blocks of a pair run the same code, 320 threads each; rank 0 is the leader):
 //   warp 0      TMA producer of this block's halves; the bytes of both blocks complete on the
 //               LEADER's full barrier (the .cta_group::2 form of the tensor copy: each block
 //               copies only into its own shared memory)
@@ -478,6 +478,8 @@ static int launch_f8(strictb200_ctx* ctx, const GemmArgs& g) {
 }
 
 // Y = ((X . Wq^T) * sx) * sw for many tokens (prefill). ERR_UNSUPPORTED for shapes this kernel does not take.
+// us for 4096 tokens, with an epilogue of one loop for all kinds of output that loaded a scale per token between its stores, and as it is: Qwen3-0.6B
+// qkv 58.8 -> 38.4, output 28.0 -> 23.6, down 34.6 -> 30.3, the expansion of latents to 5120 bf16 channels 26.0 -> 21.3; int8 2048 x 4096 x 4096 76.9 -> 73.7.
 int k_gemm_fp8_tmem_pair(strictb200_ctx* ctx, const GemmArgs& g) { return launch_f8<PAIR_F8>(ctx, g); }
 
 // The same product of int8 operands (gemm_int8.cu), which all fits as above. 2048 tokens, 4096 x 4096: see k_gemm_int8w.

@@ -957,7 +957,7 @@ template <>
 __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
 // grid (M, groups * cb): a block owns one group of a row, or one of the cb slices a cluster shares (the sum of squares is
-// then exchanged). The sums, the new residual and both outputs pass through registers once; the gains are constants and are
+// then exchanged). The sums, the new residual and both outputs pass through registers once; gains and scales are constants and are
 // fetched before the dependency wait. A thread owns NI float4s: one in the decode step's blocks, up to four in a prompt's.
 template <typename T, int NI>
 __global__ void __launch_bounds__(NI == 1 ? 1024 : 512) group_norm_kernel(GroupNormDev a, int64_t M) {
