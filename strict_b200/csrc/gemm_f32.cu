@@ -42,7 +42,8 @@ __device__ __forceinline__ float fold_sums(float* v, int lane) {
 // not declared invariant: loads of invariant data may be moved in front of the dependency wait.
 // PRE: float4 of a weight row that a lane holds, as many as its slice has where that is less than F32_PRE (one row of X). The weights in
 // flight are registers, and the blocks of the next kernel can only request theirs beside these, so a block takes what it needs and no more:
-// with F32_PRE for all, 128 registers, the blocks of a GPT-2 step's projections started when those in front had left.
+// with F32_PRE for all, 128 registers, the blocks of a GPT-2 step's projections started when those in front had left. The norm in front (LN) is
+// that of the whole row, however many warps share the weights: with it PRE holds a row of X.
 constexpr int rows_regs(int MT, int NC, bool LN, int PRE) { return MT > 1 || PRE == F32_PRE ? 128 : (40 + 4 * PRE * (NC + (LN ? 1 : 0)) + 7) / 8 * 8; }
 template <int MT, int NC, bool STAGED, bool LN, int PRE>
 __maxnreg__(rows_regs(MT, NC, LN, PRE)) __global__ void gemm_f32_kernel(int M, int N, int K, const float* x, int64_t ldx, const float* __restrict__ w,
@@ -156,6 +157,7 @@ __maxnreg__(rows_regs(MT, NC, LN, PRE)) __global__ void gemm_f32_kernel(int M, i
 
 template <int MT, int NC, bool STAGED, bool LN, int PRE = F32_PRE>
 int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
+  if (LN && g.K > 128 * PRE) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: the norm in front does not hold its row");
   const int rows = 8 / ks * NC;
   dim3 grid((unsigned)((g.N + rows - 1) / rows), (unsigned)((g.M + MT - 1) / MT));
   if (grid.y > 65535) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: M too large");
@@ -170,7 +172,7 @@ int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
 template <int MT, int NC>
 int launch_rows(strictb200_ctx* ctx, const GemmF32Args& g, int ks) {
   if constexpr (MT == 1) {
-    const int64_t pre = ((g.K / 4 + ks - 1) / ks + 31) / 32;
+    const int64_t pre = ((g.ln_gain ? g.K / 4 : (g.K / 4 + ks - 1) / ks) + 31) / 32;
     if (pre <= 3) return g.ln_gain ? launch_rows<1, NC, true, true, 3>(ctx, g, ks) : launch_rows<1, NC, false, false, 3>(ctx, g, ks);
     if (pre <= 6) return g.ln_gain ? launch_rows<1, NC, true, true, 6>(ctx, g, ks) : launch_rows<1, NC, false, false, 6>(ctx, g, ks);
   }

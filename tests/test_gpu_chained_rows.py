@@ -197,3 +197,39 @@ def test_layer_norm_of_many_rows_vs_fp64(ctx, rng, M, d):
     assert (np.abs(got - ((x64 - mean) * r * g + b)) <= bound).all()
     for v in (dx, dg, db, dy):
         v.free()
+
+
+# the layer norm in front of the product, which is that of the whole row where two warps share a channel's columns too (one row, 512 columns and more, at
+# most 1184 channels): both sides of that line, the ends of the registers that hold a row (384, 768, 1024 columns), a narrow row, a wide matrix, several rows
+@pytest.mark.parametrize("M,N_,K", [(1, 512, 512), (1, 1024, 512), (1, 700, 640), (1, 768, 768), (1, 40, 772), (1, 1184, 1024), (1, 1185, 1024), (1, 1184, 508), (1, 9, 384),
+                                    (1, 9, 388), (1, 3072, 768), (1, 64, 4), (2, 768, 768), (8, 512, 1024)])
+def test_gemm_f32_norm_in_front_vs_fp64(ctx, rng, M, N_, K):
+    x = (rng.standard_normal((M, K)) * np.linspace(0.2, 3, K) + rng.uniform(-2, 2, (M, 1))).astype(np.float32)  # a row whose parts differ in size
+    w = (rng.standard_normal((N_, K)) * 0.02).astype(np.float32)
+    g, b, c = rng.uniform(0.5, 1.5, K).astype(np.float32), rng.standard_normal(K).astype(np.float32), rng.standard_normal(N_).astype(np.float32)
+    got = _gemm_f32(ctx, x, w, np.zeros((M, N_), np.float32), bias=c, ln_gain=g, ln_bias=b, ln_eps=1e-5)
+    x64, w64 = x.astype(np.float64), np.abs(w).astype(np.float64)
+    mean = x64.mean(1, keepdims=True)
+    r = 1 / np.sqrt(x64.var(1, keepdims=True) + 1e-5)
+    n = (x64 - mean) * r * g + b
+    # of the norm: at most 16 additions in a row for each of its sums and a few roundings of the result; of the product: a lane's part of at most K columns, four at
+    # a time, 5 folds, two slices and the bias
+    unit = 2.0 ** -24
+    off = 20 * unit * (np.abs(x64).mean(1, keepdims=True) + np.abs(x64 - mean)) * r * np.abs(g) + 4 * unit * (np.abs(b) + np.abs((x64 - mean) * r * g))
+    assert (np.abs(got - (n @ w.astype(np.float64).T + c)) <= off @ w64.T + (K / 32 + 4 + 5 + 3) * unit * (np.abs(n) @ w64.T + np.abs(c))).all()
+
+
+# decode steps of one sequence of GPT-2 models whose feed-forward is narrow enough for two warps per channel
+@pytest.mark.parametrize("d,ff", [(512, 1024), (768, 768), (1024, 1152)])
+def test_gpt2_one_sequence_narrow_feed_forward_vs_oracle(ctx, oracle, d, ff):
+    cfg = dict(TINY_GPT2, d_model=d, n_q_heads=d // 64, n_kv_heads=d // 64, d_ff=ff)
+    m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 6, 1, 5, None, 4, random_gains=True)
+    for _ in range(3):
+        ids = oracle.argmax(want)
+        _, logits = kv.decode_step(ids, want_logits=True)
+        want = st.decode(ids)
+        ok, mx, rel = logits_close(logits, want, **TOL_F32)
+        assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
