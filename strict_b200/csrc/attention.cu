@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const b
   __shared__ __align__(16) bf16 q_s[FUSED ? 16 * HD : 8];    // the query heads of this KV head
   __shared__ __align__(16) bf16 kv_new[FUSED ? 2 * HD : 8];  // the new token's key row, then its value row
   __shared__ __align__(8) unsigned long long merge_bar;
+  __shared__ int len_s;
   SB_TRACE_BEGIN();
   if (MERGE) {
     if (threadIdx.x == 0) {
@@ -347,6 +348,10 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const b
   }
   pdl_trigger();
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  // One reading for the whole block: the length may change at any time until the dependency wait, and what follows from it, barriers among
+  // it, has to be the same for every thread.
+  if (threadIdx.x == 0) len_s = ld_volatile_i32(lens + b);
+  __syncthreads();
   const int G = Hq / Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   const int k_begin = split * chunk;
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const b
   // written in earlier steps are touched, never the block's last tile (it may hold the row the
   // preceding kernel appends; FUSED: whatever is read of that row is replaced by the block itself, so the last tile too), and the
   // length they are derived from is read again after the wait: if it changed, the tiles are loaded again from scratch.
-  const int len_early = min(ld_volatile_i32(lens + b) + len_add, maxlen);
+  const int len_early = min(len_s + len_add, maxlen);
   int npre = 0;
   if (prefetch && k_begin < len_early) {
     const int nt = (min(len_early, k_begin + chunk) - k_begin + KT - 1) / KT;

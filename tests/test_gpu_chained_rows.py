@@ -233,3 +233,29 @@ def test_gpt2_one_sequence_narrow_feed_forward_vs_oracle(ctx, oracle, d, ff):
     for o in (kv, m):
         o.dispose()
     st.close(), om.close()
+
+
+# lengths that a kernel in front changes while the attention has already asked for keys: a product of one block that takes half a millisecond, the lengths'
+# increment behind it, attention behind both, all three launched at once. Longer, shorter, across chunks and tiles, no keys at first
+@pytest.mark.parametrize("lens,inc", [([200, 64, 1], 1), ([300, 63, 900], 100), ([1000, 700, 129], -100), ([0, 512, 5], 1)])
+def test_decode_attention_takes_a_length_that_changes(ctx, oracle, rng, lens, inc):
+    B, Hq, Hkv, D, maxlen, K = len(lens), 8, 2, 128, 1024, 1 << 22
+    dq, dk, dv = (DV.of(ctx, oracle.f32_to_bf16(rng.standard_normal(s).astype(np.float32))) for s in ((B, Hq, D), (B, Hkv, maxlen, D), (B, Hkv, maxlen, D)))
+    dx, dw, dy = DV.of(ctx, np.ones(K, np.float32)), DV.of(ctx, np.ones(K, np.float32)), DV(ctx, 1)
+    add = L()._Z9k_add_i32P14strictb200_ctxPiPKiil
+    add.restype, add.argtypes = C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int64]
+    out = []
+    for late in (False, True):
+        dl = DV.of(ctx, np.array(lens if late else [n + inc for n in lens], np.int32))
+        got = DV(ctx, B * Hq * D, np.uint16)
+        ctx.synchronize()
+        if late:
+            N.check(L().strictb200_gemm_f32(ctx.h, 1, 1, K, dx.p, dw.p, None, dy.p))
+            N.check(add(ctx.h, dl.p, None, inc, B))
+        N.check(L().strictb200_attn_decode(ctx.h, dq.p, dk.p, dv.p, dl.p, B, Hq, Hkv, D, maxlen, D ** -0.5, got.p))
+        out.append(got.to_host())
+        for v in (dl, got):
+            v.free()
+    assert np.array_equal(out[0], out[1])
+    for v in (dq, dk, dv, dx, dw, dy):
+        v.free()

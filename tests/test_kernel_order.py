@@ -120,3 +120,14 @@ def test_rules_of_the_chain(rule, M, N, K, takes):
     f = getattr(native.lib(), {"norm": "_Z18sb_norm_rows_takeslll", "residual": "_Z22sb_residual_rows_takeslll"}[rule])
     f.restype, f.argtypes = C.c_bool, [C.c_int64] * 3
     assert f(M, N, K) == takes
+
+
+# A length that is read before the dependency wait may change under the reader: one thread reads it, and the block takes it from there
+@pytest.mark.parametrize("name", ["attn_decode_kernel"])
+def test_early_length_is_one_reading_for_the_block(name):
+    body = KERNELS[name][2]
+    early = body[:body.index("pdl_wait()")]
+    at = [m.start() for m in re.finditer(r"ld_volatile_i32\(", early)]
+    assert len(at) == 1
+    stored = re.search(r"if \(threadIdx\.x == 0\) (\w+) = ld_volatile_i32\([^;]*;(.*?)__syncthreads\(\);(.*)", early, re.S)
+    assert stored and not re.search(r"\b%s\b" % stored[1], stored[2]) and re.search(r"\b%s\b" % stored[1], stored[3])
