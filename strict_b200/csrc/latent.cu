@@ -533,7 +533,7 @@ __device__ __forceinline__ float transposed_reduce(const float* v, int lane, Op 
 __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, AttnDecodeDev a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-  __shared__ __align__(8) uint64_t k_full[MAX_STAGES][GROUPS], k_empty[MAX_STAGES], q_full, bar_s[2], bar_p, bar_o[2], bar_m;
+  __shared__ __align__(8) uint64_t k_full[MAX_STAGES][GROUPS], k_empty[MAX_STAGES], q_full, bar_s[2], bar_p[2], bar_o[2], bar_m;
   __shared__ uint32_t tmem_slot;
   __shared__ float corr_s[4][LHEADS], mx_s[2][4][LHEADS];  // [softmax warp], [tile parity][softmax warp]
   __shared__ float2 ml_s[LHEADS];
@@ -551,8 +551,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     }
     mbar_init(smem_u32(&q_full), 1);
     mbar_init(smem_u32(&bar_m), 1);
-    mbar_init(smem_u32(&bar_p), 128);
-    for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&bar_s[i]), 1); mbar_init(smem_u32(&bar_o[i]), 1); }
+    for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&bar_s[i]), 1); mbar_init(smem_u32(&bar_p[i]), 128); mbar_init(smem_u32(&bar_o[i]), 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 5 && lane < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(lane ? &map_q : &map_k) : "memory");
@@ -651,7 +650,9 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     bool go = __all_sync(0xffffffffu, err == 0);
     uint32_t spins = 0;
     while (np < ntiles && go) {
-      if (ns > np && ready(&bar_p, pr)) {  // the weights are in shared memory, O^T follows the new maxima
+      // The weights are in shared memory, O^T follows the new maxima. A barrier for each half of the weights: the softmax warps may finish the next tile
+      // before this warp has seen this one, and of two phases that end between two polls of one barrier its parity tells nothing.
+      if (ns > np && ready(&bar_p[np & 1], pr)) {
         tc_fence_after();
         const uint64_t dc = dc0 + (uint64_t)(uint32_t)(ps * stage16), dp = dp0 + (uint64_t)(uint32_t)((np & 1) * (P_BYTES >> 4));
         if (elect_one()) {
@@ -664,8 +665,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
         __syncwarp();
         tc_commit_warp(smem_u32(&bar_o[np & 1]));
         tc_commit_warp(smem_u32(&k_empty[ps]));
-        np++;
-        pr ^= 1;
+        pr ^= np++ & 1;
         if (++ps == a.stages) ps = 0;
         spins = 0;
       } else if (ns < ntiles && ns <= np + 1 && ready(&k_full[st][sg], sp)) {
@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read what these stores wrote
       tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_p)) : "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_p[t & 1])) : "memory");
     }
     // sums over the keys; the barrier keeps them out of maxima that are still being read
     asm volatile("bar.sync 1, 128;" ::: "memory");

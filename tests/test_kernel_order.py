@@ -131,3 +131,28 @@ def test_early_length_is_one_reading_for_the_block(name):
     assert len(at) == 1
     stored = re.search(r"if \(threadIdx\.x == 0\) (\w+) = ld_volatile_i32\([^;]*;(.*?)__syncthreads\(\);(.*)", early, re.S)
     assert stored and not re.search(r"\b%s\b" % stored[1], stored[2]) and re.search(r"\b%s\b" % stored[1], stored[3])
+
+
+# The latent decode kernel's softmax warps and the warp that issues its products, as far as their barriers go. A poll tells by one bit whether the phase it asks for
+# has ended: with one barrier for the weights of all tiles two of them may end between two polls, which then never succeed.
+def test_latent_decode_weights_are_seen_in_every_order():
+    body = KERNELS["latent_attn_decode_kernel"][2]
+    n = int((re.search(r"\bbar_p\[(\d)\]", body) or [0, 1])[1])
+    if n == 2:
+        assert "mbar_init(smem_u32(&bar_p[i]), 128)" in body and "ready(&bar_p[np & 1], pr)" in body and "smem_u32(&bar_p[t & 1])" in body and "pr ^= np++ & 1" in body
+    tiles, todo, seen = 6, [(0, 0, 0, (0,) * n)], set()
+    while todo:
+        state = todo.pop()
+        if state in seen:
+            continue
+        seen.add(state)
+        t, ns, np_, ended = state  # softmax tile, products S and O issued (and, as fast as can be, complete), phases that have ended
+        after = []
+        if t < min(ns, tiles) and (t < 2 or np_ > t - 2):  # the weights of tile t take the half that the product of tile t - 2 has read
+            after.append((t + 1, ns, np_, tuple(e + (i == t % n) for i, e in enumerate(ended))))
+        if ns > np_ and ended[np_ % n] % 2 != np_ // n % 2:
+            after.append((t, ns, np_ + 1, ended))
+        elif ns < tiles and ns <= np_ + 1:
+            after.append((t, ns + 1, np_, ended))
+        assert after or np_ == tiles, f"nobody can go on: softmax at tile {t}, {ns} scores and {np_} outputs issued"
+        todo += after
