@@ -44,6 +44,7 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm vo
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // Bounded wait for the phase with the given parity. Returns false when the limit expired.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t i = 0; i < (1u << 22); i++) {
@@ -530,6 +531,21 @@ __device__ __forceinline__ float transposed_reduce(const float* v, int lane, Op 
   return op(keep, __shfl_xor_sync(0xffffffffu, send, 4));
 }
 
+// The early tiles of a length that changed are let in, and their barriers go back to where they began (one arrival completes the odd phase). Whole warp.
+// A function of its own: its code in the middle of the kernel's, hardly ever run but fetched over, took 0.15 us of a launch.
+__device__ __noinline__ int let_in(uint32_t bars, int tiles, int groups) {
+  int err = 0;
+  for (int i = 0; i < tiles; i++)
+    for (int g = 0; g < groups; g++) {
+      const uint32_t bar = bars + (uint32_t)(i * GROUPS + g) * 8;
+      if (!mbar_wait(bar, 0)) err = 17;
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+    }
+  __syncwarp();
+  return err;
+}
+
 __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, AttnDecodeDev a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -538,6 +554,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   __shared__ float corr_s[4][LHEADS], mx_s[2][4][LHEADS];  // [softmax warp], [tile parity][softmax warp]
   __shared__ float2 ml_s[LHEADS];
   __shared__ float fs[LHEADS][MAX_SPLITS];
+  __shared__ int len_s;
   SB_TRACE_BEGIN();
   const int split = blockIdx.x, h0 = blockIdx.y * LHEADS, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -554,6 +571,8 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&bar_s[i]), 1); mbar_init(smem_u32(&bar_p[i]), 128); mbar_init(smem_u32(&bar_o[i]), 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // One reading for the whole block: the length may change at any time until the dependency wait, and every thread has to walk the same tiles.
+  if (threadIdx.x == 192) len_s = ld_volatile_i32(a.lens + b);
   if (warp == 5 && lane < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(lane ? &map_q : &map_k) : "memory");
   if (warp == 4) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
@@ -589,9 +608,9 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     }
   };
   // Tiles that hold rows of earlier steps only are requested before the dependency wait; the length they are derived from is
-  // read again after it. (It belongs to the previous step and has not changed; if it had, the step would report an error.)
+  // read again after it, and if it changed they are let in and requested again.
   int kb, ke, n_early = 0;
-  const int len_early = min(ld_volatile_i32(a.lens + b) + 1, a.maxlen);
+  const int len_early = min(len_s + 1, a.maxlen);
   range(len_early, kb, ke);
   if (a.prefetch)
     for (; n_early < a.stages && kb + (n_early + 1) * LKT <= min(ke, len_early - 1); n_early++)
@@ -600,8 +619,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   SB_TRACE_WAITED();
   const int len = min(ld_volatile_i32(a.lens + b) + 1, a.maxlen);
   int err = 0;
-  if (len != len_early && n_early) err = 17;
-  else range(len, kb, ke);
+  if (__builtin_expect(len != len_early, 0)) range(len, kb, ke);
   const int ntiles = kb < ke ? (ke - kb + LKT - 1) / LKT : 0;
   auto wait = [&](uint64_t* bar, int parity, int code) {
     if (!err && !mbar_wait(smem_u32(bar), (uint32_t)parity & 1)) err = code;
@@ -609,6 +627,10 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   };
   if (warp == 5) {
     // ---- TMA producer, the whole warp in step
+    if (__builtin_expect(len != len_early, 0)) {  // before the queries are requested, which the issuing warp waits for first
+      err = let_in(smem_u32(&k_full[0][0]), n_early, (n_atoms + per_group - 1) / per_group);
+      n_early = 0;
+    }
     if (ntiles > 0) {
       mbar_expect_tx_warp(smem_u32(&q_full), (uint32_t)(n_atoms * Q_ATOM));
 #pragma unroll 1
@@ -769,7 +791,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read what these stores wrote
       tc_fence_before();
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_p[t & 1])) : "memory");
+      mbar_arrive(smem_u32(&bar_p[t & 1]));
     }
     // sums over the keys; the barrier keeps them out of maxima that are still being read
     asm volatile("bar.sync 1, 128;" ::: "memory");

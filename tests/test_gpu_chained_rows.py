@@ -239,23 +239,53 @@ def test_gpt2_one_sequence_narrow_feed_forward_vs_oracle(ctx, oracle, d, ff):
 # increment behind it, attention behind both, all three launched at once. Longer, shorter, across chunks and tiles, no keys at first
 @pytest.mark.parametrize("lens,inc", [([200, 64, 1], 1), ([300, 63, 900], 100), ([1000, 700, 129], -100), ([0, 512, 5], 1)])
 def test_decode_attention_takes_a_length_that_changes(ctx, oracle, rng, lens, inc):
-    B, Hq, Hkv, D, maxlen, K = len(lens), 8, 2, 128, 1024, 1 << 22
+    B, Hq, Hkv, D, maxlen = len(lens), 8, 2, 128, 1024
     dq, dk, dv = (DV.of(ctx, oracle.f32_to_bf16(rng.standard_normal(s).astype(np.float32))) for s in ((B, Hq, D), (B, Hkv, maxlen, D), (B, Hkv, maxlen, D)))
+    _with_lengths_that_change(ctx, lens, inc, B * Hq * D, lambda dl, out: N.check(
+        L().strictb200_attn_decode(ctx.h, dq.p, dk.p, dv.p, dl.p, B, Hq, Hkv, D, maxlen, D ** -0.5, out.p)))
+    for v in (dq, dk, dv):
+        v.free()
+
+
+def _with_lengths_that_change(ctx, lens, inc, n_out, attention):
+    K, out = 1 << 22, []
     dx, dw, dy = DV.of(ctx, np.ones(K, np.float32)), DV.of(ctx, np.ones(K, np.float32)), DV(ctx, 1)
     add = L()._Z9k_add_i32P14strictb200_ctxPiPKiil
     add.restype, add.argtypes = C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int64]
-    out = []
     for late in (False, True):
         dl = DV.of(ctx, np.array(lens if late else [n + inc for n in lens], np.int32))
-        got = DV(ctx, B * Hq * D, np.uint16)
+        got = DV(ctx, n_out, np.uint16)
         ctx.synchronize()
         if late:
             N.check(L().strictb200_gemm_f32(ctx.h, 1, 1, K, dx.p, dw.p, None, dy.p))
-            N.check(add(ctx.h, dl.p, None, inc, B))
-        N.check(L().strictb200_attn_decode(ctx.h, dq.p, dk.p, dv.p, dl.p, B, Hq, Hkv, D, maxlen, D ** -0.5, got.p))
+            N.check(add(ctx.h, dl.p, None, inc, len(lens)))
+        attention(dl, got)
         out.append(got.to_host())
+        assert ctx.device_status() == 0
         for v in (dl, got):
             v.free()
-    assert np.array_equal(out[0], out[1])
-    for v in (dq, dk, dv, dx, dw, dy):
+    assert out[0].any() and np.array_equal(out[0], out[1])
+    for v in (dx, dw, dy):
+        v.free()
+
+
+class LatentShape(C.Structure):
+    _fields_ = [("H", C.c_int), ("dim", C.c_int), ("rot", C.c_int), ("vdim", C.c_int), ("rank", C.c_int), ("window", C.c_int), ("scale", C.c_float)]
+
+
+# the same of latent attention: fewer and more early tiles than the ring has stages, a window that moves with the length, one block and clusters, rows of which one
+# block fills an SM
+@pytest.mark.parametrize("lens,inc,rank,window,nsplit", [([200, 63, 130], 1, 256, 0, 2), ([1000, 64, 500], 24, 256, 0, 4), ([900, 700, 129], -100, 256, 256, 1),
+                                                         ([500, 1000, 3], 1, 512, 0, 8), ([640, 300, 0], 65, 256, 128, 2)])
+def test_latent_attention_takes_a_length_that_changes(ctx, oracle, rng, lens, inc, rank, window, nsplit):
+    B, H, dim, rot, vdim, maxlen = len(lens), 16, 128, 64, 128, 1088
+    s = LatentShape(H, dim, rot, vdim, rank, window, (dim + rot) ** -0.5)
+    chunk = ((min(window, maxlen) if window else maxlen) + nsplit * 64 - 1) // (nsplit * 64) * 64
+    dq, dk, dw = (DV.of(ctx, oracle.f32_to_bf16(0.3 * rng.standard_normal(n).astype(np.float32))) for n in ((B, H, rank + rot), (B, maxlen, rank + rot), (2 * H * dim, rank)))
+    scratch = DV(ctx, B * H * rank, np.uint16)
+    f = L()._Z20k_latent_attn_decodeP14strictb200_ctxRK11LatentShapePK13__nv_bfloat16S6_PKiiiiiPS4_S6_S9_l
+    f.restype, f.argtypes = C.c_int, [C.c_void_p] * 5 + [C.c_int] * 4 + [C.c_void_p] * 3 + [C.c_int64]
+    _with_lengths_that_change(ctx, lens, inc, B * H * vdim, lambda dl, out: N.check(
+        f(ctx.h, C.addressof(s), dq.p, dk.p, dl.p, B, maxlen, chunk, nsplit, scratch.p, dw.p, out.p, H * vdim)))
+    for v in (dq, dk, dw, scratch):
         v.free()

@@ -123,13 +123,13 @@ def test_rules_of_the_chain(rule, M, N, K, takes):
 
 
 # A length that is read before the dependency wait may change under the reader: one thread reads it, and the block takes it from there
-@pytest.mark.parametrize("name", ["attn_decode_kernel"])
+@pytest.mark.parametrize("name", ["attn_decode_kernel", "latent_attn_decode_kernel"])
 def test_early_length_is_one_reading_for_the_block(name):
     body = KERNELS[name][2]
     early = body[:body.index("pdl_wait()")]
     at = [m.start() for m in re.finditer(r"ld_volatile_i32\(", early)]
     assert len(at) == 1
-    stored = re.search(r"if \(threadIdx\.x == 0\) (\w+) = ld_volatile_i32\([^;]*;(.*?)__syncthreads\(\);(.*)", early, re.S)
+    stored = re.search(r"if \(threadIdx\.x == \d+\) (\w+) = ld_volatile_i32\([^;]*;(.*?)__syncthreads\(\);(.*)", early, re.S)
     assert stored and not re.search(r"\b%s\b" % stored[1], stored[2]) and re.search(r"\b%s\b" % stored[1], stored[3])
 
 
@@ -156,3 +156,15 @@ def test_latent_decode_weights_are_seen_in_every_order():
             after.append((t, ns + 1, np_, ended))
         assert after or np_ == tiles, f"nobody can go on: softmax at tile {t}, {ns} scores and {np_} outputs issued"
         todo += after
+
+
+# Key tiles that were requested for another length are let in and requested again: the barrier they complete on is back in its first phase afterwards
+def test_latent_decode_reloads_for_another_length():
+    text = open(os.path.join(CSRC, "latent.cu")).read()
+    let_in = text[text.index("int let_in("):]
+    assert 0 <= let_in.index("mbar_wait(bar, 0)") < let_in.index("mbar_arrive(bar)") < let_in.index("return err")
+    body = KERNELS["latent_attn_decode_kernel"][2]
+    again = re.search(r"err = let_in\(smem_u32\(&k_full\[0\]\[0\]\), n_early, .*?n_early = 0;", body, re.S)
+    assert again and body.index("pdl_wait()") < again.start() and again.end() < body.index("mbar_expect_tx_warp(smem_u32(&q_full)")
+    issue = body[body.index("constexpr uint32_t idesc_s"):]
+    assert issue.index("wait(&q_full, 0, 20)") < issue.index("ready(&k_full")
