@@ -600,7 +600,13 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const b
     uint32_t done = 0;
     for (uint32_t spins = 0; !done && spins < (1u << 20); spins++)
       asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(0u) : "memory");
-    if (!done && threadIdx.x == 0) { *(volatile int*)status = 6; __threadfence_system(); }
+    if (__builtin_expect(!__all_sync(0xffffffffu, done), 0)) {
+      // What should have come did not: no output, and this block's shared memory stays until the others, which may be late, have left or given up too.
+      if (lane == 0) { *(volatile int*)status = 6; __threadfence_system(); }
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      return;
+    }
     for (int e = lo + (int)threadIdx.x; e < hi; e += 128) {
       const int row = e / (HD / 4), d = (e % (HD / 4)) * 4;
       float M = -INFINITY;

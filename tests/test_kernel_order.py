@@ -168,3 +168,12 @@ def test_latent_decode_reloads_for_another_length():
     assert again and body.index("pdl_wait()") < again.start() and again.end() < body.index("mbar_expect_tx_warp(smem_u32(&q_full)")
     issue = body[body.index("constexpr uint32_t idesc_s"):]
     assert issue.index("wait(&q_full, 0, 20)") < issue.index("ready(&k_full")
+
+
+# The merge of the key chunks inside a cluster: where the bounded wait ran out nothing is written, and the block stays until no other can still store into it
+def test_merge_that_gave_up_stays_until_the_others_have_left():
+    body = KERNELS["attn_decode_kernel"][2]
+    merge = body[body.index("mbarrier.try_wait"):]
+    gave_up = re.search(r"if \(\w*\(?!__all_sync\(0xffffffffu, done\)[^{]*\{(.*?)return;", merge, re.S)
+    assert gave_up and gave_up.end() < merge.index("*(uint2*)(out +")
+    assert 0 <= gave_up[1].index("barrier.cluster.arrive") < gave_up[1].index("barrier.cluster.wait")
