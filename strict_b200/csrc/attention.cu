@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const bf16* q, const b
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&merge_bar)));
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncwarp();  // .aligned: the whole warp at once
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
   pdl_trigger();

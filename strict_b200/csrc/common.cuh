@@ -839,6 +839,7 @@ __device__ __forceinline__ void cluster_exchange_init(ClusterExchange* x) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&x->bar[1])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  __syncwarp();  // .aligned: the whole warp at once
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
 // All threads of all blocks call this with a block-uniform value, at most once per `which` (0,

@@ -177,3 +177,11 @@ def test_merge_that_gave_up_stays_until_the_others_have_left():
     gave_up = re.search(r"if \(\w*\(?!__all_sync\(0xffffffffu, done\)[^{]*\{(.*?)return;", merge, re.S)
     assert gave_up and gave_up.end() < merge.index("*(uint2*)(out +")
     assert 0 <= gave_up[1].index("barrier.cluster.arrive") < gave_up[1].index("barrier.cluster.wait")
+
+
+# The first arrival at a cluster's barrier is of the .aligned form, which a warp has to execute together: lane 0 has set up barriers alone just before
+@pytest.mark.parametrize("path", ["attention.cu", "common.cuh"])
+def test_first_cluster_arrival_follows_a_warp_barrier(path):
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, path)).read())
+    at = [m.start() for m in re.finditer(r'asm volatile\("barrier\.cluster\.arrive\.release\.aligned;"', text)]
+    assert len(at) == 1 and re.search(r"__syncwarp\(\);\s*$", text[:at[0]])
