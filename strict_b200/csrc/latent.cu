@@ -15,6 +15,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <climits>
 #include <mutex>
 
 #include "common.cuh"
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   __shared__ float corr_s[4][LHEADS], mx_s[2][4][LHEADS];  // [softmax warp], [tile parity][softmax warp]
   __shared__ float2 ml_s[LHEADS];
   __shared__ float fs[LHEADS][MAX_SPLITS];
-  __shared__ int len_s;
+  __shared__ int len_s, err_s;
   SB_TRACE_BEGIN();
   const int split = blockIdx.x, h0 = blockIdx.y * LHEADS, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -562,6 +563,7 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
   const uint32_t sK = smem_u32(smem), sQ = sK + (uint32_t)(a.stages * stage_bytes), sP = sQ + (uint32_t)(n_atoms * Q_ATOM);
   const uint32_t tmem_cols = n_mb <= 2 ? 256u : 512u;  // two S^T tiles of 32 columns, then 64 columns per block of latents
   if (threadIdx.x == 0) {
+    err_s = INT_MAX;
     for (int i = 0; i < a.stages; i++) {
       for (int g = 0; g < GROUPS; g++) mbar_init(smem_u32(&k_full[i][g]), 1);
       mbar_init(smem_u32(&k_empty[i]), 1);
@@ -884,7 +886,8 @@ __global__ void __launch_bounds__(256) latent_attn_decode_kernel(const __grid_co
     }
     *(uint2*)(a.out + ((int64_t)b * a.H + h0 + first + h) * a.rank_p + c) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
   }
-  if (err) { *(volatile int*)a.status = err; __threadfence_system(); }
+  // Of the block's codes the smallest stays, that of the wait nearest to the cause: 26 and 27 are what those report that waited for it.
+  if (err && atomicMin(&err_s, err) > err) { *(volatile int*)a.status = err; __threadfence_system(); }
   __syncwarp();
   cluster_wait();  // nobody leaves while another block may still read its shared memory
   SB_TRACE_END(SB_K_ATTN, 0);

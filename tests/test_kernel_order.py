@@ -185,3 +185,10 @@ def test_first_cluster_arrival_follows_a_warp_barrier(path):
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, path)).read())
     at = [m.start() for m in re.finditer(r'asm volatile\("barrier\.cluster\.arrive\.release\.aligned;"', text)]
     assert len(at) == 1 and re.search(r"__syncwarp\(\);\s*$", text[:at[0]])
+
+
+# an expired wait is reported by the code nearest to its cause, not by that of whoever waited for the one that gave up
+def test_latent_decode_reports_the_code_nearest_to_the_cause():
+    body = KERNELS["latent_attn_decode_kernel"][2]
+    assert "if (err && atomicMin(&err_s, err) > err) { *(volatile int*)a.status = err;" in body and body.count("a.status") == 1
+    assert body.index("err_s = INT_MAX") < body.index("__syncthreads()")
