@@ -295,6 +295,7 @@ int strictb200_free(strictb200_ctx* ctx, void* d_ptr) {
   if (!d_ptr) return STRICTB200_OK;
   SB_CUDA(cudaStreamSynchronize(ctx->stream));
   SB_CUDA(cudaFree(d_ptr));
+  ctx->planes_refused = SIZE_MAX;
   return STRICTB200_OK;
 }
 int strictb200_memset(strictb200_ctx* ctx, void* d_ptr, int byte, size_t bytes) {

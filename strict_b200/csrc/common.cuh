@@ -114,6 +114,7 @@ struct strictb200_ctx {
   // bf16 planes of the operands of a large fp32 product (gemm_f32_pair.cu), grow-only and bounded
   void* planes = nullptr;
   size_t planes_bytes = 0;
+  size_t planes_refused = SIZE_MAX;  // a size that could not be had, until something is freed
   uint64_t ws_generation = 0;  // advanced whenever a scratch buffer is re-allocated (recorded sequences check it)
 };
 

@@ -306,15 +306,23 @@ int planes_map(CUtensorMap* map, const bf16* base, int64_t rows, int64_t K, int6
 constexpr int64_t MIN_TILES = 44;                // fewer leave most pairs idle; below
 constexpr size_t PLANES_MAX = (size_t)1 << 30;  // scratch a context keeps for the planes at most
 constexpr int64_t ROWS_MAX = 32768;             // rows of X per pass
-// Grow-only scratch of its own. Nothing that was recorded refers to it (below), so it may move.
+// Grow-only scratch of its own. Nothing that was recorded refers to it (below), so it may move. A larger one is had before the smaller one goes, and a size
+// that could not be had is not asked for again until the context has freed something: neither costs the products behind it their scratch or a wait each.
 bool planes_scratch(strictb200_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->planes_bytes) return true;
-  if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
-  if (ctx->planes) cudaFree(ctx->planes);
-  ctx->planes = nullptr;
-  ctx->planes_bytes = 0;
-  const size_t want = std::min(bytes + (bytes >> 2), PLANES_MAX);
-  if (cudaMalloc(&ctx->planes, want) != cudaSuccess) { cudaGetLastError(); return false; }
+  if (bytes >= ctx->planes_refused) return false;
+  void* larger = nullptr;
+  size_t want = std::min(bytes + (bytes >> 2), PLANES_MAX);
+  if (cudaMalloc(&larger, want) != cudaSuccess && cudaMalloc(&larger, want = bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->planes_refused = bytes;
+    return false;
+  }
+  if (ctx->planes) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->planes);
+  }
+  ctx->planes = larger;
   ctx->planes_bytes = want;
   return true;
 }

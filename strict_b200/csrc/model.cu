@@ -876,6 +876,7 @@ int strictb200_model_destroy(strictb200_model* m) {
   cudaStreamSynchronize(m->ctx->stream);
   for (void* p : m->allocs) cudaFree(p);
   sb_stack_destroy(m);
+  m->ctx->planes_refused = SIZE_MAX;
   delete m;
   return STRICTB200_OK;
 }
@@ -1063,6 +1064,7 @@ int strictb200_kv_destroy(strictb200_kv* kv) {
   cudaStreamSynchronize(kv->m->ctx->stream);
   if (kv->graph) cudaGraphExecDestroy(kv->graph);
   for (void* p : kv->allocs) cudaFree(p);
+  kv->m->ctx->planes_refused = SIZE_MAX;
   delete kv;
   return STRICTB200_OK;
 }

@@ -192,3 +192,15 @@ def test_latent_decode_reports_the_code_nearest_to_the_cause():
     body = KERNELS["latent_attn_decode_kernel"][2]
     assert "if (err && atomicMin(&err_s, err) > err) { *(volatile int*)a.status = err;" in body and body.count("a.status") == 1
     assert body.index("err_s = INT_MAX") < body.index("__syncthreads()")
+
+
+# The scratch of the fp32 products on SM pairs: the smaller one goes when the larger one is there, and what could not be had is not asked for by every product
+def test_scratch_of_fp32_products_survives_a_refusal():
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "gemm_f32_pair.cu")).read())
+    body = text[text.index("bool planes_scratch("):]
+    body = body[:body.index("\n}")]
+    assert body.index("planes_refused) return false") < body.index("cudaMalloc(") < body.index("ctx->planes_refused = bytes") < body.index("cudaStreamSynchronize(") < body.index("cudaFree(ctx->planes)")
+    for path, call in (("api.cu", "int strictb200_free("), ("model.cu", "int strictb200_kv_destroy("), ("model.cu", "int strictb200_model_destroy(")):
+        text = open(os.path.join(CSRC, path)).read()
+        body = text[text.index(call):]
+        assert "planes_refused = SIZE_MAX" in body[:body.index("\n}")]
