@@ -89,6 +89,19 @@ int sb_check_status(strictb200_ctx* ctx, const char* what) {
                                              "); the results of this call are not valid");
 }
 
+cudaError_t sb_malloc(strictb200_ctx* ctx, void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->planes) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->planes);
+    ctx->planes = nullptr;
+    ctx->planes_bytes = 0;
+    e = cudaMalloc(out, bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();  // reported by this call's status, not by the next launch's
+  return e;
+}
+
 int sb_ws(strictb200_ctx* ctx, size_t bytes, void** out) {
   if (bytes > ctx->ws_bytes) {
     ctx->ws_generation++;
@@ -97,7 +110,7 @@ int sb_ws(strictb200_ctx* ctx, size_t bytes, void** out) {
     ctx->ws = nullptr;
     ctx->ws_bytes = 0;
     size_t want = bytes + (bytes >> 2) + (1 << 20);
-    SB_CUDA(cudaMalloc(&ctx->ws, want));
+    SB_CUDA(sb_malloc(ctx, &ctx->ws, want));
     ctx->ws_bytes = want;
   }
   *out = ctx->ws;
@@ -112,7 +125,7 @@ int sb_ws2(strictb200_ctx* ctx, size_t bytes, void** out) {
     ctx->ws2 = nullptr;
     ctx->ws2_bytes = 0;
     size_t want = bytes + (bytes >> 2) + (1 << 20);
-    SB_CUDA(cudaMalloc(&ctx->ws2, want));
+    SB_CUDA(sb_malloc(ctx, &ctx->ws2, want));
     ctx->ws2_bytes = want;
   }
   *out = ctx->ws2;
@@ -145,8 +158,8 @@ int strictb200_trace_begin(strictb200_ctx* ctx, int capacity) {
   SB_REQUIRE(capacity > 0 && capacity <= (1 << 24), "capacity must be between 1 and 2^24 records");
   SB_REQUIRE(!ctx->trace_rec, "a trace is already armed on this context");
   SB_TRY(sb_sync(ctx, "trace_begin"));
-  SB_CUDA(cudaMalloc(&ctx->trace_rec, (size_t)capacity * 64));
-  SB_CUDA(cudaMalloc(&ctx->trace_count, 256));
+  SB_CUDA(sb_malloc(ctx, (void**)&ctx->trace_rec, (size_t)capacity * 64));
+  SB_CUDA(sb_malloc(ctx, (void**)&ctx->trace_count, 256));
   SB_CUDA(cudaMemset(ctx->trace_count, 0, 256));
   ctx->trace_capacity = (unsigned)capacity;
   if (trace_set_all(SbTraceDev{ctx->trace_rec, ctx->trace_count, ctx->trace_capacity})) return sb_fail(STRICTB200_ERR_CUDA, "trace: cannot set the device variables");
@@ -287,7 +300,7 @@ int strictb200_malloc(strictb200_ctx* ctx, size_t bytes, void** d_out) {
   SB_REQUIRE(d_out, "null out pointer");
   *d_out = nullptr;
   if (bytes == 0) return STRICTB200_OK;
-  SB_CUDA(cudaMalloc(d_out, bytes));
+  SB_CUDA(sb_malloc(ctx, d_out, bytes));
   return STRICTB200_OK;
 }
 int strictb200_free(strictb200_ctx* ctx, void* d_ptr) {
@@ -393,7 +406,7 @@ int strictb200_flush_l2(strictb200_ctx* ctx) {
   SB_ENTER(ctx);
   if (!ctx->flush_buf) {
     ctx->flush_bytes = (size_t)256 << 20;  // 2x the 126 MB L2
-    SB_CUDA(cudaMalloc(&ctx->flush_buf, ctx->flush_bytes));
+    SB_CUDA(sb_malloc(ctx, &ctx->flush_buf, ctx->flush_bytes));
   }
   flush_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>((uint4*)ctx->flush_buf, ctx->flush_bytes / 16);
   SB_LAUNCHED(ctx);

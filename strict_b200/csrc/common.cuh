@@ -126,6 +126,8 @@ int sb_fail(int code, const std::string& msg);
 // ERR_NCCL / ERR_TIMEOUT instead of hanging.
 int sb_sync(strictb200_ctx* ctx, const char* what);
 int sb_check_status(strictb200_ctx* ctx, const char* what);  // after a stream synchronise: ERR_TIMEOUT if a kernel's wait expired
+// cudaMalloc that gives the planes of the fp32 products back before it fails: what a caller may allocate is not less for scratch that is only kept.
+cudaError_t sb_malloc(strictb200_ctx* ctx, void** out, size_t bytes);
 int sb_ws(strictb200_ctx* ctx, size_t bytes, void** out);  // grow-only context scratch
 int sb_ws2(strictb200_ctx* ctx, size_t bytes, void** out);  // a second one, for calls that already hold the first
 

@@ -383,7 +383,7 @@ int gemm_workspace(strictb200_ctx* ctx, size_t count_bytes, size_t part_bytes, i
     size_t cb = count_bytes > ctx->gemm_count_bytes ? count_bytes * 2 : ctx->gemm_count_bytes;
     size_t pb = part_bytes > ctx->gemm_part_bytes ? part_bytes : ctx->gemm_part_bytes;
     ctx->gemm_count_bytes = ctx->gemm_part_bytes = 0;
-    SB_CUDA(cudaMalloc(&ctx->gemm_ws, cb + pb));
+    SB_CUDA(sb_malloc(ctx, &ctx->gemm_ws, cb + pb));
     SB_CUDA(cudaMemsetAsync(ctx->gemm_ws, 0, cb, ctx->stream));
     ctx->gemm_count_bytes = cb;
     ctx->gemm_part_bytes = pb;

@@ -943,7 +943,7 @@ int strictb200_model_set_tensor(strictb200_model* m, const char* name, const voi
       // fp32 host rows -> bf16 device rows through a staging buffer
       float* tmp;
       size_t n = (size_t)s.n_rows[i] * s.ncols;
-      SB_CUDA(cudaMalloc((void**)&tmp, n * 4));
+      SB_CUDA(sb_malloc(ctx, (void**)&tmp, n * 4));
       cudaError_t e = cudaMemcpy2DAsync(tmp, s.ncols * 4, (const char*)h_data + ((size_t)s.src_row[i] * s.cols + s.col0) * 4, s.cols * 4,
                                         s.ncols * 4, s.n_rows[i], cudaMemcpyHostToDevice, ctx->stream);
       int st = e == cudaSuccess ? k_f32_to_bf16(ctx, tmp, n, (bf16*)s.dev + (size_t)s.dst_row[i] * s.ncols) : STRICTB200_ERR_CUDA;
@@ -978,7 +978,7 @@ int strictb200_model_get_tensor(strictb200_model* m, const char* name, void* h_d
   if (bytes != n * helem) return sb_fail(STRICTB200_ERR_INVALID_ARG, std::string("tensor ") + name + " holds " + std::to_string(n * helem) + " bytes");
   if (s.host_f32) {
     float* tmp;
-    SB_CUDA(cudaMalloc((void**)&tmp, n * 4));
+    SB_CUDA(sb_malloc(ctx, (void**)&tmp, n * 4));
     int st = k_bf16_to_f32(ctx, (const bf16*)s.dev, n, tmp);
     cudaError_t e = cudaMemcpyAsync(h_data, tmp, n * 4, cudaMemcpyDeviceToHost, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
@@ -1024,7 +1024,7 @@ int strictb200_kv_create(strictb200_model* m, int batch, int maxlen, strictb200_
   }
   auto fail = [&](int s) { strictb200_kv_destroy(kv); return s; };
   auto alloc = [&](void** p, size_t n) -> int {
-    SB_CUDA(cudaMalloc(p, n ? n : 1));
+    SB_CUDA(sb_malloc(ctx, p, n ? n : 1));
     kv->allocs.push_back(*p);
     return STRICTB200_OK;
   };
@@ -1188,7 +1188,7 @@ int strictb200_generate(strictb200_model* m, strictb200_kv* kv, const int32_t* h
   for (int b = 0; b < kv->B; b++) SB_REQUIRE(h_ids[b] >= 0 && h_ids[b] < m->c.vocab, "token id outside the vocabulary");
   if (kv->hist_cap < n_steps) {
     void* p;
-    SB_CUDA(cudaMalloc(&p, (size_t)n_steps * kv->B * 4));
+    SB_CUDA(sb_malloc(ctx, &p, (size_t)n_steps * kv->B * 4));
     kv->allocs.push_back(p);
     kv->d_hist = (int32_t*)p;
     kv->hist_cap = n_steps;

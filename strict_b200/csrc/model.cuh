@@ -81,7 +81,7 @@ inline int dalloc(strictb200_model* m, T** p, size_t count) {
   *p = nullptr;
   if (!count) return STRICTB200_OK;
   void* v;
-  SB_CUDA(cudaMalloc(&v, count * sizeof(T)));
+  SB_CUDA(sb_malloc(m->ctx, &v, count * sizeof(T)));
   m->allocs.push_back(v);
   *p = (T*)v;
   return STRICTB200_OK;
@@ -155,7 +155,7 @@ inline int prefill_scratch(strictb200_ctx* ctx, size_t bytes, char** out) {
     if (ctx->prefill_ws) SB_CUDA(cudaFree(ctx->prefill_ws));
     ctx->prefill_ws = nullptr;
     ctx->prefill_ws_bytes = 0;
-    SB_CUDA(cudaMalloc(&ctx->prefill_ws, bytes));
+    SB_CUDA(sb_malloc(ctx, &ctx->prefill_ws, bytes));
     ctx->prefill_ws_bytes = bytes;
   }
   *out = (char*)ctx->prefill_ws;

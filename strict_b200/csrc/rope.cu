@@ -282,8 +282,8 @@ int sb_rope_table(strictb200_ctx* ctx, int max_pos, int D, double theta, float**
       s[(size_t)p * h + i] = (float)(gain * std::sin(ang));
     }
   size_t bytes = c.size() * sizeof(float);
-  SB_CUDA(cudaMalloc((void**)d_cos, bytes));
-  SB_CUDA(cudaMalloc((void**)d_sin, bytes));
+  SB_CUDA(sb_malloc(ctx, (void**)d_cos, bytes));
+  SB_CUDA(sb_malloc(ctx, (void**)d_sin, bytes));
   SB_CUDA(cudaMemcpyAsync(*d_cos, c.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
   SB_CUDA(cudaMemcpyAsync(*d_sin, s.data(), bytes, cudaMemcpyHostToDevice, ctx->stream));
   SB_CUDA(cudaStreamSynchronize(ctx->stream));

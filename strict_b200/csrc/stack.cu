@@ -880,7 +880,7 @@ int sb_stack_tensor(strictb200_model* m, const char* name, const void* h_in, voi
     return STRICTB200_OK;
   }
   void* tmp;
-  SB_CUDA(cudaMalloc(&tmp, bytes));
+  SB_CUDA(sb_malloc(ctx, &tmp, bytes));
   int st = STRICTB200_OK;
   cudaError_t e = cudaSuccess;
   if (h_in) e = cudaMemcpyAsync(tmp, h_in, bytes, cudaMemcpyHostToDevice, ctx->stream);
@@ -902,7 +902,7 @@ int sb_stack_init_random(strictb200_model* m, uint64_t seed) {
     if (!find_slot(m, name, &s)) return STRICTB200_OK;  // a part this layer does not have
     const int64_t n = s.rows * s.cols;
     void* tmp;
-    SB_CUDA(cudaMalloc(&tmp, (size_t)n * 2));
+    SB_CUDA(sb_malloc(ctx, &tmp, (size_t)n * 2));
     int r = k_gen_normal_bf16(ctx, sb_stream_key(seed, id), 0, n, SD, (bf16*)tmp);
     if (r == STRICTB200_OK) r = place(ctx, s, tmp, false, false);
     cudaStreamSynchronize(ctx->stream);

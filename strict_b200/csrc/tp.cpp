@@ -224,9 +224,9 @@ int strictb200_tp_comm_handle(strictb200_ctx* ctx, void* h_handle64) {
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "IPC handle size");
   TpState* tp = ctx->tp;
   if (!tp->comm_buf) {
-    SB_CUDA(cudaMalloc(&tp->comm_buf, COMM_BYTES));
+    SB_CUDA(sb_malloc(ctx, &tp->comm_buf, COMM_BYTES));
     SB_CUDA(cudaMemset(tp->comm_buf, 0, COMM_BYTES));
-    SB_CUDA(cudaMalloc((void**)&tp->local, 256 + COMM_ROWS * sizeof(int)));
+    SB_CUDA(sb_malloc(ctx, (void**)&tp->local, 256 + COMM_ROWS * sizeof(int)));
     SB_CUDA(cudaMemset(tp->local, 0, 256 + COMM_ROWS * sizeof(int)));
   }
   cudaIpcMemHandle_t h;
@@ -260,11 +260,11 @@ int strictb200_tp_comm_open_absent_peers(strictb200_ctx* ctx, int world) {
   ctx->tp_world = world;
   ctx->tp_rank = 0;
   for (int r = 0; r < world; r++) {
-    SB_CUDA(cudaMalloc(&tp->peer_buf[r], COMM_BYTES));
+    SB_CUDA(sb_malloc(ctx, &tp->peer_buf[r], COMM_BYTES));
     SB_CUDA(cudaMemset(tp->peer_buf[r], 0, COMM_BYTES));
   }
   tp->comm_buf = tp->peer_buf[0];
-  SB_CUDA(cudaMalloc((void**)&tp->local, 256 + COMM_ROWS * sizeof(int)));
+  SB_CUDA(sb_malloc(ctx, (void**)&tp->local, 256 + COMM_ROWS * sizeof(int)));
   SB_CUDA(cudaMemset(tp->local, 0, 256 + COMM_ROWS * sizeof(int)));
   fill_comm_dev(ctx);
   return STRICTB200_OK;

@@ -289,3 +289,20 @@ def test_latent_attention_takes_a_length_that_changes(ctx, oracle, rng, lens, in
         f(ctx.h, C.addressof(s), dq.p, dk.p, dl.p, B, maxlen, chunk, nsplit, scratch.p, dw.p, out.p, H * vdim)))
     for v in (dq, dk, dw, scratch):
         v.free()
+
+
+# the scratch that the products on SM pairs keep is given back before an allocation through the context is refused, and had again by the next product
+def test_scratch_is_given_back_before_an_allocation_fails(ctx, rng):
+    import torch
+    x, w = rng.standard_normal((2000, 1024)).astype(np.float32), rng.standard_normal((4096, 1024)).astype(np.float32)
+    planes = 3 * 2 * (2000 + 4096) * 1024
+    clean = _gemm_f32(ctx, x, w, np.zeros((2000, 4096), np.float32))
+    ctx.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    p = C.c_void_p()
+    assert L().strictb200_malloc(ctx.h, C.c_size_t(1 << 50), C.byref(p)) != 0 and not p.value
+    given = torch.cuda.mem_get_info()[0]
+    assert given >= before + planes
+    assert np.array_equal(_gemm_f32(ctx, x, w, np.zeros((2000, 4096), np.float32)), clean)
+    ctx.synchronize()
+    assert torch.cuda.mem_get_info()[0] <= given - planes
