@@ -795,6 +795,8 @@ SB_TRACE_TU(attention)
 // full cache): a cache that holds 2100 of 2432 keys in chunks of 512 runs four full chunks and a
 // stub per sequence, chunks of 448 run five even ones (14 % less attention time, measured). The
 // attn_blocks_per_sm option restores the plain "that many blocks per SM" rule. `fused`: the kernel with the RoPE prologue will run.
+// (The form that merges its chunks in a cluster holds as many blocks on an SM up to 11 query heads per KV head and two from 12 on; a step of that form has then at
+// most 2 KV heads and 16 sequences, 256 blocks, which are one wave either way.)
 static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool fused = false, bool short_chunks = true) {
   const int per_sm = ctx->opt.attn_blocks_per_sm;
   const int tiles = (maxlen + KT - 1) / KT;

@@ -306,3 +306,19 @@ def test_scratch_is_given_back_before_an_allocation_fails(ctx, rng):
     assert np.array_equal(_gemm_f32(ctx, x, w, np.zeros((2000, 4096), np.float32)), clean)
     ctx.synchronize()
     assert torch.cuda.mem_get_info()[0] <= given - planes
+
+
+# key chunks merged in a cluster for KV heads with more than 8 query heads: 9, and the 16 that are the most
+@pytest.mark.parametrize("heads,B", [(18, 2), (32, 16)])
+def test_many_heads_merged_in_a_cluster_vs_oracle(ctx, oracle, heads, B):
+    cfg = dict(TINY_QWEN, n_layers=1, vocab=512, n_q_heads=heads, n_kv_heads=2, d_model=256, max_pos=512)
+    m, om, kv, st, _, logits, want = _run_pair(ctx, oracle, cfg, 8, B, 200, [200 - 11 * i for i in range(B)], 4, random_gains=True)
+    for _ in range(2):
+        ids = oracle.argmax(want)
+        _, logits = kv.decode_step(ids, want_logits=True)
+        want = st.decode(ids)
+        ok, mx, rel = logits_close(logits, want, **TOL_FP8)
+        assert ok, (mx, rel)
+    for o in (kv, m):
+        o.dispose()
+    st.close(), om.close()
