@@ -395,7 +395,7 @@ int k_attn_f32(strictb200_ctx* ctx, const float* qkv, float* kc, float* vc, cons
     ctx->launches++;
     // Blocks of 16 queries while those of 32 would all be resident (four per SM): 1 x 901 tokens 3.80 -> 3.60 ms for a GPT-2 prompt, 4 x 300 the same; with
     // more blocks those of 32 read the keys half as often (8 x 600: 9.05 ms against 9.41, and 9.17 with 64).
-    if ((int64_t)((prompts->max_new + 31) / 32) * H * prompts->nb <= 4 * 148) return launch_prompt<64>(ctx, prompts, qkv, kc, vc, H, maxlen, scale, out);
+    if ((int64_t)((prompts->max_new + 31) / 32) * H * prompts->nb <= 4 * (int64_t)ctx->sm_count) return launch_prompt<64>(ctx, prompts, qkv, kc, vc, H, maxlen, scale, out);
     return launch_prompt<128>(ctx, prompts, qkv, kc, vc, H, maxlen, scale, out);
   }
   const int threads = 256;

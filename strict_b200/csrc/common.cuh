@@ -83,9 +83,11 @@ struct SbDeviceOnce {
   }
 };
 
+constexpr int SB_SMS = 148;  // of a B200; the rules that are told no context draw their lines for it
+
 struct strictb200_ctx {
   int device = 0;
-  int sm_count = 148;
+  int sm_count = SB_SMS;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   uint64_t launches = 0;

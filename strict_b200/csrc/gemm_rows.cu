@@ -291,7 +291,7 @@ SB_TRACE_TU(gemm_rows)
 // A decode step of Qwen3-0.6B: 774 -> 711 us (batch 1).
 bool sb_gemm_rows_takes(int64_t M, int64_t N, int64_t K, bool f8, bool finished) {
   if (M > 16 || K % (f8 ? 16 : 8)) return false;
-  constexpr int64_t one_round = 2 * 148 * TILE;  // channels whose blocks are resident at once
+  constexpr int64_t one_round = 2 * SB_SMS * TILE;  // channels whose blocks are resident at once
   const int64_t weights = N * K;
   const bool short_rounds = M <= 8 ? N <= one_round || (N <= 2 * one_round && (!f8 || K >= 512))
                                    : f8 ? N * std::min<int64_t>((K + 1023) / 1024, 8) <= one_round : N <= one_round || (N <= 2 * one_round && K >= 768);

@@ -285,9 +285,9 @@ SB_TRACE_TU(gemm_rows_chain)
 // registers, so that the next kernel's blocks wait (8192 to 14336 channels of 1024: 7 to 12 us with the norm in front, 6.9 as two launches; 1024
 // channels of 5120: 5.3 us in whole blocks against 2.3 in K splits).
 // Rows of at most 1024 columns, and channels whose blocks are all resident at once.
-bool sb_norm_rows_takes(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= 16 && K <= MAX_D && K % 128 == 0 && N <= 2 * 148 * TILE; }
+bool sb_norm_rows_takes(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= 16 && K <= MAX_D && K % 128 == 0 && N <= 2 * SB_SMS * TILE; }
 // Columns whose weights eight warps hold, and channels that are one round of blocks.
-bool sb_residual_rows_takes(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= 16 && N <= 8 * 148 && K % 16 == 0 && K <= 8 * WARPS * STEP; }
+bool sb_residual_rows_takes(int64_t M, int64_t N, int64_t K) { return M >= 1 && M <= 16 && N <= 8 * SB_SMS && K % 16 == 0 && K <= 8 * WARPS * STEP; }
 
 int k_norm_rows(strictb200_ctx* ctx, const NormRowsGemm& g) {
   if (!sb_norm_rows_takes(g.M, g.N, g.K) || (g.out_glu && g.N % 2)) return sb_fail(STRICTB200_ERR_UNSUPPORTED, "norm_rows: shape");

@@ -54,11 +54,11 @@ bool fuses_rope(strictb200_model* m, int64_t B, int s1) {
 }
 
 // A step of few sequences of a narrow model: norms in front of the products, sums straight into the residual, key chunks merged inside
-// their cluster (gemm_rows_chain.cu): 5 launches per layer instead of 8.
+// their cluster (gemm_rows_chain.cu): 5 launches per layer instead of 8. On a part with fewer SMs the blocks of its products would not all be resident.
 bool chained_step(strictb200_model* m, int64_t B) {
   const auto& c = m->c;
   const int64_t d = c.d_model, nq = (int64_t)m->Hq_l * c.head_dim, nqkv = nq + 2 * (int64_t)m->Hkv_l * c.head_dim;
-  return m->world == 1 && m->I_l % 16 == 0 && m->Hq_l / m->Hkv_l <= 16 && sb_norm_rows_takes(B, nqkv, d) && sb_norm_rows_takes(B, 2 * (int64_t)m->I_l, d) &&
+  return m->ctx->sm_count >= SB_SMS && m->world == 1 && m->I_l % 16 == 0 && m->Hq_l / m->Hkv_l <= 16 && sb_norm_rows_takes(B, nqkv, d) && sb_norm_rows_takes(B, 2 * (int64_t)m->I_l, d) &&
          sb_residual_rows_takes(B, d, nq) && sb_residual_rows_takes(B, d, m->I_l);
 }
 

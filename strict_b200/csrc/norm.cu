@@ -840,7 +840,7 @@ int k_rownorm(strictb200_ctx* ctx, const RowNormArgs& a, int64_t M, int64_t d) {
 }
 int k_layernorm(strictb200_ctx* ctx, const float* x, const float* g, const float* b, float eps, int64_t M, int64_t d, float* y) {
   // from two blocks per SM on; fewer rows are quicker with a block each, which has eight times the loads of a row in flight
-  if (M >= 2 * 148 * (ROW_THREADS / 32) && d <= 1024 && d % 4 == 0 && (((uintptr_t)x | (uintptr_t)g | (uintptr_t)b | (uintptr_t)y) & 15) == 0) {
+  if (M >= 2 * (int64_t)ctx->sm_count * (ROW_THREADS / 32) && d <= 1024 && d % 4 == 0 && (((uintptr_t)x | (uintptr_t)g | (uintptr_t)b | (uintptr_t)y) & 15) == 0) {
     SB_CUDA(sb_launch(ctx, layernorm_rows_kernel, dim3((unsigned)((M + ROW_THREADS / 32 - 1) / (ROW_THREADS / 32))), dim3(ROW_THREADS), 0, x, g, b, eps, M, (int)d, y));
     ctx->launches++;
     return STRICTB200_OK;

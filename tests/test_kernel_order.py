@@ -204,3 +204,13 @@ def test_scratch_of_fp32_products_survives_a_refusal():
         text = open(os.path.join(CSRC, path)).read()
         body = text[text.index(call):]
         assert "planes_refused = SIZE_MAX" in body[:body.index("\n}")]
+
+
+# rules ask the context for its SMs; the few that are told no context share one constant, and what they choose is taken on a part with that many only
+def test_rules_do_not_assume_a_number_of_sms():
+    for path in glob.glob(os.path.join(CSRC, "*.c*")):
+        code = re.sub(r"//[^\n]*", "", open(path).read()).replace("constexpr int SB_SMS = 148;", "")
+        assert not re.search(r"\b148\b", code), path
+    text = open(os.path.join(CSRC, "model.cu")).read()
+    body = text[text.index("bool chained_step("):]
+    assert "sm_count >= SB_SMS" in body[:body.index("\n}")]
