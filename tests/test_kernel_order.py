@@ -214,3 +214,22 @@ def test_rules_do_not_assume_a_number_of_sms():
     text = open(os.path.join(CSRC, "model.cu")).read()
     body = text[text.index("bool chained_step("):]
     assert "sm_count >= SB_SMS" in body[:body.index("\n}")]
+
+
+# the structures that tests hand to internal functions are those of the library: names, order and types of the members
+@pytest.mark.parametrize("name", ["GemmF32Args", "LatentShape"])
+def test_structures_of_the_tests_match_the_library(name):
+    import ctypes as C
+    import test_gpu_chained_rows as t
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "common.cuh")).read())
+    body = text[text.index("struct %s {" % name):]
+    body = body[body.index("{") + 1:body.index("};")]
+    types = {"int64_t": C.c_int64, "int": C.c_int, "float": C.c_float}
+    members = []
+    for line in body.split(";"):
+        m = re.match(r"(?:const )?(\w+)([ *].*)", line.strip(), re.S)
+        if not m or "(" in line:
+            continue
+        for part in m[2].split(","):
+            members.append((re.search(r"\w+", part)[0], C.c_void_p if "*" in part else types[m[1]]))
+    assert members == t.__dict__[name]._fields_
