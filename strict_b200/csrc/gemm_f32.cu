@@ -252,6 +252,7 @@ int k_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float
 int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   const int64_t M = g.M, N = g.N, K = g.K;
   if (K % 4 || g.ldx % 4 || g.ldw % 4) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: K and the row strides must be multiples of 4");
+  if (((uintptr_t)g.x | (uintptr_t)g.w | (uintptr_t)g.ln_gain | (uintptr_t)g.ln_bias) % 16) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: operands must be 16-byte aligned");
   if (g.ln_gain && !sb_gemm_f32_takes_norm(M, K)) return sb_fail(STRICTB200_ERR_INVALID_ARG, "gemm_f32: rows for the layer norm in front are at most 8 of 1024");
   // One pass over the weights per eight rows (this kernel) or per 32 to 128 (the tensor cores). Measured, us, rows = 9 / 16 / 32 / 128 / 4700:
   //   N 768  K 768    7.1 / 7.1 / 13.0 /  37.8 / 1197   against   8.5 / 8.5 /  8.7 / 13.9 /  62
@@ -261,7 +262,7 @@ int k_gemm_f32(strictb200_ctx* ctx, const GemmF32Args& g) {
   // Errors against 64 bits (2-norm, normal operands, K 768 / 3072 / 14336): 9.2e-8 / 1.0e-7 / 1.6e-7 here, 7.6e-8..8.7e-8 /
   // 9.6e-8 / 1.3e-7 there.
   const bool few = M <= 4 || (M <= F32_MT && (g.ln_gain || N * K <= (8 << 20))) || (M <= 2 * F32_MT && N * K <= (1 << 20));
-  if (!few && ((uintptr_t)g.x | (uintptr_t)g.w) % 16 == 0) {
+  if (!few) {
     const int st = k_gemm_f32_pair(ctx, g);
     return st == STRICTB200_ERR_UNSUPPORTED ? k_gemm_f32_tc(ctx, g) : st;
   }

@@ -233,3 +233,17 @@ def test_structures_of_the_tests_match_the_library(name):
         for part in m[2].split(","):
             members.append((re.search(r"\w+", part)[0], C.c_void_p if "*" in part else types[m[1]]))
     assert members == t.__dict__[name]._fields_
+
+
+# every kernel behind this entry reads its operands 16 bytes at a time: others are refused on the host
+@pytest.mark.parametrize("M,off_x,off_w", [(1, 4, 0), (4, 0, 8), (300, 12, 0), (3000, 0, 4)])
+def test_fp32_operands_that_are_not_aligned_are_refused(M, off_x, off_w):
+    import ctypes as C
+    from strict_b200 import native
+    here = C.create_string_buffer(4096 + 16)  # stands for a context and for data: a refused call reads neither
+    p = (C.addressof(here) + 15) // 16 * 16
+    import test_gpu_chained_rows as t
+    f = native.lib()._Z10k_gemm_f32P14strictb200_ctxRK11GemmF32Args
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_void_p]
+    a = t.GemmF32Args(M=M, N=3072, K=768, x=p + off_x, ldx=768, w=p + off_w, ldw=768, y=p, ldy=3072, alpha=1)
+    assert f(p, C.addressof(a)) == native.ERR_INVALID_ARG
