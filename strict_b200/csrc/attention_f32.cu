@@ -27,8 +27,10 @@ __global__ void kv_append_f32_kernel(const float* qkv, float* __restrict__ kc, f
 // 19.5 with a thread per column.
 __global__ void __launch_bounds__(256) kv_append_f32_vec_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc, const int32_t* seq, const int32_t* pos,
                                                                 const int32_t* lens, uint32_t n, uint32_t hd, uint32_t Dh, int H, int maxlen) {
-  pdl_trigger();
+  // The attention behind this may start only when the product in front has left: its blocks, which all wait for the keys anyway, were dealt out over the
+  // SMs that product had left free, the longest rows on top of each other. GPT-2 prompts of width 128, 3 x 500: 869 -> 790 us, 1 x 900: 1026 -> 892.
   pdl_wait();
+  pdl_trigger();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x, per = hd / 4;
   if (i >= n) return;
   const uint32_t t = i / per, e = (i - t * per) * 4, h = e / Dh;

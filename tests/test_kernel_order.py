@@ -247,3 +247,9 @@ def test_fp32_operands_that_are_not_aligned_are_refused(M, off_x, off_w):
     f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_void_p]
     a = t.GemmF32Args(M=M, N=3072, K=768, x=p + off_x, ldx=768, w=p + off_w, ldw=768, y=p, ldy=3072, alpha=1)
     assert f(p, C.addressof(a)) == native.ERR_INVALID_ARG
+
+
+# the blocks of fp32 prompt attention are dealt out when the product in front of the cache append has left its SMs
+def test_cache_append_of_prompts_triggers_after_its_wait():
+    body = KERNELS["kv_append_f32_vec_kernel"][2]
+    assert 0 <= body.index("pdl_wait()") < body.index("pdl_trigger()")
