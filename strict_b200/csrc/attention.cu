@@ -788,16 +788,53 @@ int k_attn_prefill(strictb200_ctx* ctx, const bf16* q, const bf16* kc, const bf1
 
 SB_TRACE_TU(attention)
 
+static int merge_set_up(strictb200_ctx* ctx) {
+  static SbDeviceOnce once;
+  SB_CUDA(once.run(ctx->device, [&] {
+    const int most = (int)(2 * DEC_STAGES * KT * 256 + merge_bytes(16, D));
+    const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e == cudaSuccess ? cudaFuncSetAttribute(attn_decode_kernel<D, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) : e;
+  }));
+  return STRICTB200_OK;
+}
+// Clusters of `size` blocks of the merging form that run at once. A cluster needs its blocks' places in one part of the GPU, and of more than four blocks the calculator's
+// number did not all start together: 48 of 48 clusters of eight, 56 of 56 of seven, 80 of 82 of five, 64 of 71 of six and 30 of 33 of eight (with 16 heads) left
+// some for a second wave, 40 of 48, 48 of 71, 64 of 82 and 28 of 33 did not; 96 of 104 clusters of four and 128 of 142 of three neither.
+static int64_t merge_clusters(strictb200_ctx* ctx, bool fused, int heads, int size) {
+  static std::mutex mu;
+  static int known[64][2][17][MERGE_MAX + 1] = {};
+  std::lock_guard<std::mutex> lock(mu);
+  int& n = known[ctx->device & 63][fused][std::min(heads, 16)][std::min(size, MERGE_MAX)];
+  if (!n) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = 2 * DEC_STAGES * KT * 256 + merge_bytes(heads, D);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaErrorUnknown;
+    if (merge_set_up(ctx) == STRICTB200_OK)
+      e = fused ? cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel<D, true, true>, &cfg) : cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel<D, false, true>, &cfg);
+    if (e != cudaSuccess || n < 1) { cudaGetLastError(); n = 1; }
+    if (size > 4) n = std::max(1, n - n / 8);
+  }
+  return n;
+}
+
 // Keys per block. All blocks of a launch take about the same time, so the grid runs in waves of
 // (blocks resident per SM) x (SM count): the chunk is the multiple of the tile size that
 // minimises waves x (tiles per chunk + per-block overhead) among the chunk sizes that leave at
 // most 8 chunks for a full cache. The waves are counted for sequences of `len_plan` keys (0: a
 // full cache): a cache that holds 2100 of 2432 keys in chunks of 512 runs four full chunks and a
 // stub per sequence, chunks of 448 run five even ones (14 % less attention time, measured). The
-// attn_blocks_per_sm option restores the plain "that many blocks per SM" rule. `fused`: the kernel with the RoPE prologue will run.
-// (The form that merges its chunks in a cluster holds as many blocks on an SM up to 11 query heads per KV head and two from 12 on; a step of that form has then at
-// most 2 KV heads and 16 sequences, 256 blocks, which are one wave either way.)
-static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool fused = false, bool short_chunks = true) {
+// attn_blocks_per_sm option restores the plain "that many blocks per SM" rule. `fused`: the kernel with the RoPE prologue will run;
+// `merge_heads`: the form that merges its chunks in a cluster, with that many query heads per KV head (0: not that one). Its waves are clusters (blocks without keys
+// leave at once and are not counted). Planned by blocks, 10 sequences of 2000 keys with 8 KV heads ran 80 clusters of five in two waves: 27.0 us; 80 of four: 17.3.
+static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool fused = false, bool short_chunks = true, int merge_heads = 0) {
   const int per_sm = ctx->opt.attn_blocks_per_sm;
   const int tiles = (maxlen + KT - 1) / KT;
   const int tiles_plan = len_plan > 0 && len_plan < maxlen ? (len_plan + KT - 1) / KT : tiles;
@@ -825,6 +862,12 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
   const int res0 = (fused ? resident_fused_of : resident_of)[ctx->device & 63];
   const int resident = res0 > 0 ? res0 : 1;
   const int64_t slots = (int64_t)ctx->sm_count * resident, pairs = (int64_t)B * Hkv;
+  auto waves_of = [&](int c) -> int64_t {
+    const int chunks = (tiles_plan + c - 1) / c;
+    if (!merge_heads) return (pairs * chunks + slots - 1) / slots;
+    const int64_t at_once = merge_clusters(ctx, fused, merge_heads, chunks);
+    return (pairs + at_once - 1) / at_once;
+  };
   int best = tiles;
   double best_cost = 1e30;
   // At most 8 chunks per sequence: that is what the fast merge kernel takes. 16 chunks for the few
@@ -834,10 +877,10 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
   // walked four tiles one after the other on some SMs and one on others, 8.7 us; chunks of 128, 5.7 us). In several waves short chunks gain nothing and
   // multiply the partial results (`short_chunks` false: never).
   for (int c = (tiles + 7) / 8; c <= tiles; c++) {
-    if (c < 4 && c < tiles && (!short_chunks || pairs * ((tiles_plan + c - 1) / c) > slots)) continue;
+    const int64_t waves = waves_of(c);
+    if (c < 4 && c < tiles && (!short_chunks || waves > 1)) continue;
     // (counting a stub as a whole block is deliberate: weighting blocks by their length made the rule pick three long
     // chunks where five short ones measured 47 us against 66)
-    const int64_t blocks = pairs * ((tiles_plan + c - 1) / c), waves = (blocks + slots - 1) / slots;
     const double cost = (double)waves * ((double)std::min(c, tiles_plan) + 1.5);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = c; }
   }
@@ -845,7 +888,9 @@ static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len
 }
 static int splits_of(int maxlen, int chunk) { return (maxlen + chunk - 1) / chunk; }
 int sb_attn_decode_splits(strictb200_ctx* ctx, int B, int Hkv, int maxlen) { return splits_of(maxlen, decode_chunk(ctx, B, Hkv, maxlen)); }
-int sb_attn_decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan, bool fused) { return decode_chunk(ctx, B, Hkv, maxlen, len_plan, fused); }
+int sb_attn_decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan, bool fused, int merge_heads) {
+  return decode_chunk(ctx, B, Hkv, maxlen, len_plan, fused, true, merge_heads);
+}
 size_t sb_attn_decode_scratch(int B, int Hq, int Dh, int nsplit) { return (size_t)B * Hq * nsplit * (Dh + 2) * sizeof(float); }
 
 // The key chunks alone, for a merge of the caller's: rows of HD = 64 or 128 dims, len_add = 1 (the new token's row is in the cache).
@@ -887,12 +932,7 @@ int k_attn_decode(strictb200_ctx* ctx, const bf16* q, const bf16* kc, const bf16
   }
   if (cluster_merge) {
     if (q_out || nsplit > MERGE_MAX) return sb_fail(STRICTB200_ERR_INVALID_ARG, "attention: the merge inside a cluster writes bf16 rows of at most 8 key chunks");
-    static SbDeviceOnce once;
-    SB_CUDA(once.run(ctx->device, [&] {
-      const int most = (int)(smem + merge_bytes(16, D));
-      const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-      return e == cudaSuccess ? cudaFuncSetAttribute(attn_decode_kernel<D, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) : e;
-    }));
+    SB_TRY(merge_set_up(ctx));
     auto go = [&](auto kernel) -> int {
       SB_CUDA(sb_launch_cluster(ctx, kernel, grid, dim3(128), smem + merge_bytes(Hq / Hkv, D), dim3(nsplit, 1, 1), q, kc, vc, lens, len_add, B, Hq, Hkv, maxlen, chunk,
                                 nsplit, scale * LOG2E, o_part, ml_part, rf, ctx->opt.attn_prefetch, out, ctx->d_status));

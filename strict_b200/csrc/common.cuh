@@ -601,7 +601,7 @@ bool sb_retention_decode_fits(const HeadShape& s);
 int k_retention_decode(strictb200_ctx*, const RetentionArgs& a, int64_t B);
 size_t sb_attn_decode_scratch(int B, int Hq, int D, int nsplit);
 int sb_attn_decode_splits(strictb200_ctx*, int B, int Hkv, int maxlen);
-int sb_attn_decode_chunk(strictb200_ctx*, int B, int Hkv, int maxlen, int len_plan, bool fused = false);  // keys per block for sequences of about len_plan keys (at most 8 chunks cover maxlen)
+int sb_attn_decode_chunk(strictb200_ctx*, int B, int Hkv, int maxlen, int len_plan, bool fused = false, int merge_heads = 0);  // keys per block for sequences of about len_plan keys (at most 8 chunks cover maxlen)
 // rope != null: the queries and the new token's key/value rows are computed inside the attention kernel from the qkv
 // projection's partial results (what k_rope_qknorm_kvappend would do in a kernel of its own); q is then unused.
 // cluster_merge: at most 8 key chunks, merged inside a cluster straight to bf16 rows (no q_out, no scratch)

@@ -394,8 +394,8 @@ int decode_enqueue(strictb200_model* m, strictb200_kv* kv) {
     for (int b = 0; b < kv->B; b++) longest = std::max(longest, kv->h_lens[b] + 1);
     if (!kv->chunk || longest > kv->plan_until) {
       const int64_t nqkv = ((int64_t)m->Hq_l + 2 * m->Hkv_l) * m->c.head_dim;
-      const bool fused = fuses_rope(m, kv->B, chained_step(m, kv->B) ? 1 : plan_splits(m, kv->B, nqkv, m->c.d_model));
-      const int chunk = sb_attn_decode_chunk(ctx, kv->B, m->Hkv_l, kv->maxlen, std::min(kv->maxlen, longest + 128), fused);
+      const bool chained = chained_step(m, kv->B), fused = fuses_rope(m, kv->B, chained ? 1 : plan_splits(m, kv->B, nqkv, m->c.d_model));
+      const int chunk = sb_attn_decode_chunk(ctx, kv->B, m->Hkv_l, kv->maxlen, std::min(kv->maxlen, longest + 128), fused, chained ? m->Hq_l / m->Hkv_l : 0);
       if (chunk != kv->chunk) {
         kv->chunk = chunk;
         kv->nsplit = (kv->maxlen + chunk - 1) / chunk;

@@ -322,3 +322,12 @@ def test_many_heads_merged_in_a_cluster_vs_oracle(ctx, oracle, heads, B):
     for o in (kv, m):
         o.dispose()
     st.close(), om.close()
+
+
+# key chunks that are merged in clusters are planned so that all clusters start together: sequences x KV heads, cache, query heads per KV head
+@pytest.mark.parametrize("B,Hkv,maxlen,merge_heads,chunk", [(5, 8, 2032, 2, 256), (6, 8, 2032, 2, 320), (7, 8, 2032, 2, 384), (10, 8, 2032, 2, 512), (16, 8, 2032, 2, 704), (8, 8, 1032, 2, 256),
+                                                            (8, 8, 545, 2, 128), (1, 8, 54, 2, 64), (14, 2, 2032, 16, 256), (16, 2, 2032, 16, 320)])
+def test_merged_chunks_are_planned_in_clusters(ctx, B, Hkv, maxlen, merge_heads, chunk):
+    f = L()._Z20sb_attn_decode_chunkP14strictb200_ctxiiiibi
+    f.restype, f.argtypes = C.c_int, [C.c_void_p] + [C.c_int] * 4 + [C.c_bool, C.c_int]
+    assert f(ctx.h, B, Hkv, maxlen, maxlen, True, merge_heads) == chunk
