@@ -126,7 +126,8 @@ int strictb200_get_option(strictb200_ctx* ctx, const char* name, int* out);
  * this: the calls made on the context between begin and end are recorded into a CUDA graph
  * instead of being run, and graph_launch replays them `times` times on the context's stream
  * with one submission each. While recording, make no call that synchronises, copies to or from
- * host memory, or grows a scratch buffer: run the sequence once before recording it. */
+ * host memory, or grows a scratch buffer: run the sequence once before recording it. (Large
+ * fp32 products need no such run: recorded, they take a kernel without scratch.) */
 typedef struct strictb200_graph strictb200_graph;
 int strictb200_graph_begin(strictb200_ctx* ctx);
 int strictb200_graph_end(strictb200_ctx* ctx, strictb200_graph** out);
@@ -231,7 +232,13 @@ int strictb200_gemm_int8w(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, 
 /* Y[M,N] = X[M,K] . W[N,K]^T, bf16 operands, fp32 accumulation on the tensor cores. out_dtype: 0 bf16, 1 fp32. K % 8 == 0. */
 int strictb200_gemm_bf16(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const uint16_t* d_x, const uint16_t* d_w, void* d_y,
                          int out_dtype);
-/* fp32 Y[M,N] = X[M,K] . W[N,K]^T + bias[N] (bias may be NULL). */
+/* fp32 Y[M,N] = X[M,K] . W[N,K]^T + bias[N] (bias may be NULL). K % 4 == 0; X and W 16-byte aligned.
+ * Large products (more than 128 rows and 44 tiles of 256 channels x 128 rows) run on pairs of SMs over the operands' bf16
+ * terms, which they keep in a scratch of the context: 6 bytes per value of X (at most 32768 rows at a time) and W, at most
+ * 1 GiB. It grows with the first call of a size (a cudaMalloc, and a wait for the stream where an older one goes), stays with
+ * the context, and is given back before any allocation through the context fails. Where it cannot be had, with the option
+ * gemm_pair = 0, and in a recorded sequence, a kernel without scratch takes the product: the same precision, other last bits,
+ * up to 1.5 times the time. */
 int strictb200_gemm_f32(strictb200_ctx* ctx, int64_t M, int64_t N, int64_t K, const float* d_x, const float* d_w,
                         const float* d_bias, float* d_y);
 
