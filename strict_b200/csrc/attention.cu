@@ -799,7 +799,7 @@ static int merge_set_up(strictb200_ctx* ctx) {
 }
 // Clusters of `size` blocks of the merging form that run at once. A cluster needs its blocks' places in one part of the GPU, and of more than four blocks the calculator's
 // number did not all start together: 48 of 48 clusters of eight, 56 of 56 of seven, 80 of 82 of five, 64 of 71 of six and 30 of 33 of eight (with 16 heads) left
-// some for a second wave, 40 of 48, 48 of 71, 64 of 82 and 28 of 33 did not; 96 of 104 clusters of four and 128 of 142 of three neither.
+// some for a second wave, 40 of 48, 48 of 71, 64 of 82 and 28 of 33 did not; 96 of 104 clusters of four neither, 128 of 142 of three hardly ever.
 static int64_t merge_clusters(strictb200_ctx* ctx, bool fused, int heads, int size) {
   static std::mutex mu;
   static int known[64][2][17][MERGE_MAX + 1] = {};
@@ -833,7 +833,7 @@ static int64_t merge_clusters(strictb200_ctx* ctx, bool fused, int heads, int si
 // stub per sequence, chunks of 448 run five even ones (14 % less attention time, measured). The
 // attn_blocks_per_sm option restores the plain "that many blocks per SM" rule. `fused`: the kernel with the RoPE prologue will run;
 // `merge_heads`: the form that merges its chunks in a cluster, with that many query heads per KV head (0: not that one). Its waves are clusters (blocks without keys
-// leave at once and are not counted). Planned by blocks, 10 sequences of 2000 keys with 8 KV heads ran 80 clusters of five in two waves: 27.0 us; 80 of four: 17.3.
+// leave at once and are not counted). Planned by blocks, 10 sequences of 2000 keys with 8 KV heads ran 80 clusters of five in two waves: 25.3 us; 80 of four: 18.8.
 static int decode_chunk(strictb200_ctx* ctx, int B, int Hkv, int maxlen, int len_plan = 0, bool fused = false, bool short_chunks = true, int merge_heads = 0) {
   const int per_sm = ctx->opt.attn_blocks_per_sm;
   const int tiles = (maxlen + KT - 1) / KT;
